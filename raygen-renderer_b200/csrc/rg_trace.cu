@@ -709,57 +709,89 @@ __global__ void __launch_bounds__(128) k_connect(const DevJob* __restrict__ jobs
   warpAddStat(&Q.stats[5], rays);
 }
 
-// ---- 8-wide traversal kernels with per-lane ray refill ----------------------
-// Persistent warps (Aila & Laine's persistent threads with ray refill, with
-// the triangle postponing of Ylitie et al.'s compressed wide BVH traversal):
-// * a lane whose ray finished is refilled once enough lanes of its warp are
-//   idle (warp ballot + one atomic per warp);
-// * every step a lane either intersects one node or tests one triangle; a
-//   lane with pending triangles pushes them as a triangle group and keeps
-//   descending unless enough lanes of the warp have triangles to test, so the
-//   warp runs mostly one kind of step at a time.
-// Stack entries: node group (childBase, hits | imask << 8) or triangle group
-// (triBase | 0x80000000, triangle mask).
-// Refill and triangle-vote thresholds, per traversal kind (closest hit /
-// shadow rays); build-time overridable (-D) for sweeps.
+// ---- 8-wide traversal kernels: node steps per lane, triangle tests per warp -----
+// Persistent warps (Aila & Laine's persistent threads with ray refill).  A lane
+// holds one ray and walks its nodes; a lane whose ray finished is refilled once
+// enough lanes of its warp are idle, from a run of rays that the warp claimed.
+//
+// A lane that has triangles and a lane that has a node cannot step together, and
+// testing its own triangles left 13 of 32 lanes active (292 warp instructions per
+// closest-hit ray on the 4M-triangle scene).  So the two kinds of work are kept
+// apart.  Every lane with a node takes a node step; then
+// * while kDirect or more lanes hold triangles, each of them tests one of its own
+//   (coherent rays, small scenes: the warp is full enough as it is);
+// * the triangles left go into a queue of the warp in shared memory, and once it
+//   holds a full warp's worth (or few lanes have a node to visit) every lane
+//   tests one of them for the ray of whichever lane queued it, whose origin and
+//   direction come by shuffles.  The owner folds the hits found for it in queue
+//   order.  A lane goes on to its next node while its triangles wait.
+// Measured (closest / shadow rays, serial kernels, the previous per-lane tests
+// before the arrow): 4M triangles at 1080p, 32 spp 113.4 -> 90.5 / 44.3 -> 33.6 ms;
+// 1M triangles in fog 52.0 -> 41.1 / 26.1 -> 19.2; 20k triangles at 800x600, 4 spp
+// 2.24 -> 1.64 / 1.67 -> 1.20; the cube room at 256x256, 16 spp 0.52 -> 0.38 /
+// 0.29 -> 0.22.  kDirect: 4 / 8 / 12 / 16 / 24 / never gives 99.5 / 91.9 / 90.5 /
+// 90.2 / 92.4 / 90.3 ms on the first and 1.77 / 1.69 / 1.64 / 1.78 / 2.03 / 2.16
+// ms on the 20k-triangle scene.  The batch's lower bound on lanes with a node
+// (4 - 20) moves nothing.
+// All build-time overridable (-D) for sweeps, per kind (closest hit / shadow rays).
 #ifndef RG_REFILL_IDLE_CLOSEST
-#define RG_REFILL_IDLE_CLOSEST 8
+#define RG_REFILL_IDLE_CLOSEST 12
 #endif
 #ifndef RG_REFILL_IDLE_ANY
-#define RG_REFILL_IDLE_ANY 8
+#define RG_REFILL_IDLE_ANY 12
 #endif
-#ifndef RG_TRI_VOTES_CLOSEST
-#define RG_TRI_VOTES_CLOSEST 4
+// idle lanes at which the warp is refilled (4 / 8 / 12 / 16: 104 / 92.1 / 89.5 / 89.7 ms of closest hits)
+constexpr int kRefillIdleClosest = RG_REFILL_IDLE_CLOSEST, kRefillIdleAny = RG_REFILL_IDLE_ANY;
+#ifndef RG_LOW_NODES
+#define RG_LOW_NODES 12
 #endif
-#ifndef RG_TRI_VOTES_ANY
-#define RG_TRI_VOTES_ANY 4
+constexpr int kLowNodes = RG_LOW_NODES;  // lanes with a node below which a partial batch is tested
+#ifndef RG_DIRECT_CLOSEST
+#define RG_DIRECT_CLOSEST 12
 #endif
-constexpr int kRefillIdle = RG_REFILL_IDLE_CLOSEST;  // refill once this many lanes are idle
+#ifndef RG_DIRECT_ANY
+#define RG_DIRECT_ANY 12
+#endif
+constexpr int kDirectClosest = RG_DIRECT_CLOSEST, kDirectAny = RG_DIRECT_ANY;
 #ifndef RG_SHARED_STACK
 #define RG_SHARED_STACK 8
 #endif
 constexpr int kSharedStack = RG_SHARED_STACK;  // traversal stack entries kept in shared memory (the rest in local)
 constexpr int kTraceBlock = 128;   // block size of the persistent traversal kernels
-constexpr int kTriVotes = RG_TRI_VOTES_CLOSEST;  // lanes with triangles needed to run a triangle step (swept: 2-4 best, 10 -1.6%)
+constexpr int kTraceWarps = kTraceBlock / 32;
+// Triangle queue of a warp (a power of two; a node's leaves hold at most 32 triangles).
+constexpr int kTriQueue = 128;
+static_assert((kTriQueue & (kTriQueue - 1)) == 0 && kTriQueue >= 64, "ring of at least a batch and one node's triangles");
 
 template <bool ANY, bool MULTI>
 __device__ __forceinline__ void traverseWave8(const DevScene& S0, const DevJob* __restrict__ jobs, int count, int* fetch, const float4* __restrict__ rO,
                                               const float4* __restrict__ rD, uint32_t occ, float4* __restrict__ hitsOut,
                                               const float4* __restrict__ contrib, float4* __restrict__ pathL,
                                               uint32_t& nodes, uint32_t& tris, uint32_t& rays) {
-  const int lane = threadIdx.x & 31;
+  constexpr unsigned kAll = 0xffffffffu;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const unsigned ltMask = (1u << lane) - 1u;
   int q = -1;  // -1: needs a ray, -2: none left
   V3 o = v3(0, 0, 0), d = v3(0, 0, 1), inv = v3(0, 0, 0);
   uint32_t oct = 0;
   float tmax = 0.0f, hu = 0.0f, hv = 0.0f;
-  int prim = -1, pid = 0;
+  int prim = -1;
+  bool occluded = false;
   uint32_t gInner = 0, gImask = 0, tMask = 0;
   int gBase = 0, tBase = 0, sp = 0, steps = 0;
-  // traversal stack: entries [0, kSharedStack) in shared memory, entry-major so a
-  // warp at one depth touches consecutive words; deeper entries in local memory
+  // traversal stack of node groups (childBase, hits | imask << 8): entries
+  // [0, kSharedStack) in shared memory, entry-major so a warp at one depth touches
+  // consecutive words; deeper entries in local memory
   __shared__ uint2 sStack[kSharedStack > 0 ? kSharedStack : 1][kTraceBlock];
   uint2 lStack[kStack8 - kSharedStack];
+  // triangle queue: entries [head, tail) modulo kTriQueue, head and tail alike in all lanes
+  __shared__ int sTri[kTraceWarps][kTriQueue];
+  __shared__ uint8_t sOwner[kTraceWarps][kTriQueue];
+  __shared__ unsigned sHits[kTraceWarps][32];  // per owner: the batch entries that hit
+  int head = 0, tail = 0;
+  int qEnd = 0;  // queue position after this lane's last entry
+  sHits[warp][lane] = 0u;
+  __syncwarp();
   auto push = [&](uint2 e) {
     if (sp < kSharedStack) sStack[sp][threadIdx.x] = e;
     else lStack[sp - kSharedStack] = e;
@@ -769,49 +801,49 @@ __device__ __forceinline__ void traverseWave8(const DevScene& S0, const DevJob* 
     --sp;
     return sp < kSharedStack ? sStack[sp][threadIdx.x] : lStack[sp - kSharedStack];
   };
-  const float4* nodesP = nullptr;
-  const float4* trisP = nullptr;
-  int numNodes = 0;
-  int* errP = nullptr;
+  const float4* nodesP = MULTI ? nullptr : S0.nodes8;
+  const float4* trisP = MULTI ? nullptr : S0.triVerts;
+  int numNodes = MULTI ? 0 : S0.numNodes8;
+  int* errP = MULTI ? nullptr : S0.error;
+  // Rays are claimed in runs of `chunk`, at least a warp's worth (a refill wants at most 32)
+  constexpr int chunk = 32;
+  int next = 0, end = 0;
   for (;;) {
-    // ---- refill idle lanes
+    // ---- refill idle lanes (none of theirs is left in the queue)
     const bool need = q == -1;
-    const unsigned needMask = __ballot_sync(0xffffffffu, need);
+    const unsigned needMask = __ballot_sync(kAll, need);
     if (needMask) {
-      const int leader = __ffs(needMask) - 1;
-      int base = 0;
-      if (lane == leader) base = atomicAdd(fetch, __popc(needMask));
-      base = __shfl_sync(0xffffffffu, base, leader);
+      // from the warp's claimed run of rays [next, end), and past its end from a new one
+      const int want = __popc(needMask), left = end - next;
+      int fresh = 0;
+      if (want > left) {
+        if (lane == 0) fresh = atomicAdd(fetch, chunk);
+        fresh = __shfl_sync(kAll, fresh, 0);
+        // the new run's rays into L1 while the warp goes on with the lanes it fills now
+        if (lane < chunk && fresh + lane < count) {
+          asm volatile("prefetch.global.L1 [%0];" ::"l"(rO + fresh + lane));
+          asm volatile("prefetch.global.L1 [%0];" ::"l"(rD + fresh + lane));
+        }
+      }
       if (need) {
-        const int idx = base + __popc(needMask & ltMask);
+        const int rank = __popc(needMask & ltMask);
+        const int idx = rank < left ? next + rank : fresh + (rank - left);
         if (idx < count) {
           q = idx;
           const float4 a = rO[q], b = rD[q];
           o = xyz(a);
           d = xyz(b);
-          int slot;
-          if (ANY) {
-            tmax = b.w;
-            pid = __float_as_int(a.w);
-            slot = __float_as_int(contrib[q].w);
-          } else {
-            tmax = kMaxRayDistance;
-            slot = __float_as_int(b.w);
-          }
+          tmax = ANY ? b.w : kMaxRayDistance;
           if (MULTI) {
-            const DevScene& S = jobs[slot].S;
+            const DevScene& S = jobs[__float_as_int(ANY ? contrib[q].w : b.w)].S;
             nodesP = S.nodes8;
             trisP = S.triVerts;
             numNodes = S.numNodes8;
             errP = S.error;
-          } else {
-            nodesP = S0.nodes8;
-            trisP = S0.triVerts;
-            numNodes = S0.numNodes8;
-            errP = S0.error;
           }
           prim = -1;
           hu = hv = 0.0f;
+          occluded = false;
           inv = safeInv(d);
           oct = rayOctant(inv);
           gBase = 0;
@@ -825,47 +857,76 @@ __device__ __forceinline__ void traverseWave8(const DevScene& S0, const DevJob* 
           q = -2;
         }
       }
+      if (want > left) {
+        next = fresh + (want - left);
+        end = fresh + chunk;
+      } else {
+        next += want;
+      }
     }
-    if (__ballot_sync(0xffffffffu, q >= 0) == 0) break;
+    if (__ballot_sync(kAll, q >= 0) == 0) break;
     // ---- traversal steps until enough lanes are idle
     for (;;) {
-      const bool alive = q >= 0;
-      int result = 0;  // 1: finished (closest: hit record, any: unoccluded), 2: occluded
-      if (alive && tMask == 0 && gInner == 0) {
-        if (sp == 0) {
-          result = 1;
+      if (gInner == 0 && sp > 0) {
+        const uint2 e = pop();
+        gBase = (int)e.x;
+        gInner = e.y & 0xffu;
+        gImask = e.y >> 8;
+      }
+      // ---- node step of every lane that has one (its last triangles are queued)
+      const bool ready = gInner != 0 && tMask == 0;
+      const unsigned readyMask = __ballot_sync(kAll, ready);
+      if (ready) {
+        const int pos = 31 - __clz(gInner);
+        gInner &= ~(1u << pos);
+        const int slot = pos ^ (int)oct;
+        const int node = gBase + __popc(gImask & ((1u << slot) - 1u));
+        if (gInner) {
+          if (sp < kStack8) push(make_uint2((uint32_t)gBase, gInner | (gImask << 8)));
+          else atomicCAS(errP, 0, kErrStackOverflow);
+        }
+        if (node >= numNodes || ++steps > c_traversalStepCap) {
+          atomicCAS(errP, 0, kErrTraversalSteps);
+          gInner = 0;
+          sp = 0;
+          occluded = true;
         } else {
-          const uint2 e = pop();
-          if (e.x & 0x80000000u) {
-            tBase = (int)(e.x & 0x7fffffffu);
-            tMask = e.y;
-          } else {
-            gBase = (int)e.x;
-            gInner = e.y & 0xffu;
-            gImask = e.y >> 8;
+          const Node8Hit g = intersectNode8(nodesP + (size_t)node * kNode8Vec, o, inv, tmax, oct);
+          nodes++;
+          gInner = g.inner;
+          gImask = g.imask;
+          gBase = g.childBase;
+          tMask = g.tris;
+          tBase = g.triBase;
+          const int nslot = (31 - __clz(gInner)) ^ (int)oct;
+          const int nnode = gBase + __popc(gImask & ((1u << nslot) - 1u));
+          // closest hit: the node this group visits next into L1 while the warp's other
+          // lanes finish their step (for shadow rays it measured slower)
+          if (!ANY && gInner && nnode < numNodes) {
+            const char* np = reinterpret_cast<const char*>(nodesP + (size_t)nnode * kNode8Vec);
+            asm volatile("prefetch.global.L1 [%0];" ::"l"(np));
+            asm volatile("prefetch.global.L1 [%0];" ::"l"(np + 128));
+            asm volatile("prefetch.global.L1 [%0];" ::"l"(np + 207));
           }
         }
       }
-      const bool hasTri = alive && result == 0 && tMask != 0;
-      const int triVotes = __popc(__ballot_sync(0xffffffffu, hasTri));
-      if (alive && result == 0) {
-        const bool doTri = hasTri && (gInner == 0 || triVotes >= (ANY ? RG_TRI_VOTES_ANY : kTriVotes));
-        if (doTri) {
-          // up to two triangles per step: a triangle step costs about half a node
-          // step, so two keep the triangle and node branches of a divergent warp
-          // closer in length (swept: 1 / 2 / 3 / 4 per step)
-#pragma unroll 1
-         for (int rep = 0; rep < 2 && tMask && result == 0; rep++) {
-          const int i = __ffs(tMask) - 1;
+      // ---- while most lanes hold triangles, each tests one of its own: the warp is full as it is
+      while (__popc(__ballot_sync(kAll, tMask != 0)) >= (ANY ? kDirectAny : kDirectClosest)) {
+        if (tMask) {
+          const int tk = tBase + __ffs(tMask) - 1;
           tMask &= tMask - 1u;
-          const int tk = tBase + i;
           const float4* tp = trisP + (size_t)tk * 3;
           const float4 b = ldTri4(tp + 1);
           if (!ANY || (__float_as_uint(b.w) & occ)) {
             const float4 a = ldTri4(tp), c = ldTri4(tp + 2);
             tris++;
             if (ANY) {
-              if (mtAny(o, d, xyz(a), xyz(b), xyz(c), tmax)) result = 2;
+              if (mtAny(o, d, xyz(a), xyz(b), xyz(c), tmax)) {
+                occluded = true;
+                gInner = 0;
+                sp = 0;
+                tMask = 0;
+              }
             } else {
               ClosestHit h;
               h.t = tmax;
@@ -879,49 +940,99 @@ __device__ __forceinline__ void traverseWave8(const DevScene& S0, const DevJob* 
               }
             }
           }
-         }
-        } else {
-          // node step (pending triangles are postponed onto the stack)
-          if (hasTri) {
-            if (sp < kStack8) push(make_uint2((uint32_t)tBase | 0x80000000u, tMask));
-            else atomicCAS(errP, 0, kErrStackOverflow);
-            tMask = 0;
+        }
+      }
+      // ---- queue the triangles found, as many lanes (in lane order) as fit
+      if (__any_sync(kAll, tMask != 0)) {
+        const int n = __popc(tMask);
+        int incl = n;
+#pragma unroll
+        for (int s = 1; s < 32; s <<= 1) {
+          const int up = __shfl_up_sync(kAll, incl, s);
+          if (lane >= s) incl += up;
+        }
+        const int room = kTriQueue - (tail - head);
+        const unsigned fit = __ballot_sync(kAll, incl <= room);  // a run of lanes from lane 0
+        if (n > 0 && incl <= room) {
+          int at = tail + incl - n;
+          while (tMask) {
+            sTri[warp][at & (kTriQueue - 1)] = tBase + __ffs(tMask) - 1;
+            sOwner[warp][at & (kTriQueue - 1)] = (uint8_t)lane;
+            tMask &= tMask - 1u;
+            at++;
           }
-          const int pos = 31 - __clz(gInner);
-          gInner &= ~(1u << pos);
-          const int slot = pos ^ (int)oct;
-          const int node = gBase + __popc(gImask & ((1u << slot) - 1u));
-          if (gInner) {
-            if (sp < kStack8) push(make_uint2((uint32_t)gBase, gInner | (gImask << 8)));
-            else atomicCAS(errP, 0, kErrStackOverflow);
+          qEnd = at;
+        }
+        if (fit) tail += __shfl_sync(kAll, incl, 31 - __clz(fit));
+        __syncwarp();
+      }
+      // ---- test a batch of queued triangles, one per lane
+      const int queued = tail - head;
+      if (queued >= 32 || (queued > 0 && __popc(readyMask) < kLowNodes)) {
+        const int n = min(queued, 32);
+        const bool mine = lane < n;
+        const int at = (head + (mine ? lane : 0)) & (kTriQueue - 1);
+        const int tk = sTri[warp][at], own = sOwner[warp][at];
+        const V3 ro = v3(__shfl_sync(kAll, o.x, own), __shfl_sync(kAll, o.y, own), __shfl_sync(kAll, o.z, own));
+        const V3 rd = v3(__shfl_sync(kAll, d.x, own), __shfl_sync(kAll, d.y, own), __shfl_sync(kAll, d.z, own));
+        const float4* base = MULTI ? reinterpret_cast<const float4*>(
+                                         __shfl_sync(kAll, reinterpret_cast<unsigned long long>(trisP), own))
+                                   : trisP;
+        ClosestHit h;
+        h.t = __shfl_sync(kAll, tmax, own);
+        h.u = h.v = 0.0f;
+        bool hit = false;
+        if (mine) {
+          const float4* tp = base + (size_t)tk * 3;
+          const float4 b = ldTri4(tp + 1);
+          if (!ANY || (__float_as_uint(b.w) & occ)) {
+            const float4 a = ldTri4(tp), c = ldTri4(tp + 2);
+            tris++;
+            if (ANY) hit = mtAny(ro, rd, xyz(a), xyz(b), xyz(c), h.t);
+            else hit = mtClosest(ro, rd, xyz(a), xyz(b), xyz(c), h);
           }
-          if (node >= numNodes || ++steps > c_traversalStepCap) {
-            atomicCAS(errP, 0, kErrTraversalSteps);
-            result = ANY ? 2 : 1;
+        }
+        head += n;
+        if (__any_sync(kAll, hit)) {
+          if (hit) atomicOr(&sHits[warp][own], 1u << lane);
+          __syncwarp();
+          unsigned m = sHits[warp][lane];
+          if (m) sHits[warp][lane] = 0u;
+          __syncwarp();
+          if (ANY) {
+            if (m) {
+              occluded = true;
+              gInner = 0;
+              sp = 0;
+              tMask = 0;
+            }
           } else {
-            const Node8Hit g = intersectNode8(nodesP + (size_t)node * kNode8Vec, o, inv, tmax, oct);
-            nodes++;
-            gInner = g.inner;
-            gImask = g.imask;
-            gBase = g.childBase;
-            tMask = g.tris;
-            tBase = g.triBase;
-            const int nslot = (31 - __clz(gInner)) ^ (int)oct;
-            const int nnode = gBase + __popc(gImask & ((1u << nslot) - 1u));
-            // closest hit: the node this group visits next into L1 while the warp's other
-            // lanes finish their step (for shadow rays it measured slower)
-            if (!ANY && gInner && nnode < numNodes) {
-              const char* np = reinterpret_cast<const char*>(nodesP + (size_t)nnode * kNode8Vec);
-              asm volatile("prefetch.global.L1 [%0];" ::"l"(np));
-              asm volatile("prefetch.global.L1 [%0];" ::"l"(np + 128));
-              asm volatile("prefetch.global.L1 [%0];" ::"l"(np + 207));
+            int best = -1;
+            while (__any_sync(kAll, m != 0)) {  // in queue order: the first of equal distances stays
+              const int k = m ? __ffs(m) - 1 : lane;
+              const float t = __shfl_sync(kAll, h.t, k);
+              if (m && t < tmax) {
+                tmax = t;
+                best = k;
+              }
+              m &= m - 1u;
+            }
+            const int k = best < 0 ? lane : best;
+            const float u = __shfl_sync(kAll, h.u, k), v = __shfl_sync(kAll, h.v, k);
+            const int p = __shfl_sync(kAll, tk, k);
+            if (best >= 0) {
+              hu = u;
+              hv = v;
+              prim = p;
             }
           }
         }
       }
-      if (result != 0) {
+      // ---- finished rays: nothing left to visit, none of their triangles queued
+      if (q >= 0 && gInner == 0 && sp == 0 && tMask == 0 && qEnd <= head) {
         if (ANY) {
-          if (result == 1) {
+          if (!occluded) {
+            const int pid = __float_as_int(rO[q].w);
             const float4 c = contrib[q];
             float4 l = pathL[pid];
             l.x += c.x;
@@ -934,9 +1045,9 @@ __device__ __forceinline__ void traverseWave8(const DevScene& S0, const DevJob* 
         }
         q = -1;
       }
-      const unsigned idle = __ballot_sync(0xffffffffu, q == -1);
-      const unsigned live = __ballot_sync(0xffffffffu, q >= 0);
-      if (live == 0 || __popc(idle) >= (ANY ? RG_REFILL_IDLE_ANY : kRefillIdle)) break;
+      const unsigned idle = __ballot_sync(kAll, q == -1);
+      const unsigned live = __ballot_sync(kAll, q >= 0);
+      if (live == 0 || __popc(idle) >= (ANY ? kRefillIdleAny : kRefillIdleClosest)) break;
     }
   }
 }
