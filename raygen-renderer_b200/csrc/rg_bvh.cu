@@ -17,6 +17,7 @@
 #include <cstdio>
 #include <cstdlib>
 #include <cub/device/device_scan.cuh>
+#include <cuda_fp16.h>
 
 #include <cfloat>
 #include <vector>
@@ -647,11 +648,15 @@ __global__ void k_gather(int n, const int* __restrict__ primIdx, const float4* _
 
 
 // ---- 8-wide BVH (collapse of the binary build) ---------------------------------
-// Node (208 B = kNode8Vec float4): (childBase, triBase, meta[0..3], meta[4..7]), then
-// per axis x, y, z the 8 children's lo planes and their 8 hi planes (2 float4 each).
-// meta[s] = 0x80: slot s is an inner child, stored at childBase + (inner slots
-// below s); ((count - 1) << 5) | offset: a leaf of `count` (1..4) triangles at
-// triBase + offset; an empty slot has an inverted box and is never entered.
+// Node (128 B = kNode8Vec float4; word k is stored at word k ^ (node index % 8)):
+//   (childBase, triBase, meta[0..3], meta[4..7])
+//   (origin x, y, z, scale | inner mask)
+//   per axis x, y, z: 8 half lo planes, 8 half hi planes of the child boxes
+// A plane lies at origin + scale * half value; scale is a power of two (its exponent
+// bits, in place) that maps the node's extent to at most 2^15, so thin axes keep
+// their precision, and planes are rounded outward.  meta[s] = (count << 5) | offset: a
+// leaf of `count` (1..4) triangles at triBase + offset; 0 for an inner child, stored at
+// childBase + (inner slots below s), and for an empty slot, which has an inverted box.
 // Slots are assigned per octant: a child whose centre lies on the negative side
 // of the node centre along axis k prefers slots with bit k set, so visiting hit
 // slots in descending order of (slot XOR ray octant) is roughly front to back.
@@ -731,29 +736,56 @@ __global__ void k_collapse(int numTasks, const int2* __restrict__ tasks, const B
   int childAt[8];
   for (int sl = 0; sl < 8; sl++) childAt[sl] = -1;
   for (int j = 0; j < nc; j++) childAt[slotOf[j]] = ch[j];
-  // float planes of the child boxes (each widened by the inflate margin); an empty
-  // slot keeps an inverted box (+inf / -inf) that no ray enters
-  float pl[3][2][8];
+  // planes of the child boxes (each widened by the inflate margin) as half values; an
+  // empty slot keeps an inverted box.  A node that is not of finite size has boxes
+  // that every ray enters.
+  // The origin of the planes is, per axis, the node's low end, centre or high end: the one
+  // closest to the planes of thin boxes (walls, floors, lamps), whose rounding matters most
+  // because rays start and end at such surfaces.
+  float org[3], ext = 0.0f;
+  for (int k = 0; k < 3; k++) {
+    const float cand[3] = {ctr[k], lo[k], hi[k]}, thin = (hi[k] - lo[k]) * (1.0f / 256.0f);
+    float best = FLT_MAX;
+    org[k] = ctr[k];
+    for (int q = 0; q < 3; q++) {
+      float cost = 0.0f;
+      for (int i = 0; i < nc; i++) {
+        const BNode& c = nodes[ch[i]];
+        cost += (fabsf(c.bmin[k] - cand[q]) + fabsf(c.bmax[k] - cand[q])) / (c.bmax[k] - c.bmin[k] + thin);
+      }
+      if (cost < best) {
+        best = cost;
+        org[k] = cand[q];
+      }
+    }
+    ext = fmaxf(ext, fmaxf(__fsub_ru(hi[k], org[k]), __fsub_ru(org[k], lo[k])));
+  }
+  const bool finite = ext < 1e30f;
+  int exponent = 0;
+  if (finite) frexpf(ext, &exponent);  // ext < 2^exponent
+  exponent = max(exponent - 15, -126);
+  const float scale = ldexpf(1.0f, exponent), toHalf = ldexpf(1.0f, -exponent);
+  __half pl[3][2][8];
   for (int k = 0; k < 3; k++)
     for (int sl = 0; sl < 8; sl++) {
-      pl[k][0][sl] = INFINITY;
-      pl[k][1][sl] = -INFINITY;
+      pl[k][0][sl] = __float2half_rn(65504.0f);
+      pl[k][1][sl] = __float2half_rn(-65504.0f);
     }
-  uint32_t meta[2] = {0, 0};
+  uint32_t meta[2] = {0, 0}, inner = 0;
   int ni = 0, ntri = 0;
   for (int sl = 0; sl < 8; sl++) {
     const int c = childAt[sl];
     if (c < 0) continue;
     const BNode& cn = nodes[c];
     for (int k = 0; k < 3; k++) {
-      pl[k][0][sl] = inflateLo(cn.bmin[k]);
-      pl[k][1][sl] = inflateHi(cn.bmax[k]);
+      pl[k][0][sl] = finite ? __float2half_rd(__fsub_rd(inflateLo(cn.bmin[k]), org[k]) * toHalf) : __float2half_rd(-INFINITY);
+      pl[k][1][sl] = finite ? __float2half_ru(__fsub_ru(inflateHi(cn.bmax[k]), org[k]) * toHalf) : __float2half_ru(INFINITY);
     }
     if (cn.left >= 0) {
-      meta[sl >> 2] |= 0x80u << (8 * (sl & 3));
+      inner |= 1u << sl;
       ni++;
     } else {
-      meta[sl >> 2] |= (uint32_t)(((cn.count - 1) << 5) | ntri) << (8 * (sl & 3));
+      meta[sl >> 2] |= (uint32_t)((cn.count << 5) | ntri) << (8 * (sl & 3));
       ntri += cn.count;
     }
   }
@@ -764,12 +796,15 @@ __global__ void k_collapse(int numTasks, const int2* __restrict__ tasks, const B
     return;
   }
   float4* o = nodes8 + (size_t)task.y * kNode8Vec;
-  o[0] = make_float4(__int_as_float(childBase), __int_as_float(triBase), __uint_as_float(meta[0]), __uint_as_float(meta[1]));
+  const int sw = task.y & 7;
+  o[0 ^ sw] = make_float4(__int_as_float(childBase), __int_as_float(triBase), __uint_as_float(meta[0]), __uint_as_float(meta[1]));
+  o[1 ^ sw] = make_float4(finite ? org[0] : 0.0f, finite ? org[1] : 0.0f, finite ? org[2] : 0.0f,
+                     __uint_as_float(__float_as_uint(scale) | inner));
   for (int k = 0; k < 3; k++)
     for (int h = 0; h < 2; h++) {
-      const float* q = pl[k][h];
-      o[1 + 4 * k + 2 * h] = make_float4(q[0], q[1], q[2], q[3]);
-      o[2 + 4 * k + 2 * h] = make_float4(q[4], q[5], q[6], q[7]);
+      __align__(16) __half2 q[4];
+      for (int j = 0; j < 4; j++) q[j] = __halves2half2(pl[k][h][2 * j], pl[k][h][2 * j + 1]);
+      o[(2 + 2 * k + h) ^ sw] = *reinterpret_cast<const float4*>(q);
     }
   int k = 0, off = 0;
   for (int sl = 0; sl < 8; sl++) {

@@ -15,14 +15,10 @@ constexpr float kRRMin = 0.05f, kRRMax = 0.95f;  // rayrenderer.cpp:44-45
 constexpr int kMaxLeaf = 8;                   // triangles per leaf in the device BVH
 constexpr int kMaxMediumCount = 64;           // cap on a medium's octaves, strata and march steps
 constexpr int kStackSize = 64;
-// 8-wide BVH node: a header float4 (child base, triangle base, 8 meta bytes) and the
-// float planes of the 8 child boxes, per axis 8 lo then 8 hi values (12 float4);
-// the node stride in float4 is build-time overridable (-D) for sweeps (>= 13)
-#ifndef RG_NODE8_VEC
-#define RG_NODE8_VEC 13
-#endif
-constexpr int kNode8Vec = RG_NODE8_VEC;
-static_assert(kNode8Vec >= 13, "an 8-wide node holds 13 float4");
+// 8-wide BVH node, 128 bytes (8 float4): child base, triangle base, 8 meta bytes; the
+// node's centre and a word of plane scale, inner and leaf masks; then per axis the 8
+// child boxes' lo and hi planes as half values relative to the centre (k_collapse).
+constexpr int kNode8Vec = 8;
 
 // occluder classes (bit per shadow-ray predicate)
 constexpr uint32_t kOccArea = 1u;   // transparency < 0.01 && emission <= 0   (rayrenderer.cpp:1956-1959)
@@ -138,7 +134,7 @@ struct DevScene {
   const DevTexture* textures;
   int numTextures;
   int* error;                 // device error word (first error code wins)
-  const float4* nodes8;       // 5 float4 per 8-wide compressed node (when bvhWidth == 8)
+  const float4* nodes8;       // kNode8Vec float4 per 8-wide node (when bvhWidth == 8)
   int numNodes8;
   int bvhWidth;               // 2 or 8
   // equirectangular environment map, looked up by view-space direction

@@ -891,7 +891,7 @@ __device__ __forceinline__ void traverseWave8(const DevScene& S0, const DevJob* 
           sp = 0;
           occluded = true;
         } else {
-          const Node8Hit g = intersectNode8(nodesP + (size_t)node * kNode8Vec, o, inv, tmax, oct);
+          const Node8Hit g = intersectNode8(nodesP, node, o, inv, tmax, oct);
           nodes++;
           gInner = g.inner;
           gImask = g.imask;
@@ -902,12 +902,8 @@ __device__ __forceinline__ void traverseWave8(const DevScene& S0, const DevJob* 
           const int nnode = gBase + __popc(gImask & ((1u << nslot) - 1u));
           // closest hit: the node this group visits next into L1 while the warp's other
           // lanes finish their step (for shadow rays it measured slower)
-          if (!ANY && gInner && nnode < numNodes) {
-            const char* np = reinterpret_cast<const char*>(nodesP + (size_t)nnode * kNode8Vec);
-            asm volatile("prefetch.global.L1 [%0];" ::"l"(np));
-            asm volatile("prefetch.global.L1 [%0];" ::"l"(np + 128));
-            asm volatile("prefetch.global.L1 [%0];" ::"l"(np + 207));
-          }
+          if (!ANY && gInner && nnode < numNodes)
+            asm volatile("prefetch.global.L1 [%0];" ::"l"(nodesP + (size_t)nnode * kNode8Vec));
         }
       }
       // ---- while most lanes hold triangles, each tests one of its own: the warp is full as it is
