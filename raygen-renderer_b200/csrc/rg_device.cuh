@@ -342,41 +342,51 @@ __host__ __device__ __forceinline__ uint32_t pcg4d_x(uint32_t a, uint32_t b, uin
   return v0;
 }
 
-template <int BASE>
-__device__ __forceinline__ float radicalInverseT(uint32_t i) {
-  const float invBase = 1.0f / (float)BASE;
+// Halton bases (the first 16 primes), 1 / base, and the multiplier of the division by the
+// base: for i < 2^26, i / b = (i m) >> 32 with m = floor(2^32 / b) + 1 (2^31 for b = 2),
+// since i (m b - 2^32) <= 2^26 53 < 2^32.
+struct HaltonBase {
+  uint32_t base, mul;
+  float inv;
+};
+#define RG_HALTON(b) {b, b == 2 ? 0x80000000u : (uint32_t)(0x100000000ull / b) + 1u, 1.0f / (float)b}
+static __constant__ HaltonBase c_halton[16] = {
+    RG_HALTON(2),  RG_HALTON(3),  RG_HALTON(5),  RG_HALTON(7),  RG_HALTON(11), RG_HALTON(13), RG_HALTON(17), RG_HALTON(19),
+    RG_HALTON(23), RG_HALTON(29), RG_HALTON(31), RG_HALTON(37), RG_HALTON(41), RG_HALTON(43), RG_HALTON(47), RG_HALTON(53)};
+#undef RG_HALTON
+
+// Sample indices of 2^26 and more: the digits in 64 bits.
+static __device__ __noinline__ float radicalInverseLarge(uint32_t i, uint32_t base, float inv) {
   float invBaseN = 1.0f;
   uint64_t rev = 0;
   while (i > 0) {
-    const uint32_t next = i / BASE;
-    const uint32_t digit = i - next * BASE;
-    rev = rev * BASE + digit;
-    invBaseN = __fmul_rn(invBaseN, invBase);
+    const uint32_t next = i / base;
+    rev = rev * base + (i - next * base);
+    invBaseN = __fmul_rn(invBaseN, inv);
     i = next;
   }
   const float v = __fmul_rn((float)rev, invBaseN);
   return v < 1.0f ? v : 0.9999999f;
 }
 
+// radicalInverse(i, prime[dim]), raycommon.cpp:48-61.  One loop over a table instead of a
+// copy of the loop per base: the shade kernel draws up to four per vertex in several
+// places, and instruction fetch is one of its main stalls.  The reversed digits of
+// i < 2^26 fit 32 bits (below i base).
 __device__ __forceinline__ float radicalInverseDim(uint32_t i, int dim) {
-  switch (dim) {
-    case 0: return radicalInverseT<2>(i);
-    case 1: return radicalInverseT<3>(i);
-    case 2: return radicalInverseT<5>(i);
-    case 3: return radicalInverseT<7>(i);
-    case 4: return radicalInverseT<11>(i);
-    case 5: return radicalInverseT<13>(i);
-    case 6: return radicalInverseT<17>(i);
-    case 7: return radicalInverseT<19>(i);
-    case 8: return radicalInverseT<23>(i);
-    case 9: return radicalInverseT<29>(i);
-    case 10: return radicalInverseT<31>(i);
-    case 11: return radicalInverseT<37>(i);
-    case 12: return radicalInverseT<41>(i);
-    case 13: return radicalInverseT<43>(i);
-    case 14: return radicalInverseT<47>(i);
-    default: return radicalInverseT<53>(i);
+  const HaltonBase h = c_halton[dim];
+  if (i >> 26) return radicalInverseLarge(i, h.base, h.inv);
+  float invBaseN = 1.0f;
+  uint32_t rev = 0;
+#pragma unroll 1
+  while (i > 0) {
+    const uint32_t next = __umulhi(i, h.mul);
+    rev = rev * h.base + (i - next * h.base);
+    invBaseN = __fmul_rn(invBaseN, h.inv);
+    i = next;
   }
+  const float v = __fmul_rn((float)rev, invBaseN);
+  return v < 1.0f ? v : 0.9999999f;
 }
 
 enum Slot {

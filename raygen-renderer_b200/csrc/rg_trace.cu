@@ -785,8 +785,7 @@ __device__ __forceinline__ void traverseWave8(const DevScene& S0, const DevJob* 
   __shared__ uint2 sStack[kSharedStack > 0 ? kSharedStack : 1][kTraceBlock];
   uint2 lStack[kStack8 - kSharedStack];
   // triangle queue: entries [head, tail) modulo kTriQueue, head and tail alike in all lanes
-  __shared__ int sTri[kTraceWarps][kTriQueue];
-  __shared__ uint8_t sOwner[kTraceWarps][kTriQueue];
+  __shared__ int2 sTri[kTraceWarps][kTriQueue];  // (triangle, owner lane)
   __shared__ unsigned sHits[kTraceWarps][32];  // per owner: the batch entries that hit
   int head = 0, tail = 0;
   int qEnd = 0;  // queue position after this lane's last entry
@@ -951,13 +950,12 @@ __device__ __forceinline__ void traverseWave8(const DevScene& S0, const DevJob* 
         const unsigned fit = __ballot_sync(kAll, incl <= room);  // a run of lanes from lane 0
         if (n > 0 && incl <= room) {
           int at = tail + incl - n;
-          while (tMask) {
-            sTri[warp][at & (kTriQueue - 1)] = tBase + __ffs(tMask) - 1;
-            sOwner[warp][at & (kTriQueue - 1)] = (uint8_t)lane;
+          qEnd = tail + incl;
+          do {
+            sTri[warp][at & (kTriQueue - 1)] = make_int2(tBase + __ffs(tMask) - 1, lane);
             tMask &= tMask - 1u;
             at++;
-          }
-          qEnd = at;
+          } while (tMask);
         }
         if (fit) tail += __shfl_sync(kAll, incl, 31 - __clz(fit));
         __syncwarp();
@@ -967,8 +965,8 @@ __device__ __forceinline__ void traverseWave8(const DevScene& S0, const DevJob* 
       if (queued >= 32 || (queued > 0 && __popc(readyMask) < kLowNodes)) {
         const int n = min(queued, 32);
         const bool mine = lane < n;
-        const int at = (head + (mine ? lane : 0)) & (kTriQueue - 1);
-        const int tk = sTri[warp][at], own = sOwner[warp][at];
+        const int2 entry = sTri[warp][(head + (mine ? lane : 0)) & (kTriQueue - 1)];
+        const int tk = entry.x, own = entry.y;
         const V3 ro = v3(__shfl_sync(kAll, o.x, own), __shfl_sync(kAll, o.y, own), __shfl_sync(kAll, o.z, own));
         const V3 rd = v3(__shfl_sync(kAll, d.x, own), __shfl_sync(kAll, d.y, own), __shfl_sync(kAll, d.z, own));
         const float4* base = MULTI ? reinterpret_cast<const float4*>(
@@ -1115,8 +1113,15 @@ void launchTriMaterial(const DevScene& S, int n, int* triMat, cudaStream_t st) {
 // cone / path emission, heat haze) and volume-light NEE.  Scenes without
 // those features run a smaller kernel (instruction fetch is this kernel's
 // main stall).
+// Two blocks per SM (128 registers) for every variant: left to itself the compiler gave the
+// multi-job kernel 173-222 registers, which is one block (24 jobs through the server: 64 -> 53
+// ms of device time, with 0-100 bytes of spills).  Three blocks (80 registers) spill more
+// than they hide: 43.3 -> 53.3 ms on the 4M-triangle scene.
+#ifndef RG_SHADE_MIN_BLOCKS
+#define RG_SHADE_MIN_BLOCKS 2
+#endif
 template <bool MULTI, bool ENV, int MEDL>
-__global__ void __launch_bounds__(256) k_shade(DevScene S0, DevRender R0, const DevJob* __restrict__ jobs, DevQueues Q,
+__global__ void __launch_bounds__(256, RG_SHADE_MIN_BLOCKS) k_shade(DevScene S0, DevRender R0, const DevJob* __restrict__ jobs, DevQueues Q,
                                                int iter) {
   const int count = Q.counters[iter * kCountersPerIter + C_RAYS];
   const int inB = iter & 1, outB = (iter + 1) & 1;
