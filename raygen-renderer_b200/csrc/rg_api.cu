@@ -1821,17 +1821,11 @@ rg_status rg_denoise_atrous(int32_t w, int32_t h, const float* color, const floa
   for (int i = 0; i < N; i++) c4[i] = make_float4(color[i * 3], color[i * 3 + 1], color[i * 3 + 2], 1.0f);
   DevBuf<float4> c, a, b, o;
   DevBuf<float> fn, fa, fd, faa;
-  DevBuf<__half> hn, ha, hd, haa;
   cudaStream_t st = 0;
   if (!c.upload(c4.data(), N, st) || !a.alloc(N) || !b.alloc(N) || !o.alloc(N) || !fn.upload(normal, (size_t)N * 3, st) ||
-      !fa.upload(albedo, (size_t)N * 3, st) || !fd.upload(depth, N, st) || !faa.upload(albedo_alpha, N, st) ||
-      !hn.alloc((size_t)N * 3) || !ha.alloc((size_t)N * 3) || !hd.alloc(N) || !haa.alloc(N))
+      !fa.upload(albedo, (size_t)N * 3, st) || !fd.upload(depth, N, st) || !faa.upload(albedo_alpha, N, st))
     return RG_ERR_OUT_OF_MEMORY;
-  launchFloatToHalf(N * 3, fn.p, hn.p, st);
-  launchFloatToHalf(N * 3, fa.p, ha.p, st);
-  launchFloatToHalf(N, fd.p, hd.p, st);
-  launchFloatToHalf(N, faa.p, haa.p, st);
-  launchDenoise(w, h, c.p, hn.p, hd.p, ha.p, haa.p, levels, sigma_color, sigma_normal, sigma_depth, intensity, a.p, b.p,
+  launchDenoise(w, h, c.p, fn.p, fd.p, fa.p, faa.p, levels, sigma_color, sigma_normal, sigma_depth, intensity, a.p, b.p,
                 o.p, st);
   RG_CUDA_CHECK(cudaMemcpy(c4.data(), o.p, sizeof(float4) * N, cudaMemcpyDeviceToHost));
   for (int i = 0; i < N; i++) { out[i * 3] = c4[i].x; out[i * 3 + 1] = c4[i].y; out[i * 3 + 2] = c4[i].z; }

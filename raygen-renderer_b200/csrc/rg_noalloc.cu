@@ -12,8 +12,8 @@
 // statically sized __device__ array of this module, so a call makes no
 // cudaMalloc / cudaFree / allocating-library call of any kind.
 //
-// It runs exactly the kernels of rg_denoise_atrous (float -> half guide
-// conversion, firefly pre-clamp + albedo demodulation, the A-Trous levels,
+// It runs exactly the kernels of rg_denoise_atrous (firefly pre-clamp + albedo
+// demodulation with the guides rounded to half precision, the A-Trous levels,
 // remodulation), so the two agree bit for bit on the same inputs.
 //
 // Limits and rules (also stated in the C header):
@@ -48,20 +48,13 @@ namespace rg {
 namespace {
 
 constexpr size_t kMaxPixels = size_t(1) << 20;
-// Layout of the working array, each part 256-byte aligned:
-//   two float4 ping-pong colour buffers, then the half guides
-//   (normal x3, albedo x3, depth, albedo alpha).
+// Layout of the working array: two float4 ping-pong colour buffers (the packed
+// guides lie in the caller's output buffer until the last pass writes it).
 constexpr size_t kColourBytes = kMaxPixels * sizeof(float4);
 constexpr size_t kOffA = 0;
 constexpr size_t kOffB = kOffA + kColourBytes;
-constexpr size_t kOffNormal = kOffB + kColourBytes;
-constexpr size_t kOffAlbedo = kOffNormal + kMaxPixels * 3 * sizeof(__half);
-constexpr size_t kOffDepth = kOffAlbedo + kMaxPixels * 3 * sizeof(__half);
-constexpr size_t kOffAlbedoA = kOffDepth + kMaxPixels * sizeof(__half);
-constexpr size_t kScratchBytes = kOffAlbedoA + kMaxPixels * sizeof(__half);  // 48 MiB
-static_assert(kOffB % 256 == 0 && kOffNormal % 256 == 0 && kOffAlbedo % 256 == 0 && kOffDepth % 256 == 0 &&
-                  kOffAlbedoA % 256 == 0,
-              "working buffer parts must stay 256-byte aligned");
+constexpr size_t kScratchBytes = kOffB + kColourBytes;  // 32 MiB
+static_assert(kOffB % 256 == 0, "working buffer parts must stay 256-byte aligned");
 
 static __device__ __align__(256) unsigned char g_atrousScratch[kScratchBytes];
 
@@ -254,17 +247,8 @@ extern "C" rg_status rg_denoise_atrous_noalloc(int32_t w, int32_t h, const float
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   float4* bufA = reinterpret_cast<float4*>(s + kOffA);
   float4* bufB = reinterpret_cast<float4*>(s + kOffB);
-  __half* hn = reinterpret_cast<__half*>(s + kOffNormal);
-  __half* ha = reinterpret_cast<__half*>(s + kOffAlbedo);
-  __half* hd = reinterpret_cast<__half*>(s + kOffDepth);
-  __half* haa = reinterpret_cast<__half*>(s + kOffAlbedoA);
-  const int N = (int)n;
-  launchFloatToHalf(N * 3, normal, hn, st);
-  launchFloatToHalf(N * 3, albedo, ha, st);
-  launchFloatToHalf(N, depth, hd, st);
-  launchFloatToHalf(N, albedo_alpha, haa, st);
-  launchDenoise(w, h, reinterpret_cast<const float4*>(color_rgba), hn, hd, ha, haa, levels, sigma_color, sigma_normal,
-                sigma_depth, intensity, bufA, bufB, reinterpret_cast<float4*>(out_rgba), st);
+  launchDenoise(w, h, reinterpret_cast<const float4*>(color_rgba), normal, depth, albedo, albedo_alpha, levels,
+                sigma_color, sigma_normal, sigma_depth, intensity, bufA, bufB, reinterpret_cast<float4*>(out_rgba), st);
   const cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) {
     setLastError(std::string("rg_denoise_atrous_noalloc: launch failed: ") + cudaGetErrorString(e));

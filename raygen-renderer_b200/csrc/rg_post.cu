@@ -33,9 +33,21 @@ __global__ void k_resolve(int n, const float4* __restrict__ sum, const int* __re
                        fmaxf(s.z * invN * exposure, 0.0f), 1.0f);
 }
 
-// Firefly pre-clamp + albedo demodulation (rayrenderer.cpp:2685-2722).
-__global__ void k_prepass(int w, int h, const float4* __restrict__ noisy, const __half* __restrict__ albedo,
-                          const __half* __restrict__ albedoA, float4* __restrict__ out) {
+// A guide value as the filter sees it: half precision, whether it is stored as a half
+// (the renderer's guides) or as a float (the callers' of the A-Trous entry points).
+__device__ __forceinline__ __half guideHalf(__half v) { return v; }
+__device__ __forceinline__ __half guideHalf(float v) { return __float2half(v); }
+template <typename T>
+__device__ __forceinline__ float guideAt(const T* g, int i) { return __half2float(guideHalf(g[i])); }
+
+// Firefly pre-clamp + albedo demodulation (rayrenderer.cpp:2685-2722), and what the
+// levels read per tap: the colour with its luminance in w, and the normal and depth
+// guides as one 8-byte word.
+template <typename T>
+__global__ void __launch_bounds__(256) k_prepass(int w, int h, const float4* __restrict__ noisy, const T* __restrict__ normal,
+                                                 const T* __restrict__ depth, const T* __restrict__ albedo,
+                                                 const T* __restrict__ albedoA, float4* __restrict__ out,
+                                                 uint2* __restrict__ guide) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= w * h) return;
   const int x = i % w, y = i / w;
@@ -59,68 +71,105 @@ __global__ void k_prepass(int w, int h, const float4* __restrict__ noisy, const 
     const float s = cap / cl;
     c.x *= s; c.y *= s; c.z *= s;
   }
-  if (__half2float(albedoA[i]) > 0.5f) {
-    const float ar = fmaxf(__half2float(albedo[i * 3]), 0.3f), ag = fmaxf(__half2float(albedo[i * 3 + 1]), 0.3f),
-                ab = fmaxf(__half2float(albedo[i * 3 + 2]), 0.3f);
-    out[i] = make_float4(fminf(c.x / ar, 3.0f), fminf(c.y / ag, 3.0f), fminf(c.z / ab, 3.0f), 1.0f);
-  } else {
-    out[i] = c;
+  if (guideAt(albedoA, i) > 0.5f) {
+    const float ar = fmaxf(guideAt(albedo, i * 3), 0.3f), ag = fmaxf(guideAt(albedo, i * 3 + 1), 0.3f),
+                ab = fmaxf(guideAt(albedo, i * 3 + 2), 0.3f);
+    c = make_float4(fminf(c.x / ar, 3.0f), fminf(c.y / ag, 3.0f), fminf(c.z / ab, 3.0f), 1.0f);
   }
+  c.w = lum3(c.x, c.y, c.z);
+  out[i] = c;
+  const __half2 g0 = __halves2half2(guideHalf(normal[i * 3]), guideHalf(normal[i * 3 + 1]));
+  const __half2 g1 = __halves2half2(guideHalf(normal[i * 3 + 2]), guideHalf(depth[i]));
+  guide[i] = make_uint2(*reinterpret_cast<const uint32_t*>(&g0), *reinterpret_cast<const uint32_t*>(&g1));
 }
 
-// One edge-avoiding A-Trous level (rayrenderer.cpp:2536-2608).
-__global__ void __launch_bounds__(256) k_atrous(int w, int h, const float4* __restrict__ src, float4* __restrict__ dst,
-                                                const __half* __restrict__ normal, const __half* __restrict__ depth,
-                                                int step, float invC2, float sigN, float dScale) {
-  const int x = blockIdx.x * blockDim.x + threadIdx.x;
-  const int y = blockIdx.y * blockDim.y + threadIdx.y;
-  if (x >= w || y >= h) return;
+struct Guide {
+  float nx, ny, nz, d;
+};
+__device__ __forceinline__ Guide unpackGuide(uint2 u) {
+  const float2 a = __half22float2(*reinterpret_cast<const __half2*>(&u.x)), b = __half22float2(*reinterpret_cast<const __half2*>(&u.y));
+  return Guide{a.x * 2.0f - 1.0f, a.y * 2.0f - 1.0f, b.x * 2.0f - 1.0f, b.y};
+}
+// Base-2 logarithm and exponential, denormals as zero: a dot of half normals is zero or at
+// least 2^-48, and a weight below 2^-126 adds nothing to sums that count (> 1e-8).
+__device__ __forceinline__ float lg2Ftz(float x) {
+  float y;
+  asm("lg2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+  return y;
+}
+__device__ __forceinline__ float ex2Ftz(float x) {
+  float y;
+  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+  return y;
+}
+
+// One edge-avoiding A-Trous level (rayrenderer.cpp:2536-2608).  Bound by the instructions
+// of its 25 taps (about 30 each) and their L1 reads; a tap is one 16-byte and one 8-byte
+// load (five loads when normal and depth came as separate half arrays).  A block whose taps
+// all lie inside the image skips the bounds of each tap.
+template <bool INSIDE>
+__device__ __forceinline__ void atrousPixel(int w, int h, int x, int y, const float4* __restrict__ src, float4* __restrict__ dst,
+                                            const uint2* __restrict__ guide, int step, float invC2, float sigN, float dScale) {
   const float kw[5] = {1.0f / 16.0f, 1.0f / 4.0f, 3.0f / 8.0f, 1.0f / 4.0f, 1.0f / 16.0f};
   const int ci = y * w + x;
   const float4 cc = src[ci];
-  const float cnx = __half2float(normal[ci * 3]) * 2.0f - 1.0f, cny = __half2float(normal[ci * 3 + 1]) * 2.0f - 1.0f,
-              cnz = __half2float(normal[ci * 3 + 2]) * 2.0f - 1.0f;
-  const float cd = __half2float(depth[ci]);
-  const float cl = lum3(cc.x, cc.y, cc.z);
+  const Guide cg = unpackGuide(guide[ci]);
   float sx = 0, sy = 0, sz = 0, ws = 0;
+#pragma unroll
   for (int ky = 0; ky < 5; ++ky) {
     const int ny = y + (ky - 2) * step;
-    if (ny < 0 || ny >= h) continue;
+    if (!INSIDE && (ny < 0 || ny >= h)) continue;
+#pragma unroll
     for (int kx = 0; kx < 5; ++kx) {
       const int nx = x + (kx - 2) * step;
-      if (nx < 0 || nx >= w) continue;
+      if (!INSIDE && (nx < 0 || nx >= w)) continue;
       const int si = ny * w + nx;
       const float4 sc = __ldg(&src[si]);
-      const float snx = __half2float(normal[si * 3]) * 2.0f - 1.0f, sny = __half2float(normal[si * 3 + 1]) * 2.0f - 1.0f,
-                  snz = __half2float(normal[si * 3 + 2]) * 2.0f - 1.0f;
-      const float sl = lum3(sc.x, sc.y, sc.z);
-      const float ld = sl - cl;
-      float nd = snx * cnx + sny * cny + snz * cnz;
+      const Guide sg = unpackGuide(__ldg(&guide[si]));
+      const float ld = sc.w - cc.w;
+      float nd = sg.nx * cg.nx + sg.ny * cg.ny + sg.nz * cg.nz;
       if (nd < 0.0f) nd = 0.0f;
       // exp(-ld^2 / 2sc^2) * max(n.n', 0)^sigN * exp(-|dd| / (sd step)) as one
       // base-2 exponential of the summed logarithms (powf(0, 0) = 1 kept)
-      const float lnC = -(ld * ld) * invC2 - fabsf(__half2float(depth[si]) - cd) * dScale;
-      const float lg2N = sigN == 0.0f ? 0.0f : (nd > 0.0f ? sigN * __log2f(nd) : -INFINITY);
-      const float wgt = kw[kx] * kw[ky] * exp2f(fmaf(lnC, 1.44269504088896341f, lg2N));
+      const float lnC = -(ld * ld) * invC2 - fabsf(sg.d - cg.d) * dScale;
+      const float lg2N = sigN == 0.0f ? 0.0f : (nd > 0.0f ? sigN * lg2Ftz(nd) : -INFINITY);
+      const float wgt = kw[kx] * kw[ky] * ex2Ftz(fmaf(lnC, 1.44269504088896341f, lg2N));
       sx += sc.x * wgt; sy += sc.y * wgt; sz += sc.z * wgt;
       ws += wgt;
     }
   }
-  dst[ci] = ws > 1e-8f ? make_float4(sx / ws, sy / ws, sz / ws, cc.w) : cc;
+  float4 r = cc;
+  if (ws > 1e-8f) {
+    r = make_float4(sx / ws, sy / ws, sz / ws, 0.0f);
+    r.w = lum3(r.x, r.y, r.z);
+  }
+  dst[ci] = r;
+}
+
+__global__ void __launch_bounds__(256) k_atrous(int w, int h, const float4* __restrict__ src, float4* __restrict__ dst,
+                                                const uint2* __restrict__ guide, int step, float invC2, float sigN,
+                                                float dScale) {
+  const int x0 = blockIdx.x * blockDim.x, y0 = blockIdx.y * blockDim.y;
+  const int x = x0 + threadIdx.x, y = y0 + threadIdx.y;
+  const int r = 2 * step;
+  if (x0 >= r && y0 >= r && x0 + (int)blockDim.x + r <= w && y0 + (int)blockDim.y + r <= h)
+    atrousPixel<true>(w, h, x, y, src, dst, guide, step, invC2, sigN, dScale);
+  else if (x < w && y < h)
+    atrousPixel<false>(w, h, x, y, src, dst, guide, step, invC2, sigN, dScale);
 }
 
 // Remodulate and blend with the noisy input (rayrenderer.cpp:2752-2771).
-__global__ void k_remod(int n, const float4* __restrict__ filtered, const float4* __restrict__ noisy,
-                        const __half* __restrict__ albedo, const __half* __restrict__ albedoA, float intensity,
-                        float4* __restrict__ out) {
+template <typename T>
+__global__ void __launch_bounds__(256) k_remod(int n, const float4* __restrict__ filtered, const float4* __restrict__ noisy,
+                                               const T* __restrict__ albedo, const T* __restrict__ albedoA, float intensity,
+                                               float4* __restrict__ out) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
   const float t = fminf(fmaxf(intensity, 0.0f), 1.0f), s = 1.0f - t;
   const float4 f = filtered[i], nz = noisy[i];
   float4 r = f;
-  if (__half2float(albedoA[i]) > 0.5f)
-    r = make_float4(f.x * __half2float(albedo[i * 3]), f.y * __half2float(albedo[i * 3 + 1]),
-                    f.z * __half2float(albedo[i * 3 + 2]), 1.0f);
+  if (guideAt(albedoA, i) > 0.5f)
+    r = make_float4(f.x * guideAt(albedo, i * 3), f.y * guideAt(albedo, i * 3 + 1), f.z * guideAt(albedo, i * 3 + 2), 1.0f);
   out[i] = make_float4(nz.x * s + r.x * t, nz.y * s + r.y * t, nz.z * s + r.z * t, 1.0f);
 }
 
@@ -233,10 +282,6 @@ __global__ void k_h2f(int n, const __half* in, float* out) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i < n) out[i] = __half2float(in[i]);
 }
-__global__ void k_f2h(int n, const float* in, __half* out) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i < n) out[i] = __float2half(in[i]);
-}
 
 inline int g256(int n) { return (n + 255) / 256; }
 
@@ -340,11 +385,14 @@ void launchResolve(int n, const float4* sum, const int* cnt, float exposure, flo
   k_resolve<<<g256(n), 256, 0, st>>>(n, sum, cnt, exposure, hdr);
 }
 
-void launchDenoise(int w, int h, const float4* noisy, const __half* normal, const __half* depth, const __half* albedo,
-                   const __half* albedoA, int levels, float sigC, float sigN, float sigD, float intensity,
-                   float4* bufA, float4* bufB, float4* out, cudaStream_t st) {
+// The packed guides (8 bytes a pixel) lie in `out` until the last pass writes it.
+template <typename T>
+static void denoisePasses(int w, int h, const float4* noisy, const T* normal, const T* depth, const T* albedo,
+                          const T* albedoA, int levels, float sigC, float sigN, float sigD, float intensity, float4* bufA,
+                          float4* bufB, float4* out, cudaStream_t st) {
   const int n = w * h;
-  k_prepass<<<g256(n), 256, 0, st>>>(w, h, noisy, albedo, albedoA, bufA);
+  uint2* guide = reinterpret_cast<uint2*>(out);
+  k_prepass<<<g256(n), 256, 0, st>>>(w, h, noisy, normal, depth, albedo, albedoA, bufA, guide);
   float4* src = bufA;
   float4* dst = bufB;
   const float invC2 = 1.0f / (2.0f * sigC * sigC + 1e-8f);
@@ -352,12 +400,24 @@ void launchDenoise(int w, int h, const float4* noisy, const __half* normal, cons
   for (int l = 0; l < (levels < 1 ? 1 : levels); ++l) {
     const int step = 1 << l;
     const float dScale = 1.0f / (sigD * (float)step + 1e-8f);
-    k_atrous<<<grd, blk, 0, st>>>(w, h, src, dst, normal, depth, step, invC2, sigN, dScale);
+    k_atrous<<<grd, blk, 0, st>>>(w, h, src, dst, guide, step, invC2, sigN, dScale);
     float4* t = src;
     src = dst;
     dst = t;
   }
   k_remod<<<g256(n), 256, 0, st>>>(n, src, noisy, albedo, albedoA, intensity, out);
+}
+
+void launchDenoise(int w, int h, const float4* noisy, const __half* normal, const __half* depth, const __half* albedo,
+                   const __half* albedoA, int levels, float sigC, float sigN, float sigD, float intensity,
+                   float4* bufA, float4* bufB, float4* out, cudaStream_t st) {
+  denoisePasses(w, h, noisy, normal, depth, albedo, albedoA, levels, sigC, sigN, sigD, intensity, bufA, bufB, out, st);
+}
+
+void launchDenoise(int w, int h, const float4* noisy, const float* normal, const float* depth, const float* albedo,
+                   const float* albedoA, int levels, float sigC, float sigN, float sigD, float intensity,
+                   float4* bufA, float4* bufB, float4* out, cudaStream_t st) {
+  denoisePasses(w, h, noisy, normal, depth, albedo, albedoA, levels, sigC, sigN, sigD, intensity, bufA, bufB, out, st);
 }
 
 void launchTonemap(int n, const float4* hdr, float4* ldr, cudaStream_t st) { k_tonemap<<<g256(n), 256, 0, st>>>(n, hdr, ldr); }
@@ -416,6 +476,5 @@ void launchAdaptiveTiles(int w, int h, const float4* sum, const float4* sumSq, c
 }
 
 void launchHalfToFloat(int n, const __half* in, float* out, cudaStream_t st) { k_h2f<<<g256(n), 256, 0, st>>>(n, in, out); }
-void launchFloatToHalf(int n, const float* in, __half* out, cudaStream_t st) { k_f2h<<<g256(n), 256, 0, st>>>(n, in, out); }
 
 }  // namespace rg

@@ -44,6 +44,10 @@ void launchResolve(int n, const float4* sum, const int* cnt, float exposure, flo
 void launchDenoise(int w, int h, const float4* noisy, const __half* normal, const __half* depth, const __half* albedo,
                    const __half* albedoA, int levels, float sigC, float sigN, float sigD, float intensity,
                    float4* bufA, float4* bufB, float4* out, cudaStream_t st);
+// the same with float guides, rounded to half precision as they are read
+void launchDenoise(int w, int h, const float4* noisy, const float* normal, const float* depth, const float* albedo,
+                   const float* albedoA, int levels, float sigC, float sigN, float sigD, float intensity,
+                   float4* bufA, float4* bufB, float4* out, cudaStream_t st);
 void launchTonemap(int n, const float4* hdr, float4* ldr, cudaStream_t st);
 // HDR bloom: glow buffer size and the normalised Gaussian taps (host), then
 // extract + area downsample, 2 x (horizontal, vertical) blur, upsample + add.
@@ -60,6 +64,5 @@ void launchAdaptivePixels(int n, const float4* sum, const float4* sumSq, const i
 void launchAdaptiveTiles(int w, int h, const float4* sum, const float4* sumSq, const int* cnt, int target,
                          float threshold, int* list, int* outCount, cudaStream_t st);
 void launchHalfToFloat(int n, const __half* in, float* out, cudaStream_t st);
-void launchFloatToHalf(int n, const float* in, __half* out, cudaStream_t st);
 
 }  // namespace rg
