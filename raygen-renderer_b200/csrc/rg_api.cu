@@ -13,6 +13,7 @@
 #include <chrono>
 #include <condition_variable>
 #include <climits>
+#include <functional>
 #include <cstdlib>
 #include <unordered_map>
 #include <cmath>
@@ -278,7 +279,28 @@ void buildMedia(const rg_scene_desc* d, const Mat4& view, MediaTables& T) {
 
 using namespace rg;
 
+// Buffers of the ray-batch queries, kept between calls: allocating and freeing them took a
+// third of a 1000-ray query.  Inputs and outputs lie in one device array each, so a batch of
+// up to kSmall rays is one copy in and one out through a page-locked array (a larger one is
+// copied from and to the caller's arrays).  More than 64 MB are given back after the call.
+struct QueryBuffers {
+  static constexpr int kSmall = 8192;
+  static constexpr size_t kHostBytes = (size_t)kSmall * 28 + 16;  // 7 floats in; 4 words and the error word out
+  DevBuf<float> in;   // rays (6 n), tmax (n)
+  DevBuf<float> out;  // the error word, then t, u, v (3 n) and triangle (n), or a byte per ray
+  unsigned char* host = nullptr;
+  ~QueryBuffers() {
+    if (host) cudaFreeHost(host);
+  }
+  void trim() {
+    if (in.bytes() + out.bytes() <= (size_t(64) << 20)) return;
+    in.release();
+    out.release();
+  }
+};
+
 struct rg_handle {
+  StageUser stage;
   rg_settings st;
   std::mutex mu;
   cudaStream_t stream = nullptr;
@@ -295,6 +317,7 @@ struct rg_handle {
   rg_denoiser* denoiser = nullptr;           // learned denoiser (NULL: A-Trous)
   DevBuf<float> bloomW;                     // Gaussian taps
   DevBuf<int> cnt, pixelList, listCount;
+  QueryBuffers query;
   DevBuf<__half> aovNormal, aovAlbedo, aovAlbedoA, aovDepth;
   int W = 0, H = 0;
   bool haveResult = false;
@@ -611,6 +634,10 @@ rg_status rg_create(const rg_settings* s, rg_handle** out) {
     setLastError("cudaStreamCreate failed");
     delete h;
     return RG_ERR_CUDA;
+  }
+  if (cudaHostAlloc((void**)&h->query.host, QueryBuffers::kHostBytes, cudaHostAllocDefault) != cudaSuccess) {
+    cudaGetLastError();  // small queries copy from and to the caller's arrays then
+    h->query.host = nullptr;
   }
   *out = h;
   return RG_OK;
@@ -1630,7 +1657,7 @@ rg_status rg_get_hdr(rg_handle* h, float* rgba, size_t count) {
   std::lock_guard<std::mutex> lk(h->mu);
   if (!h->haveResult) return RG_ERR_NO_SCENE;
   if (count < (size_t)h->W * h->H * 4) return RG_ERR_INVALID_ARGUMENT;
-  RG_CUDA_CHECK(cudaMemcpy(rgba, h->hdr.p, sizeof(float4) * h->W * h->H, cudaMemcpyDeviceToHost));
+  RG_CUDA_CHECK(copyToHost(rgba, h->hdr.p, sizeof(float4) * h->W * h->H, h->stream));
   return RG_OK;
 }
 
@@ -1639,7 +1666,7 @@ rg_status rg_get_ldr(rg_handle* h, float* rgba, size_t count) {
   std::lock_guard<std::mutex> lk(h->mu);
   if (!h->haveResult) return RG_ERR_NO_SCENE;
   if (count < (size_t)h->W * h->H * 4) return RG_ERR_INVALID_ARGUMENT;
-  RG_CUDA_CHECK(cudaMemcpy(rgba, h->ldr.p, sizeof(float4) * h->W * h->H, cudaMemcpyDeviceToHost));
+  RG_CUDA_CHECK(copyToHost(rgba, h->ldr.p, sizeof(float4) * h->W * h->H, h->stream));
   return RG_OK;
 }
 
@@ -1653,18 +1680,15 @@ rg_status rg_get_aovs(rg_handle* h, float* normal, float* albedo, float* depth, 
   if (!tmp.alloc((size_t)N * 3)) return RG_ERR_OUT_OF_MEMORY;
   if (normal) {
     launchHalfToFloat(N * 3, h->aovNormal.p, tmp.p, h->stream);
-    RG_CUDA_CHECK(cudaMemcpyAsync(normal, tmp.p, sizeof(float) * N * 3, cudaMemcpyDeviceToHost, h->stream));
-    RG_CUDA_CHECK(cudaStreamSynchronize(h->stream));
+    RG_CUDA_CHECK(copyToHost(normal, tmp.p, sizeof(float) * N * 3, h->stream));
   }
   if (albedo) {
     launchHalfToFloat(N * 3, h->aovAlbedo.p, tmp.p, h->stream);
-    RG_CUDA_CHECK(cudaMemcpyAsync(albedo, tmp.p, sizeof(float) * N * 3, cudaMemcpyDeviceToHost, h->stream));
-    RG_CUDA_CHECK(cudaStreamSynchronize(h->stream));
+    RG_CUDA_CHECK(copyToHost(albedo, tmp.p, sizeof(float) * N * 3, h->stream));
   }
   if (depth) {
     launchHalfToFloat(N, h->aovDepth.p, tmp.p, h->stream);
-    RG_CUDA_CHECK(cudaMemcpyAsync(depth, tmp.p, sizeof(float) * N, cudaMemcpyDeviceToHost, h->stream));
-    RG_CUDA_CHECK(cudaStreamSynchronize(h->stream));
+    RG_CUDA_CHECK(copyToHost(depth, tmp.p, sizeof(float) * N, h->stream));
   }
   return RG_OK;
 }
@@ -1674,7 +1698,7 @@ rg_status rg_get_sample_counts(rg_handle* h, int32_t* counts, size_t count) {
   std::lock_guard<std::mutex> lk(h->mu);
   if (!h->haveResult) return RG_ERR_NO_SCENE;
   if (count < (size_t)h->W * h->H) return RG_ERR_INVALID_ARGUMENT;
-  RG_CUDA_CHECK(cudaMemcpy(counts, h->cnt.p, sizeof(int) * h->W * h->H, cudaMemcpyDeviceToHost));
+  RG_CUDA_CHECK(copyToHost(counts, h->cnt.p, sizeof(int) * h->W * h->H, h->stream));
   return RG_OK;
 }
 
@@ -1753,21 +1777,44 @@ rg_status rg_get_view_matrix(rg_handle* h, float* m16) {
   return RG_OK;
 }
 
-rg_status rg_trace_closest(rg_handle* h, const float* rays, int32_t n, float* out_tuv, int32_t* out_prim) {
-  if (!h || n < 0 || (n > 0 && (!rays || !out_tuv || !out_prim))) return RG_ERR_INVALID_ARGUMENT;
-  std::lock_guard<std::mutex> lk(h->mu);
-  if (!h->hasScene) return RG_ERR_NO_SCENE;
-  if (n == 0) return RG_OK;
-  DevBuf<float> r, t;
-  DevBuf<int> p;
-  if (!r.upload(rays, (size_t)n * 6, h->stream) || !t.alloc((size_t)n * 3) || !p.alloc(n)) return RG_ERR_OUT_OF_MEMORY;
-  RG_CUDA_CHECK(cudaMemsetAsync(h->error.p, 0, sizeof(int), h->stream));  // this query's flag only
-  launchQueryClosest(h->dscene, r.p, n, t.p, p.p, h->stream);
-  RG_CUDA_CHECK(cudaMemcpyAsync(out_tuv, t.p, sizeof(float) * n * 3, cudaMemcpyDeviceToHost, h->stream));
-  RG_CUDA_CHECK(cudaMemcpyAsync(out_prim, p.p, sizeof(int) * n, cudaMemcpyDeviceToHost, h->stream));
+// One batch query: `rays` (and `tmax`) in, `launch(in, out)` on h->stream, then the results
+// at word 1 of the output array in two parts (host array, bytes).
+static rg_status runQuery(rg_handle* h, const float* rays, const float* tmax, int n, size_t outWords,
+                          const std::function<void(const float*, float*)>& launch, void* out0, size_t bytes0, void* out1,
+                          size_t bytes1) {
+  QueryBuffers& b = h->query;
+  const size_t inWords = (size_t)n * (tmax ? 7 : 6);
+  if (!b.in.alloc(inWords) || !b.out.alloc(1 + outWords)) {
+    b.trim();
+    return RG_ERR_OUT_OF_MEMORY;
+  }
+  const bool small = n <= QueryBuffers::kSmall && b.host;
+  cudaStream_t st = h->stream;
   int derr = 0;
-  RG_CUDA_CHECK(cudaMemcpyAsync(&derr, h->error.p, sizeof(int), cudaMemcpyDeviceToHost, h->stream));
-  RG_CUDA_CHECK(cudaStreamSynchronize(h->stream));
+  RG_CUDA_CHECK(cudaMemsetAsync(h->error.p, 0, sizeof(int), st));  // this query's flag only
+  if (small) {
+    std::memcpy(b.host, rays, sizeof(float) * 6 * n);
+    if (tmax) std::memcpy(b.host + sizeof(float) * 6 * n, tmax, sizeof(float) * n);
+    RG_CUDA_CHECK(cudaMemcpyAsync(b.in.p, b.host, sizeof(float) * inWords, cudaMemcpyHostToDevice, st));
+  } else {
+    RG_CUDA_CHECK(copyToDevice(b.in.p, rays, sizeof(float) * 6 * n, st));
+    if (tmax) RG_CUDA_CHECK(copyToDevice(b.in.p + (size_t)6 * n, tmax, sizeof(float) * n, st));
+  }
+  launch(b.in.p, b.out.p + 1);
+  RG_CUDA_CHECK(cudaMemcpyAsync(b.out.p, h->error.p, sizeof(int), cudaMemcpyDeviceToDevice, st));
+  if (small) {
+    RG_CUDA_CHECK(cudaMemcpyAsync(b.host, b.out.p, sizeof(int) + bytes0 + bytes1, cudaMemcpyDeviceToHost, st));
+    RG_CUDA_CHECK(cudaStreamSynchronize(st));
+    std::memcpy(&derr, b.host, sizeof(int));
+    std::memcpy(out0, b.host + sizeof(int), bytes0);
+    if (bytes1) std::memcpy(out1, b.host + sizeof(int) + bytes0, bytes1);
+  } else {
+    const unsigned char* o = reinterpret_cast<const unsigned char*>(b.out.p + 1);
+    RG_CUDA_CHECK(copyToHost(out0, o, bytes0, st));
+    if (bytes1) RG_CUDA_CHECK(copyToHost(out1, o + bytes0, bytes1, st));
+    RG_CUDA_CHECK(copyToHost(&derr, b.out.p, sizeof(int), st));
+    b.trim();
+  }
   if (derr) {
     setLastError("device error flag raised: " + std::to_string(derr));
     return RG_ERR_DEVICE_STATUS;
@@ -1775,27 +1822,32 @@ rg_status rg_trace_closest(rg_handle* h, const float* rays, int32_t n, float* ou
   return RG_OK;
 }
 
+rg_status rg_trace_closest(rg_handle* h, const float* rays, int32_t n, float* out_tuv, int32_t* out_prim) {
+  if (!h || n < 0 || (n > 0 && (!rays || !out_tuv || !out_prim))) return RG_ERR_INVALID_ARGUMENT;
+  std::lock_guard<std::mutex> lk(h->mu);
+  if (!h->hasScene) return RG_ERR_NO_SCENE;
+  if (n == 0) return RG_OK;
+  return runQuery(
+      h, rays, nullptr, n, (size_t)n * 4,
+      [&](const float* in, float* out) {
+        launchQueryClosest(h->dscene, in, n, out, reinterpret_cast<int*>(out + (size_t)3 * n), h->stream);
+      },
+      out_tuv, sizeof(float) * 3 * n, out_prim, sizeof(int) * n);
+}
+
 rg_status rg_trace_any(rg_handle* h, const float* rays, const float* tmax, int32_t n, int32_t predicate, uint8_t* out) {
   if (!h || n < 0 || predicate < 0 || predicate > 4 || (n > 0 && (!rays || !tmax || !out))) return RG_ERR_INVALID_ARGUMENT;
   std::lock_guard<std::mutex> lk(h->mu);
   if (!h->hasScene) return RG_ERR_NO_SCENE;
   if (n == 0) return RG_OK;
-  DevBuf<float> r, tm;
-  DevBuf<uint8_t> o;
-  if (!r.upload(rays, (size_t)n * 6, h->stream) || !tm.upload(tmax, n, h->stream) || !o.alloc(n)) return RG_ERR_OUT_OF_MEMORY;
   const uint32_t occs[5] = {kOccArea, kOccPoint, kOccAO, kOccAll, kOccVol};
   const uint32_t occ = occs[predicate];
-  RG_CUDA_CHECK(cudaMemsetAsync(h->error.p, 0, sizeof(int), h->stream));  // this query's flag only
-  launchQueryAny(h->dscene, r.p, tm.p, n, occ, o.p, h->stream);
-  RG_CUDA_CHECK(cudaMemcpyAsync(out, o.p, n, cudaMemcpyDeviceToHost, h->stream));
-  int derr = 0;
-  RG_CUDA_CHECK(cudaMemcpyAsync(&derr, h->error.p, sizeof(int), cudaMemcpyDeviceToHost, h->stream));
-  RG_CUDA_CHECK(cudaStreamSynchronize(h->stream));
-  if (derr) {
-    setLastError("device error flag raised: " + std::to_string(derr));
-    return RG_ERR_DEVICE_STATUS;
-  }
-  return RG_OK;
+  return runQuery(
+      h, rays, tmax, n, ((size_t)n + 3) / 4,
+      [&](const float* in, float* o) {
+        launchQueryAny(h->dscene, in, in + (size_t)6 * n, n, occ, reinterpret_cast<uint8_t*>(o), h->stream);
+      },
+      out, n, nullptr, 0);
 }
 
 rg_status rg_denoise_atrous(int32_t w, int32_t h, const float* color, const float* normal, const float* depth,

@@ -39,6 +39,20 @@ struct DevTexture;
 void keepPoolMemory();
 void trimPoolMemory();
 
+// Copies between the caller's memory and the device (rg_stage.cpp): large ones from or to
+// pageable memory are made by several host threads through page-locked slots.  The copy
+// comes after the work already on `after`.  copyToHost returns when dst holds the bytes;
+// copyToDevice when src may be changed, with work later put on `after` behind the copy.
+cudaError_t copyToHost(void* dst, const void* devSrc, size_t bytes, cudaStream_t after);
+cudaError_t copyToDevice(void* devDst, const void* src, size_t bytes, cudaStream_t after);
+// Held by each renderer and denoiser: the pooled slots live as long as any does.
+struct StageUser {
+  StageUser();
+  ~StageUser();
+  StageUser(const StageUser&) = delete;
+  StageUser& operator=(const StageUser&) = delete;
+};
+
 // Owning device allocation from the stream-ordered pool.  Allocation and free
 // are ordered on the calling thread's per-thread stream, so releasing a buffer
 // does not synchronise the device; callers release a buffer only after the
@@ -77,7 +91,7 @@ struct DevBuf {
   }
   bool upload(const T* src, size_t count, cudaStream_t st) {
     if (!alloc(count)) return false;
-    if (count && src) return cudaMemcpyAsync(p, src, count * sizeof(T), cudaMemcpyHostToDevice, st) == cudaSuccess;
+    if (count && src) return copyToDevice(p, src, count * sizeof(T), st) == cudaSuccess;
     return true;
   }
 };

@@ -718,6 +718,7 @@ __global__ void k_blend(int n, const float4* __restrict__ noisy, const float4* _
 }  // namespace
 
 struct KpcnNet {
+  StageUser stage;
   std::mutex mu;  // one user of the work buffers at a time (renderers, servers, API calls)
   cudaStream_t st = nullptr;
   int numSMs = 148;
@@ -1016,8 +1017,8 @@ bool uploadInputs(KpcnNet& n, size_t P, const float* noisy, const float* normal,
                   float spp, const float* ref) {
   DevBuf<float> nb, ab, db;
   if (!nb.upload(normal, P * 3, n.st) || !ab.upload(albedo, P * 3, n.st) || !db.upload(depth, P, n.st)) return false;
-  if (cudaMemcpyAsync(n.noisy.p, noisy, sizeof(float4) * P, cudaMemcpyHostToDevice, n.st) != cudaSuccess) return false;
-  if (ref && cudaMemcpyAsync(n.ref.p, ref, sizeof(float4) * P, cudaMemcpyHostToDevice, n.st) != cudaSuccess) return false;
+  if (copyToDevice(n.noisy.p, noisy, sizeof(float4) * P, n.st) != cudaSuccess) return false;
+  if (ref && copyToDevice(n.ref.p, ref, sizeof(float4) * P, n.st) != cudaSuccess) return false;
   k_features<float><<<(unsigned)((P + 255) / 256), 256, 0, n.st>>>((int)P, n.noisy.p, nb.p, ab.p, db.p, nullptr, spp,
                                                                    n.X0.p);
   return cudaStreamSynchronize(n.st) == cudaSuccess;  // the temporaries die here
@@ -1293,7 +1294,7 @@ rg_status rg_denoiser_apply(rg_denoiser* d, int32_t w, int32_t h, const float* n
   cudaEventDestroy(e0);
   cudaEventDestroy(e1);
   if (rs != RG_OK) return rs;
-  RG_CUDA_CHECK(cudaMemcpy(out_rgba, n.out.p, sizeof(float4) * P, cudaMemcpyDeviceToHost));
+  RG_CUDA_CHECK(copyToHost(out_rgba, n.out.p, sizeof(float4) * P, n.st));
   return RG_OK;
 }
 

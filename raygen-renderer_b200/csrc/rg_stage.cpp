@@ -1,0 +1,202 @@
+// rg_stage.cpp - large copies between the caller's pageable memory and the device.
+//
+// A cudaMemcpy from or to pageable memory goes through one driver thread: a
+// 33 MB image into a fresh array takes 8.7 ms, most of it the first touch of the
+// array's pages and the copy out of the driver's buffer, against 0.7 ms on the
+// link.  Here a few host threads, each with two page-locked slots and a stream
+// of its own, take chunks in turn: while one slot is on the link, the other is
+// copied.  Page-locked callers and small copies keep the direct copy.
+//
+// The page-locked slots and streams are pooled (at most kKept sets, 8 MB each)
+// while any renderer or denoiser exists, and freed with the last one; threads
+// live only for the copy.  Every set is used by one copy at a time.
+#include <cuda_runtime.h>
+
+#include <algorithm>
+#include <atomic>
+#include <cstring>
+#include <mutex>
+#include <thread>
+
+#include "rg_host.h"
+
+namespace rg {
+
+namespace {
+
+constexpr int kWorkers = 8;
+constexpr size_t kChunk = size_t(512) << 10;
+// Below this a direct copy is as fast (the threads take about 0.1 ms to start).
+constexpr size_t kStagedBytes = size_t(3) << 20;
+constexpr int kKept = 2;
+
+struct Stage {
+  int device = 0;
+  unsigned char* slots = nullptr;  // [kWorkers][2][kChunk], page-locked
+  cudaStream_t stream[kWorkers] = {};
+  cudaEvent_t done[kWorkers][2] = {};
+  cudaEvent_t start = nullptr;
+  ~Stage() {
+    for (int w = 0; w < kWorkers; ++w) {
+      for (auto e : done[w])
+        if (e) cudaEventDestroy(e);
+      if (stream[w]) cudaStreamDestroy(stream[w]);
+    }
+    if (start) cudaEventDestroy(start);
+    if (slots) cudaFreeHost(slots);
+  }
+  bool init(int dev) {
+    device = dev;
+    if (cudaHostAlloc((void**)&slots, kWorkers * 2 * kChunk, cudaHostAllocPortable) != cudaSuccess) slots = nullptr;
+    bool ok = slots && cudaEventCreateWithFlags(&start, cudaEventDisableTiming) == cudaSuccess;
+    for (int w = 0; ok && w < kWorkers; ++w) {
+      ok = cudaStreamCreateWithFlags(&stream[w], cudaStreamNonBlocking) == cudaSuccess;
+      for (int s = 0; ok && s < 2; ++s) ok = cudaEventCreateWithFlags(&done[w][s], cudaEventDisableTiming) == cudaSuccess;
+    }
+    if (!ok) cudaGetLastError();
+    return ok;
+  }
+};
+
+std::mutex g_mu;
+int g_users = 0;
+Stage* g_free[kKept] = {};
+
+Stage* acquire() {
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess) return nullptr;
+  {
+    std::lock_guard<std::mutex> lk(g_mu);
+    if (g_users == 0) return nullptr;  // nothing would keep the set: not worth its allocation
+    for (auto& f : g_free)
+      if (f && f->device == dev) return std::exchange(f, nullptr);
+  }
+  Stage* s = new (std::nothrow) Stage();
+  if (s && !s->init(dev)) {
+    delete s;
+    s = nullptr;
+  }
+  return s;
+}
+
+void release(Stage* s) {
+  {
+    std::lock_guard<std::mutex> lk(g_mu);
+    if (g_users > 0)
+      for (auto& f : g_free)
+        if (!f) {
+          f = s;
+          return;
+        }
+  }
+  delete s;
+}
+
+bool pageable(const void* p) {
+  cudaPointerAttributes a;
+  if (cudaPointerGetAttributes(&a, p) != cudaSuccess) {
+    cudaGetLastError();
+    return false;
+  }
+  return a.type == cudaMemoryTypeUnregistered;
+}
+
+// One worker's share: chunks off the common counter, two in flight.
+cudaError_t work(Stage& s, int w, bool toHost, unsigned char* host, unsigned char* dev, size_t bytes,
+                 std::atomic<size_t>& next) {
+  unsigned char* slot[2] = {s.slots + (size_t)(2 * w) * kChunk, s.slots + (size_t)(2 * w + 1) * kChunk};
+  size_t at[2] = {0, 0}, len[2] = {0, 0};
+  auto finish = [&](int k) -> cudaError_t {  // the slot's copy is over; toHost: hand its bytes to the caller
+    if (!len[k]) return cudaSuccess;
+    const cudaError_t e = cudaEventSynchronize(s.done[w][k]);
+    if (e == cudaSuccess && toHost) std::memcpy(host + at[k], slot[k], len[k]);
+    len[k] = 0;
+    return e;
+  };
+  cudaError_t err = cudaStreamWaitEvent(s.stream[w], s.start, 0);
+  for (int k = 0; err == cudaSuccess; k ^= 1) {
+    if ((err = finish(k)) != cudaSuccess) break;
+    const size_t o = next.fetch_add(kChunk);
+    if (o >= bytes) break;
+    at[k] = o;
+    len[k] = std::min(kChunk, bytes - o);
+    if (!toHost) std::memcpy(slot[k], host + o, len[k]);
+    err = toHost ? cudaMemcpyAsync(slot[k], dev + o, len[k], cudaMemcpyDeviceToHost, s.stream[w])
+                 : cudaMemcpyAsync(dev + o, slot[k], len[k], cudaMemcpyHostToDevice, s.stream[w]);
+    if (err == cudaSuccess) err = cudaEventRecord(s.done[w][k], s.stream[w]);
+  }
+  for (int k = 0; k < 2; ++k) {
+    const cudaError_t e = finish(k);
+    if (err == cudaSuccess) err = e;
+  }
+  // nothing of this copy is in flight when the slots go back to the pool
+  const cudaError_t e = cudaStreamSynchronize(s.stream[w]);
+  return err == cudaSuccess ? e : err;
+}
+
+// The staged copy; false: not done (no staging to be had), copy directly.
+bool staged(bool toHost, void* host, void* dev, size_t bytes, cudaStream_t after, cudaError_t& err) {
+  if (bytes < kStagedBytes || !pageable(host)) return false;
+  cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+  if (cudaStreamIsCapturing(after, &cap) != cudaSuccess || cap != cudaStreamCaptureStatusNone) return false;
+  Stage* s = acquire();
+  if (!s) return false;
+  const int chunks = (int)std::min<size_t>(kWorkers, (bytes + 2 * kChunk - 1) / (2 * kChunk));
+  const int cores = (int)std::thread::hardware_concurrency();
+  const int workers = std::max(1, std::min(chunks, cores > 2 ? cores / 2 : 1));
+  err = cudaEventRecord(s->start, after);
+  std::atomic<size_t> next{0};
+  cudaError_t results[kWorkers] = {};
+  std::thread threads[kWorkers];
+  if (err == cudaSuccess) {
+    for (int w = 1; w < workers; ++w) {
+      try {
+        threads[w] = std::thread([&, w] {
+          cudaSetDevice(s->device);
+          results[w] = work(*s, w, toHost, (unsigned char*)host, (unsigned char*)dev, bytes, next);
+        });
+      } catch (...) {
+        break;  // no more threads to be had: the others take its chunks
+      }
+    }
+    results[0] = work(*s, 0, toHost, (unsigned char*)host, (unsigned char*)dev, bytes, next);
+    for (auto& t : threads)
+      if (t.joinable()) t.join();
+    for (auto r : results)
+      if (err == cudaSuccess) err = r;
+  }
+  release(s);
+  return true;
+}
+
+}  // namespace
+
+StageUser::StageUser() {
+  std::lock_guard<std::mutex> lk(g_mu);
+  g_users++;
+}
+
+StageUser::~StageUser() {
+  Stage* old[kKept] = {};
+  {
+    std::lock_guard<std::mutex> lk(g_mu);
+    if (--g_users == 0)
+      for (int i = 0; i < kKept; ++i) old[i] = std::exchange(g_free[i], nullptr);
+  }
+  for (auto* s : old) delete s;
+}
+
+cudaError_t copyToHost(void* dst, const void* devSrc, size_t bytes, cudaStream_t after) {
+  cudaError_t err = cudaSuccess;
+  if (staged(true, dst, const_cast<void*>(devSrc), bytes, after, err)) return err;
+  err = cudaMemcpyAsync(dst, devSrc, bytes, cudaMemcpyDeviceToHost, after);
+  return err == cudaSuccess ? cudaStreamSynchronize(after) : err;
+}
+
+cudaError_t copyToDevice(void* devDst, const void* src, size_t bytes, cudaStream_t after) {
+  cudaError_t err = cudaSuccess;
+  if (staged(false, const_cast<void*>(src), devDst, bytes, after, err)) return err;
+  return cudaMemcpyAsync(devDst, src, bytes, cudaMemcpyHostToDevice, after);
+}
+
+}  // namespace rg
