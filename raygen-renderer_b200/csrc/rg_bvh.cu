@@ -7,16 +7,19 @@
 // The reference builds top-down and recursively on one CPU thread: widest
 // centroid axis, 16 bins, leaf <= 4, cost 1 + 1.5 (A_L N_L + A_R N_R)/A_P
 // against 1.5 N.  Here the same split rule (bin count a parameter, 32 by
-// default) runs breadth-first: every level bins all open nodes at once
-// (shared-memory bins for blocks inside one node, global atomics across
-// nodes), picks splits one thread per node, and scatters primitives with
-// warp-aggregated atomics.  Leaves hold at most kMaxLeaf (8) triangles:
+// default) runs breadth-first over nodes of more than kSubtree primitives: every
+// level bins all open nodes at once, picks splits one warp per node and moves the
+// primitives by a stable partition; below that size one block splits a node to
+// the end in shared memory.  Leaves hold at most kMaxLeaf (8) triangles:
 // where the reference would keep a larger leaf, the best SAH bin (or, for
 // coincident centroids, an index median) splits it further.
 #include <chrono>
 #include <cstdio>
 #include <cstdlib>
+#include <climits>
 #include <cub/device/device_scan.cuh>
+#include <thrust/iterator/counting_iterator.h>
+#include <thrust/iterator/transform_iterator.h>
 #include <cuda_fp16.h>
 
 #include <cfloat>
@@ -52,6 +55,9 @@ struct BinData {  // ordered-uint encoded bounds, 16 words
   uint32_t count;
   uint32_t pad[3];
 };
+
+// device counters of a build
+enum BuildCounter { C_NODES = 0, C_BUILD_ERROR = 1, C_SMALL = 2, C_BUILD_COUNTERS = 3 };
 
 // ---- triangle preparation -------------------------------------------------
 // World -> view (camera translation; angles handled on the host by rotating
@@ -109,6 +115,11 @@ __global__ void k_prepTriangles(int n, const float* __restrict__ pos, const floa
 }
 
 // ---- root bounds -------------------------------------------------------------
+__global__ void k_initBounds(uint32_t* out) {  // identities, as k_rootBounds reduces into them
+  const int k = threadIdx.x;
+  if (k < 12) out[k] = (k / 3) % 2 == 0 ? 0xFFFFFFFFu : 0u;
+}
+
 __global__ void k_rootBounds(int n, const float4* __restrict__ bmin, const float4* __restrict__ bmax, uint32_t* out) {
   // out: bmin[3] bmax[3] cmin[3] cmax[3] (encoded)
   float lo[3] = {FLT_MAX, FLT_MAX, FLT_MAX}, hi[3] = {-FLT_MAX, -FLT_MAX, -FLT_MAX};
@@ -142,9 +153,17 @@ __global__ void k_rootBounds(int n, const float4* __restrict__ bmin, const float
   }
 }
 
-__global__ void k_initRoot(int n, const uint32_t* rb, BNode* nodes, int* primIdx, int* primNode, int rootOpen) {
+// rootOpen: 0 a leaf, 1 open for the levels (task 0 of level 0), 2 small enough for k_subtrees.
+__global__ void k_initRoot(int n, const uint32_t* rb, BNode* nodes, int* primIdx, int* primNode, int rootOpen, int* counters,
+                           int* levelCount, int* tasks, int* smallTasks) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i == 0) {
+    counters[C_NODES] = 1;
+    counters[C_BUILD_ERROR] = 0;
+    counters[C_SMALL] = rootOpen == 2 ? 1 : 0;
+    levelCount[0] = rootOpen == 1 ? 1 : 0;
+    tasks[0] = 0;
+    smallTasks[0] = 0;
     BNode r;
     for (int k = 0; k < 3; k++) {
       r.bmin[k] = fdec(rb[k]); r.bmax[k] = fdec(rb[3 + k]);
@@ -155,20 +174,30 @@ __global__ void k_initRoot(int n, const uint32_t* rb, BNode* nodes, int* primIdx
   }
   if (i < n) {
     primIdx[i] = i;
-    primNode[i] = rootOpen ? 0 : -1;
+    primNode[i] = rootOpen == 1 ? 0 : -1;
   }
 }
 
-// Prepare open nodes of a level: pick the widest centroid axis (bvh.cpp:125-131).
-__global__ void k_prepareLevel(int numTasks, const int* tasks, BNode* nodes, BinData* bins, int nbins, bool resetBins) {
+// Prepare open nodes of a level: pick the widest centroid axis.
+// Task counts live on the device (`count`, of which this launch takes [first, first + most)), so
+// that levels can be launched before the previous ones have run.
+__device__ __forceinline__ int tasksOf(const int* count, int first, int most) { return max(0, min(*count - first, most)); }
+
+__device__ __forceinline__ int widestAxis(const BNode& nd) {  // bvh.cpp:125-131
+  const float ex = nd.cmax[0] - nd.cmin[0], ey = nd.cmax[1] - nd.cmin[1], ez = nd.cmax[2] - nd.cmin[2];
+  int axis = 0;
+  if (ey > ex) axis = 1;
+  if (ez > ((axis == 0) ? ex : ey)) axis = 2;
+  return axis;
+}
+
+__global__ void k_prepareLevel(const int* count, int first, int most, const int* tasks, BNode* nodes, BinData* bins, int nbins,
+                               bool resetBins) {
+  const int numTasks = tasksOf(count, first, most);
   const int t = blockIdx.x * blockDim.x + threadIdx.x;
   if (t < numTasks) {
-    BNode& nd = nodes[tasks[t]];
-    const float ex = nd.cmax[0] - nd.cmin[0], ey = nd.cmax[1] - nd.cmin[1], ez = nd.cmax[2] - nd.cmin[2];
-    int axis = 0;
-    if (ey > ex) axis = 1;
-    if (ez > ((axis == 0) ? ex : ey)) axis = 2;
-    nd.axis = axis;
+    BNode& nd = nodes[tasks[first + t]];
+    nd.axis = widestAxis(nd);
     nd.binSlot = t;
   }
   // reset bins (one thread per bin) unless the split kernel leaves them reset
@@ -208,10 +237,130 @@ constexpr int kBinChunk = RG_BIN_CHUNK;
 constexpr int kWideMaxLeaf = RG_WIDE_MAX_LEAF;
 static_assert(kWideMaxLeaf >= 1 && kWideMaxLeaf <= 4, "8 leaves of at most 4 triangles fill the 32-bit mask");
 constexpr int kMaxBins = 64;
+// Nodes of at most this many primitives are split to the end by one thread block
+// (k_subtrees); larger ones level by level over the whole device.  A level reads every
+// primitive and costs six launches; below this size the levels were 40% of the build of 4M
+// triangles and nearly all of a small scene's.
+#ifndef RG_SUBTREE
+#define RG_SUBTREE 1024
+#endif
+constexpr int kSubtree = RG_SUBTREE;
+static_assert(kSubtree >= kBinChunk, "k_bin: a chunk reaches into at most two open nodes");
 
-// bmin / bmax are in the current primitive order (they move with primIdx in
-// k_partition), so the passes over the primitives read them coalesced.
+// One primitive's bounds and centroid into a bin in shared memory (ordered-uint encoded).
+__device__ __forceinline__ void binPrim(uint32_t (&sb)[13], const uint32_t (&v)[12], uint32_t count) {
+#pragma unroll
+  for (int k = 0; k < 3; k++) {
+    atomicMin(&sb[k], v[k]);
+    atomicMax(&sb[3 + k], v[3 + k]);
+    atomicMin(&sb[6 + k], v[6 + k]);
+    atomicMax(&sb[9 + k], v[9 + k]);
+  }
+  atomicAdd(&sb[12], count);
+}
+
+// Bins of the open nodes of a level.  Open nodes hold more than kBinChunk primitives in
+// consecutive places, so a block's chunk reaches into at most two of them; it bins them in
+// shared memory and adds the bins that got any to the nodes' bins in global memory.
+// Neighbouring primitives mostly fall into the same bin, whose 13 shared-memory atomics
+// then serialise over the warp: the lanes of the bins of up to three leading lanes are
+// reduced in registers first.  bmin / bmax are in the current primitive order (they move
+// with primIdx in the partition), so the pass reads them coalesced.
 __global__ void __launch_bounds__(256) k_bin(int n, const int* __restrict__ primNode, const BNode* __restrict__ nodes,
+                                             const float4* __restrict__ bmin, const float4* __restrict__ bmax,
+                                             BinData* bins, int nbins) {
+  __shared__ uint32_t sb[2][kMaxBins][13];
+  __shared__ int sNode[2];  // lowest and highest open node id of the chunk
+  const int first = blockIdx.x * kBinChunk;
+  const int last = min(n, first + kBinChunk);
+  if (threadIdx.x == 0) {
+    sNode[0] = INT_MAX;
+    sNode[1] = -1;
+  }
+  for (int b = threadIdx.x; b < 2 * nbins; b += blockDim.x) {
+    uint32_t* r = sb[b / nbins][b % nbins];
+    for (int k = 0; k < 3; k++) {
+      r[k] = r[6 + k] = 0xFFFFFFFFu;
+      r[3 + k] = r[9 + k] = 0u;
+    }
+    r[12] = 0u;
+  }
+  __syncthreads();
+  {
+    int lo = INT_MAX, hi = -1;
+    for (int i = first + threadIdx.x; i < last; i += blockDim.x) {
+      const int nd = primNode[i];
+      if (nd >= 0) {
+        lo = min(lo, nd);
+        hi = max(hi, nd);
+      }
+    }
+    lo = __reduce_min_sync(0xffffffffu, lo);
+    hi = __reduce_max_sync(0xffffffffu, hi);
+    if ((threadIdx.x & 31) == 0 && hi >= 0) {
+      atomicMin(&sNode[0], lo);
+      atomicMax(&sNode[1], hi);
+    }
+  }
+  __syncthreads();
+  const int nodeA = sNode[0], nodeB = sNode[1];
+  if (nodeB < 0) return;
+  const BNode ndA = nodes[nodeA], ndB = nodes[nodeB];
+  const bool onA = ndA.binSlot >= 0 && ndA.cmax[ndA.axis] - ndA.cmin[ndA.axis] >= 1e-12f;
+  const bool onB = ndB.binSlot >= 0 && ndB.cmax[ndB.axis] - ndB.cmin[ndB.axis] >= 1e-12f;
+  const int lane = threadIdx.x & 31;
+  for (int i0 = first; i0 < last; i0 += blockDim.x) {  // whole warps: i0 is the block's
+    const int i = i0 + threadIdx.x;
+    const int nd = i < last ? primNode[i] : -1;
+    const bool isA = nd == nodeA, in = nd >= 0 && (isA ? onA : onB);
+    int slot = -1;  // bin of the two nodes' bins
+    uint32_t v[12];
+    if (in) {
+      const float4 lo = bmin[i], hi = bmax[i];
+      const float4 c = make_float4((lo.x + hi.x) * 0.5f, (lo.y + hi.y) * 0.5f, (lo.z + hi.z) * 0.5f, 0.0f);
+      const BNode& N = isA ? ndA : ndB;
+      slot = (isA ? 0 : kMaxBins) + binOf(N, axisOf(c, N.axis), nbins);
+      v[0] = fenc(lo.x); v[1] = fenc(lo.y); v[2] = fenc(lo.z);
+      v[3] = fenc(hi.x); v[4] = fenc(hi.y); v[5] = fenc(hi.z);
+      v[6] = v[9] = fenc(c.x); v[7] = v[10] = fenc(c.y); v[8] = v[11] = fenc(c.z);
+    }
+    unsigned left = __ballot_sync(0xffffffffu, in);
+    for (int r = 0; r < 3 && left; r++) {
+      const int lead = __ffs(left) - 1;
+      const unsigned same = __ballot_sync(0xffffffffu, slot == __shfl_sync(0xffffffffu, slot, lead));
+      if ((same >> lane) & 1u) {
+        uint32_t w[12];
+#pragma unroll
+        for (int k = 0; k < 3; k++) {
+          w[k] = __reduce_min_sync(same, v[k]);
+          w[3 + k] = __reduce_max_sync(same, v[3 + k]);
+          w[6 + k] = __reduce_min_sync(same, v[6 + k]);
+          w[9 + k] = __reduce_max_sync(same, v[9 + k]);
+        }
+        if (lane == lead) binPrim(sb[slot / kMaxBins][slot % kMaxBins], w, __popc(same));
+      }
+      left &= ~same;
+    }
+    if ((left >> lane) & 1u) binPrim(sb[slot / kMaxBins][slot % kMaxBins], v, 1u);
+  }
+  __syncthreads();
+  for (int b = threadIdx.x; b < 2 * nbins; b += blockDim.x) {
+    const uint32_t* r = sb[b / nbins][b % nbins];
+    if (r[12] == 0) continue;
+    BinData& nb = bins[(size_t)(b < nbins ? ndA.binSlot : ndB.binSlot) * nbins + b % nbins];
+    for (int k = 0; k < 3; k++) {
+      atomicMin(&nb.bmin[k], r[k]);
+      atomicMax(&nb.bmax[k], r[3 + k]);
+      atomicMin(&nb.cmin[k], r[6 + k]);
+      atomicMax(&nb.cmax[k], r[9 + k]);
+    }
+    atomicAdd(&nb.count, r[12]);
+  }
+}
+
+// Binning for more than 32 bins, where nodes of any size are open: shared-memory bins for a
+// block inside one node, global atomics across nodes.
+__global__ void __launch_bounds__(256) k_binAny(int n, const int* __restrict__ primNode, const BNode* __restrict__ nodes,
                                              const float4* __restrict__ bmin, const float4* __restrict__ bmax,
                                              BinData* bins, int nbins) {
   __shared__ uint32_t sb[kMaxBins][13];
@@ -282,11 +431,12 @@ __device__ __forceinline__ float areaOf(const float lo[3], const float hi[3]) {
 }
 
 // Split decision per open node (bvh.cpp:133-211 cost model).
-__global__ void k_split(int numTasks, const int* __restrict__ tasks, BNode* nodes, const BinData* __restrict__ bins,
-                        int nbins, int* nodeCounter, int* nextTasks, int* nextCount, int maxLeaf) {
+__global__ void k_split(const int* count, int firstTask, int most, const int* __restrict__ tasks, BNode* nodes,
+                        const BinData* __restrict__ bins, int nbins, int* nodeCounter, int* nextTasks, int* nextCount,
+                        int maxLeaf) {
   const int t = blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= numTasks) return;
-  const int id = tasks[t];
+  if (t >= tasksOf(count, firstTask, most)) return;
+  const int id = tasks[firstTask + t];
   BNode nd = nodes[id];
   const BinData* nb = bins + (size_t)nd.binSlot * nbins;
   const float ext = nd.cmax[nd.axis] - nd.cmin[nd.axis];
@@ -420,27 +570,21 @@ __device__ __forceinline__ int warpScanI(int v, int lane, bool reverse) {
   return v;
 }
 
-__global__ void __launch_bounds__(128) k_splitWarp(int numTasks, const int* __restrict__ tasks, BNode* nodes,
-                                                  BinData* bins, int nbins, int* nodeCounter, int* nextTasks,
-                                                  int* nextCount, int maxLeaf) {
-  const int t = (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 5);
+// Split of node nd from its bins, lane b's bin in (cnt, b*, c*): ordered-uint bounds of the
+// primitives and of their centroids, identities when empty.  All lanes return the split (bin,
+// -1 leaf, -2 index median) and the children's counts and bounds (bmin, bmax, cmin, cmax).
+struct WarpSplit {
+  int split;
+  int count[2];
+  float bounds[2][12];
+};
+__device__ __forceinline__ WarpSplit decideSplit(const BNode& nd, int nbins, int maxLeaf, int cnt, const uint32_t (&bin)[12]) {
   const int lane = threadIdx.x & 31;
-  if (t >= numTasks) return;
-  const int id = tasks[t];
-  BNode nd = nodes[id];
-  BinData* nb = bins + (size_t)nd.binSlot * nbins;
-  // this lane's bin (identity when empty or past nbins)
-  int cnt = 0;
-  float blo[3] = {FLT_MAX, FLT_MAX, FLT_MAX}, bhi[3] = {-FLT_MAX, -FLT_MAX, -FLT_MAX};
-  float clo[3] = {FLT_MAX, FLT_MAX, FLT_MAX}, chi[3] = {-FLT_MAX, -FLT_MAX, -FLT_MAX};
-  if (lane < nbins) {
-    const BinData b = nb[lane];
-    cnt = (int)b.count;
-    if (cnt > 0)
-      for (int k = 0; k < 3; k++) {
-        blo[k] = fdec(b.bmin[k]); bhi[k] = fdec(b.bmax[k]); clo[k] = fdec(b.cmin[k]); chi[k] = fdec(b.cmax[k]);
-      }
-    resetBin(nb + lane);
+  const bool any = cnt > 0;
+  float blo[3], bhi[3];
+  for (int k = 0; k < 3; k++) {
+    blo[k] = any ? fdec(bin[k]) : FLT_MAX;
+    bhi[k] = any ? fdec(bin[3 + k]) : -FLT_MAX;
   }
   // left: bins 0..lane, right: bins lane..nbins-1
   float llo[3], lhi[3], rlo[3], rhi[3];
@@ -450,9 +594,8 @@ __global__ void __launch_bounds__(128) k_splitWarp(int numTasks, const int* __re
     rlo[k] = warpScanF<true>(blo[k], lane, true);
     rhi[k] = warpScanF<false>(bhi[k], lane, true);
   }
-  const int lc = warpScanI(cnt, lane, false), rcAll = warpScanI(cnt, lane, true);
+  const int lc = warpScanI(cnt, lane, false), total = __shfl_sync(0xffffffffu, lc, 31), rc = total - lc;
   // split s = lane: left = bins 0..s, right = bins s+1..nbins-1 (the right sums of lane s + 1)
-  const int rc = __shfl_down_sync(0xffffffffu, rcAll, 1);
   float rl[3], rh[3];
   for (int k = 0; k < 3; k++) {
     rl[k] = __shfl_down_sync(0xffffffffu, rlo[k], 1);
@@ -477,107 +620,232 @@ __global__ void __launch_bounds__(128) k_splitWarp(int numTasks, const int* __re
   }
   const int forced = bs == 0x7fffffff ? -1 : bs;
   const int best = (forced >= 0 && bc < (float)nd.count * 1.5f) ? forced : -1;
-  int split = best;
-  if (split < 0 && nd.count > maxLeaf) split = forced >= 0 ? forced : -2;  // -2: index median
-  // child bounds: reductions over the bins of each side
-  float cb[2][12];
-  int cc[2];
-  for (int sd = 0; sd < 2; sd++) {
-    const bool mine = split >= 0 && (sd == 0 ? lane <= split : lane > split);
+  WarpSplit r;
+  r.split = best;
+  if (best < 0 && nd.count > maxLeaf) r.split = forced >= 0 ? forced : -2;  // -2: index median
+  const int at = r.split >= 0 ? r.split : 0;
+  r.count[0] = r.split >= 0 ? __shfl_sync(0xffffffffu, lc, at) : nd.count / 2;
+  r.count[1] = (r.split >= 0 ? total : nd.count) - r.count[0];
+  for (int k = 0; k < 3; k++) {
+    // bounds: the scans at the split; centroid bounds: reductions of each side's bins
+    const float l0 = __shfl_sync(0xffffffffu, llo[k], at), l1 = __shfl_sync(0xffffffffu, lhi[k], at),
+                r0 = __shfl_sync(0xffffffffu, rl[k], at), r1 = __shfl_sync(0xffffffffu, rh[k], at);
+    const bool onL = lane <= at;
+    const uint32_t cl0 = __reduce_min_sync(0xffffffffu, any && onL ? bin[6 + k] : 0xFFFFFFFFu),
+                   cl1 = __reduce_max_sync(0xffffffffu, any && onL ? bin[9 + k] : 0u),
+                   cr0 = __reduce_min_sync(0xffffffffu, any && !onL ? bin[6 + k] : 0xFFFFFFFFu),
+                   cr1 = __reduce_max_sync(0xffffffffu, any && !onL ? bin[9 + k] : 0u);
+    const bool med = r.split < 0;
+    r.bounds[0][k] = med ? nd.bmin[k] : l0;
+    r.bounds[0][3 + k] = med ? nd.bmax[k] : l1;
+    r.bounds[0][6 + k] = med ? nd.cmin[k] : fdec(cl0);
+    r.bounds[0][9 + k] = med ? nd.cmax[k] : fdec(cl1);
+    r.bounds[1][k] = med ? nd.bmin[k] : r0;
+    r.bounds[1][3 + k] = med ? nd.bmax[k] : r1;
+    r.bounds[1][6 + k] = med ? nd.cmin[k] : fdec(cr0);
+    r.bounds[1][9 + k] = med ? nd.cmax[k] : fdec(cr1);
+  }
+  return r;
+}
+
+// Child `side` of a split node (one lane each).
+__device__ __forceinline__ void writeChild(BNode* nodes, int left, int side, int start, const WarpSplit& sp) {
+  BNode c;
+  for (int k = 0; k < 3; k++) {
+    c.bmin[k] = side ? sp.bounds[1][k] : sp.bounds[0][k];
+    c.bmax[k] = side ? sp.bounds[1][3 + k] : sp.bounds[0][3 + k];
+    c.cmin[k] = side ? sp.bounds[1][6 + k] : sp.bounds[0][6 + k];
+    c.cmax[k] = side ? sp.bounds[1][9 + k] : sp.bounds[0][9 + k];
+  }
+  c.start = start + (side ? sp.count[0] : 0);
+  c.count = side ? sp.count[1] : sp.count[0];
+  c.left = -1;
+  c.axis = 0;
+  c.binSlot = -1;
+  c.splitBin = -1;
+  nodes[left + side] = c;
+}
+
+// Split decisions of a level, one warp per open node; the warp resets the bins it read.
+// Children above kSubtree primitives stay open for the next level, smaller ones that can
+// still split (BVH_LEAF_SIZE 4, bvh.cpp:23) go to the block-wise pass.
+__global__ void __launch_bounds__(128) k_splitWarp(const int* count, int first, int most, const int* __restrict__ tasks,
+                                                  BNode* nodes, BinData* bins, int nbins, int* nodeCounter, int* nextTasks,
+                                                  int* nextCount, int* smallTasks, int* smallCount, int maxLeaf) {
+  const int t = (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 5);
+  const int lane = threadIdx.x & 31;
+  if (t >= tasksOf(count, first, most)) return;
+  const int id = tasks[first + t];
+  const BNode nd = nodes[id];
+  BinData* nb = bins + (size_t)nd.binSlot * nbins;
+  int cnt = 0;
+  uint32_t bin[12];
+  for (int k = 0; k < 12; k++) bin[k] = 0u;
+  if (lane < nbins) {
+    const BinData b = nb[lane];
+    cnt = (int)b.count;
     for (int k = 0; k < 3; k++) {
-      float v0 = mine ? blo[k] : FLT_MAX, v1 = mine ? bhi[k] : -FLT_MAX, v2 = mine ? clo[k] : FLT_MAX,
-            v3 = mine ? chi[k] : -FLT_MAX;
-#pragma unroll
-      for (int o = 16; o > 0; o >>= 1) {
-        v0 = fminf(v0, __shfl_xor_sync(0xffffffffu, v0, o));
-        v1 = fmaxf(v1, __shfl_xor_sync(0xffffffffu, v1, o));
-        v2 = fminf(v2, __shfl_xor_sync(0xffffffffu, v2, o));
-        v3 = fmaxf(v3, __shfl_xor_sync(0xffffffffu, v3, o));
-      }
-      cb[sd][k] = v0; cb[sd][3 + k] = v1; cb[sd][6 + k] = v2; cb[sd][9 + k] = v3;
+      bin[k] = b.bmin[k];
+      bin[3 + k] = b.bmax[k];
+      bin[6 + k] = b.cmin[k];
+      bin[9 + k] = b.cmax[k];
     }
-    int c = mine ? cnt : 0;
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) c += __shfl_xor_sync(0xffffffffu, c, o);
-    cc[sd] = c;
+    resetBin(nb + lane);
   }
-  if (lane != 0) return;
-  nd.binSlot = -1;
-  if (split == -1) {
-    nd.left = -1;
-    nodes[id] = nd;
-    return;
+  const WarpSplit sp = decideSplit(nd, nbins, maxLeaf, cnt, bin);
+  int left = -1;
+  if (lane == 0) {
+    if (sp.split != -1) left = atomicAdd(nodeCounter, 2);
+    nodes[id].binSlot = -1;
+    nodes[id].left = left;
+    nodes[id].splitBin = sp.split;
   }
-  const int left = atomicAdd(nodeCounter, 2);
-  BNode ch[2];
-  int cnts[2];
-  for (int sd = 0; sd < 2; sd++) {
-    if (split == -2) {
-      cnts[0] = nd.count / 2;
-      cnts[1] = nd.count - cnts[0];
-      for (int k = 0; k < 3; k++) {
-        ch[sd].bmin[k] = nd.bmin[k]; ch[sd].bmax[k] = nd.bmax[k];
-        ch[sd].cmin[k] = nd.cmin[k]; ch[sd].cmax[k] = nd.cmax[k];
-      }
-    } else {
-      cnts[sd] = cc[sd];
-      for (int k = 0; k < 3; k++) {
-        ch[sd].bmin[k] = cb[sd][k]; ch[sd].bmax[k] = cb[sd][3 + k];
-        ch[sd].cmin[k] = cb[sd][6 + k]; ch[sd].cmax[k] = cb[sd][9 + k];
-      }
-    }
+  if (sp.split == -1) return;
+  left = __shfl_sync(0xffffffffu, left, 0);
+  if (lane < 2) {
+    writeChild(nodes, left, lane, nd.start, sp);
+    const int c = lane ? sp.count[1] : sp.count[0];
+    if (c > kSubtree) nextTasks[atomicAdd(nextCount, 1)] = left + lane;
+    else if (c > 4) smallTasks[atomicAdd(smallCount, 1)] = left + lane;
   }
-  for (int sd = 0; sd < 2; sd++) {
-    ch[sd].start = nd.start + (sd == 0 ? 0 : cnts[0]);
-    ch[sd].count = cnts[sd];
-    ch[sd].left = -1;
-    ch[sd].axis = 0;
-    ch[sd].binSlot = -1;
-    ch[sd].splitBin = -1;
-    nodes[left + sd] = ch[sd];
-    if (cnts[sd] > 4) {  // BVH_LEAF_SIZE (bvh.cpp:23): larger children stay open
-      const int slot = atomicAdd(nextCount, 1);
-      nextTasks[slot] = left + sd;
-    }
-  }
-  nd.left = left;
-  nd.splitBin = split;
-  nodes[id] = nd;
 }
 
-// Partition, pass 1: flag 1 for a primitive that goes to the left child of its
-// node (the split bin, or the first half of the node's range for a median split).
-__global__ void k_partitionFlags(int n, const int* __restrict__ primNode, const BNode* __restrict__ nodes,
-                                 const float4* __restrict__ bmin, const float4* __restrict__ bmax, int nbins,
-                                 int* __restrict__ flags) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n) return;
-  const int node = primNode[i];
-  int flag = 0;
-  if (node >= 0) {
+// Nodes of at most kSubtree primitives: one block splits each to the end, level by level with
+// a warp per node, bounds and order in shared memory.  The same bins, costs and stable
+// partition as the device-wide levels, so the tree is the same.  Bound by the latency of a
+// node's scans and reductions (about 1 us) over the nodes of a block's deepest chain.
+constexpr int kSubThreads = 256;
+__global__ void __launch_bounds__(kSubThreads) k_subtrees(const int* __restrict__ count, const int* __restrict__ tasks,
+                                                          BNode* nodes, int* primIdx, const float4* __restrict__ bmin,
+                                                          const float4* __restrict__ bmax, int nbins, int* nodeCounter,
+                                                          int maxLeaf) {
+  constexpr int kWarps = kSubThreads / 32, kList = kSubtree / 5 + 1;  // nodes of five primitives and more
+  __shared__ float sB[6][kSubtree];
+  __shared__ int sIdx[kSubtree];
+  __shared__ uint16_t sPerm[2][kSubtree];
+  __shared__ uint32_t sBins[kWarps][32][13];
+  __shared__ int sList[2][kList];
+  __shared__ int sCount[2], sBase;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int numTasks = *count;
+  for (int task = blockIdx.x; task < numTasks; task += gridDim.x) {
+    const int root = tasks[task];
+    const int start = nodes[root].start, n = nodes[root].count;
+    for (int i = threadIdx.x; i < n; i += kSubThreads) {
+      const float4 lo = bmin[start + i], hi = bmax[start + i];
+      sB[0][i] = lo.x; sB[1][i] = lo.y; sB[2][i] = lo.z;
+      sB[3][i] = hi.x; sB[4][i] = hi.y; sB[5][i] = hi.z;
+      sIdx[i] = primIdx[start + i];
+      sPerm[0][i] = (uint16_t)i;
+    }
+    if (threadIdx.x == 0) {
+      sList[0][0] = root;
+      sCount[0] = 1;
+    }
+    for (int cur = 0;; cur ^= 1) {
+      __syncthreads();
+      const int L = sCount[cur];
+      if (L == 0) break;
+      if (threadIdx.x == 0) {
+        sBase = atomicAdd(nodeCounter, 2 * L);  // ids for every node of this level to split
+        sCount[cur ^ 1] = 0;
+      }
+      __syncthreads();
+      for (int e = warp; e < L; e += kWarps) {
+        const int id = sList[cur][e], left = sBase + 2 * e;
+        BNode nd = nodes[id];
+        nd.axis = widestAxis(nd);
+        const int s0 = nd.start - start;
+        const bool flat = !(nd.cmax[nd.axis] - nd.cmin[nd.axis] >= 1e-12f);
+        uint32_t (&bins)[32][13] = sBins[warp];
+        for (int k = 0; k < 3; k++) {
+          bins[lane][k] = bins[lane][6 + k] = 0xFFFFFFFFu;
+          bins[lane][3 + k] = bins[lane][9 + k] = 0u;
+        }
+        bins[lane][12] = 0u;
+        __syncwarp();
+        auto binAt = [&](int p) {
+          return binOf(nd, (sB[nd.axis][p] + sB[3 + nd.axis][p]) * 0.5f, nbins);
+        };
+        if (!flat)
+          for (int j = lane; j < nd.count; j += 32) {
+            const int p = sPerm[0][s0 + j];
+            uint32_t v[12];
+            for (int k = 0; k < 3; k++) {
+              const float lo = sB[k][p], hi = sB[3 + k][p];
+              v[k] = fenc(lo);
+              v[3 + k] = fenc(hi);
+              v[6 + k] = v[9 + k] = fenc((lo + hi) * 0.5f);
+            }
+            binPrim(bins[binAt(p)], v, 1u);
+          }
+        __syncwarp();
+        uint32_t bin[12];
+        for (int k = 0; k < 12; k++) bin[k] = bins[lane][k];
+        const WarpSplit sp = decideSplit(nd, nbins, maxLeaf, lane < nbins ? (int)bins[lane][12] : 0, bin);
+        if (lane == 0) {
+          nodes[id].axis = nd.axis;
+          nodes[id].binSlot = -1;
+          nodes[id].left = sp.split == -1 ? -1 : left;
+          nodes[id].splitBin = sp.split;
+        }
+        if (sp.split == -1) {  // its two ids stay unused
+          if (lane < 2) nodes[left + lane].left = -1;
+          continue;
+        }
+        if (lane < 2) {
+          writeChild(nodes, left, lane, nd.start, sp);
+          if ((lane ? sp.count[1] : sp.count[0]) > 4) sList[cur ^ 1][atomicAdd(&sCount[cur ^ 1], 1)] = left + lane;
+        }
+        // stable partition of the node's places through the second order array
+        int nl = 0;
+        for (int j0 = 0; j0 < nd.count; j0 += 32) {
+          const int j = j0 + lane;
+          const bool in = j < nd.count;
+          const int p = in ? sPerm[0][s0 + j] : 0;
+          const bool toLeft = in && (sp.split == -2 ? j < sp.count[0] : binAt(p) <= sp.split);
+          const unsigned m = __ballot_sync(0xffffffffu, toLeft);
+          const int before = nl + __popc(m & ((1u << lane) - 1u));
+          if (in) sPerm[1][s0 + (toLeft ? before : sp.count[0] + j - before)] = (uint16_t)p;
+          nl += __popc(m);
+        }
+        __syncwarp();
+        for (int j = lane; j < nd.count; j += 32) sPerm[0][s0 + j] = sPerm[1][s0 + j];
+        __syncwarp();
+      }
+    }
+    for (int i = threadIdx.x; i < n; i += kSubThreads) primIdx[start + i] = sIdx[sPerm[0][i]];
+    __syncthreads();  // before the next task's data overwrite this one's
+  }
+}
+
+// 1 for a primitive that goes to the left child of its node (the split bin, or the first half
+// of the node's range for a median split); the input of the partition's prefix sum.
+struct LeftFlag {
+  const int* primNode;
+  const BNode* nodes;
+  const float4 *bmin, *bmax;
+  int nbins;
+  __device__ __forceinline__ int operator()(int i) const {
+    const int node = primNode[i];
+    if (node < 0) return 0;
     const BNode& nd = nodes[node];
-    if (nd.left >= 0) {
-      if (nd.splitBin == -2) {
-        flag = (i - nd.start) < nd.count / 2 ? 1 : 0;
-      } else {
-        const float4 lo = bmin[i], hi = bmax[i];
-        const float c = nd.axis == 0 ? (lo.x + hi.x) * 0.5f : (nd.axis == 1 ? (lo.y + hi.y) * 0.5f : (lo.z + hi.z) * 0.5f);
-        flag = binOf(nd, c, nbins) <= nd.splitBin ? 1 : 0;
-      }
-    }
+    if (nd.left < 0) return 0;
+    if (nd.splitBin == -2) return (i - nd.start) < nd.count / 2 ? 1 : 0;
+    const float c = (axisOf(bmin[i], nd.axis) + axisOf(bmax[i], nd.axis)) * 0.5f;
+    return binOf(nd, c, nbins) <= nd.splitBin ? 1 : 0;
   }
-  flags[i] = flag;
-}
+};
 
-// Partition, pass 2 (after an exclusive scan of the flags into `before`): a stable
+// Partition, after an exclusive scan of the flags into `before`: a stable
 // scatter of each split node's primitives into its children's ranges, with their
 // bounds; primitives of closed nodes and new leaves stay where they are.  No
 // atomics, so the order (and the BVH) is the same on every run.
 __global__ void k_partitionScatter(int n, const int* __restrict__ primIdx, const int* __restrict__ primNode,
                                    const BNode* __restrict__ nodes, const float4* __restrict__ bmin,
-                                   const float4* __restrict__ bmax, const int* __restrict__ flags,
-                                   const int* __restrict__ before, int* __restrict__ outIdx, int* __restrict__ outNode,
-                                   float4* __restrict__ outMin, float4* __restrict__ outMax, int* err) {
+                                   const float4* __restrict__ bmax, int nbins, const int* __restrict__ before,
+                                   int* __restrict__ outIdx, int* __restrict__ outNode, float4* __restrict__ outMin,
+                                   float4* __restrict__ outMax, int openCount, int* err) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
   const int node = primNode[i];
@@ -586,7 +854,7 @@ __global__ void k_partitionScatter(int n, const int* __restrict__ primIdx, const
     const BNode& nd = nodes[node];
     if (nd.left >= 0) {
       const int leftBefore = before[i] - before[nd.start];
-      const int side = flags[i] ? 0 : 1;
+      const int side = LeftFlag{primNode, nodes, bmin, bmax, nbins}(i) ? 0 : 1;
       const int rank = side == 0 ? leftBefore : (i - nd.start) - leftBefore;
       const BNode& cn = nodes[nd.left + side];
       if (rank >= cn.count) {
@@ -594,7 +862,7 @@ __global__ void k_partitionScatter(int n, const int* __restrict__ primIdx, const
         return;
       }
       pos = cn.start + rank;
-      outN = cn.count > 4 ? nd.left + side : -1;
+      outN = cn.count > openCount ? nd.left + side : -1;  // smaller ones are closed for the levels
     }
   }
   outIdx[pos] = primIdx[i];
@@ -660,14 +928,11 @@ __global__ void k_gather(int n, const int* __restrict__ primIdx, const float4* _
 // Slots are assigned per octant: a child whose centre lies on the negative side
 // of the node centre along axis k prefers slots with bit k set, so visiting hit
 // slots in descending order of (slot XOR ray octant) is roughly front to back.
-// countOnly: the same child choices, nothing written but the node count and the
-// next level's tasks (the host sizes the node array with it).
-__global__ void k_collapse(int numTasks, const int2* __restrict__ tasks, const BNode* __restrict__ nodes,
-                           const int* __restrict__ primIdx, float4* __restrict__ nodes8, int* counters,
-                           int2* __restrict__ nextTasks, int* __restrict__ triOrder, int maxNodes8, bool countOnly) {
-  const int t = blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= numTasks) return;
-  const int2 task = tasks[t];
+// One task: binary node task.x becomes wide node task.y.  Nodes past maxNodes8 are counted
+// and their children followed, but not written (the host then sizes the array and repeats).
+__device__ __forceinline__ void collapseTask(int2 task, const BNode* __restrict__ nodes, const int* __restrict__ primIdx,
+                                             float4* __restrict__ nodes8, int* counters, int2* __restrict__ nextTasks,
+                                             int* nextCount, int* __restrict__ triOrder, int maxNodes8) {
   const BNode& nd = nodes[task.x];
   int ch[8];
   int nc;
@@ -692,14 +957,6 @@ __global__ void k_collapse(int numTasks, const int2* __restrict__ tasks, const B
       ch[best] = l;
       ch[nc++] = l + 1;
     }
-  }
-  if (countOnly) {
-    for (int i = 0; i < nc; i++)
-      if (nodes[ch[i]].left >= 0) {
-        atomicAdd(&counters[0], 1);
-        nextTasks[atomicAdd(&counters[2], 1)] = make_int2(ch[i], 0);
-      }
-    return;
   }
   float lo[3] = {FLT_MAX, FLT_MAX, FLT_MAX}, hi[3] = {-FLT_MAX, -FLT_MAX, -FLT_MAX};
   float cc[8][3];
@@ -791,12 +1048,10 @@ __global__ void k_collapse(int numTasks, const int2* __restrict__ tasks, const B
   }
   const int childBase = ni ? atomicAdd(&counters[0], ni) : 0;
   const int triBase = atomicAdd(&counters[1], ntri);
-  if (childBase + ni > maxNodes8) {
-    atomicCAS(&counters[3], 0, kErrPartition);
-    return;
-  }
-  float4* o = nodes8 + (size_t)task.y * kNode8Vec;
+  const bool fits = task.y < maxNodes8;
+  float4* o = nodes8 + (size_t)(fits ? task.y : 0) * kNode8Vec;
   const int sw = task.y & 7;
+  if (fits) {
   o[0 ^ sw] = make_float4(__int_as_float(childBase), __int_as_float(triBase), __uint_as_float(meta[0]), __uint_as_float(meta[1]));
   o[1 ^ sw] = make_float4(finite ? org[0] : 0.0f, finite ? org[1] : 0.0f, finite ? org[2] : 0.0f,
                      __uint_as_float(__float_as_uint(scale) | inner));
@@ -806,13 +1061,14 @@ __global__ void k_collapse(int numTasks, const int2* __restrict__ tasks, const B
       for (int j = 0; j < 4; j++) q[j] = __halves2half2(pl[k][h][2 * j], pl[k][h][2 * j + 1]);
       o[(2 + 2 * k + h) ^ sw] = *reinterpret_cast<const float4*>(q);
     }
+  }
   int k = 0, off = 0;
   for (int sl = 0; sl < 8; sl++) {
     const int c = childAt[sl];
     if (c < 0) continue;
     const BNode& cn = nodes[c];
     if (cn.left >= 0) {
-      const int slot = atomicAdd(&counters[2], 1);
+      const int slot = atomicAdd(nextCount, 1);
       nextTasks[slot] = make_int2(c, childBase + k);
       k++;
     } else {
@@ -820,6 +1076,22 @@ __global__ void k_collapse(int numTasks, const int2* __restrict__ tasks, const B
       off += cn.count;
     }
   }
+}
+
+__global__ void __launch_bounds__(64) k_collapse(const int* __restrict__ count, const int2* __restrict__ tasks,
+                                                 const BNode* __restrict__ nodes, const int* __restrict__ primIdx,
+                                                 float4* __restrict__ nodes8, int* counters, int2* __restrict__ nextTasks,
+                                                 int* nextCount, int* __restrict__ triOrder, int maxNodes8) {
+  const int numTasks = *count;
+  for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < numTasks; t += gridDim.x * blockDim.x)
+    collapseTask(tasks[t], nodes, primIdx, nodes8, counters, nextTasks, nextCount, triOrder, maxNodes8);
+}
+
+__global__ void k_initCollapse(int* counters, int* levelCount, int2* tasks) {
+  counters[0] = 1;  // nodes: the root
+  counters[1] = 0;  // triangles
+  levelCount[0] = 1;
+  tasks[0] = make_int2(0, 0);
 }
 
 inline int gridFor(long long n, int block) { return (int)((n + block - 1) / block); }
@@ -848,7 +1120,7 @@ struct BvhScratch {
   DevBuf<float2> uvTmp;
   DevBuf<uint32_t> rb;
   DevBuf<BNode> nodes;
-  DevBuf<int> idxA, idxB, nodeA, nodeB, tasksA, tasksB, counters, pflags, pbefore;
+  DevBuf<int> idxA, idxB, nodeA, nodeB, tasksA, tasksB, smallTasks, counters, levelCount, pbefore;
   DevBuf<BinData> bins;
   DevBuf<unsigned char> scanTmp, tmp;
   DevBuf<int2> ta, tb;
@@ -887,111 +1159,115 @@ rg_status buildDeviceBvh(DeviceScene& ds, int nbins, bool wide, cudaStream_t st,
     err = "out of device memory (BVH build)";
     return RG_ERR_OUT_OF_MEMORY;
   }
-  {
-    std::vector<uint32_t> init(12);
-    for (int k = 0; k < 3; k++) { init[k] = 0xFFFFFFFFu; init[3 + k] = 0u; init[6 + k] = 0xFFFFFFFFu; init[9 + k] = 0u; }
-    cudaMemcpyAsync(rb.p, init.data(), 12 * sizeof(uint32_t), cudaMemcpyHostToDevice, st);
-  }
+  k_initBounds<<<1, 32, 0, st>>>(rb.p);
   k_rootBounds<<<std::min(gridFor(n, 256), 1184), 256, 0, st>>>(n, lo.p, hi.p, rb.p);
   const size_t maxNodes = 2 * (size_t)n + 1;
+  // up to 32 bins: nodes of at most kSubtree primitives are left to k_subtrees, and one warp
+  // per larger node decides its split
+  const bool warpSplit = nbins <= 32;
+  const int openCount = warpSplit ? kSubtree : 4;  // more primitives than this stay open for the levels
+  const int maxOpen = n / (openCount + 1) + 1;     // open nodes of a level
   // bins for at most chunkTasks open nodes at a time (<= 256 MB)
-  const int chunkTasks = (int)std::min<size_t>((size_t)n / 4 + 2, ((size_t)256 << 20) / (sizeof(BinData) * nbins));
+  const int chunkTasks = (int)std::min<size_t>((size_t)maxOpen, ((size_t)256 << 20) / (sizeof(BinData) * nbins));
   DevBuf<BNode>& nodes = X.nodes;
   DevBuf<int> &idxA = X.idxA, &idxB = X.idxB, &nodeA = X.nodeA, &nodeB = X.nodeB, &tasksA = X.tasksA,
-  &tasksB = X.tasksB, &counters = X.counters, &pflags = X.pflags, &pbefore = X.pbefore;
+  &tasksB = X.tasksB, &smallTasks = X.smallTasks, &counters = X.counters, &levelCount = X.levelCount,
+  &pbefore = X.pbefore;
   DevBuf<BinData>& bins = X.bins;
   trace.mark("prep kern", 0, n);
+  constexpr int kMaxLevels = 200;
   if (!nodes.alloc(maxNodes) || !idxA.alloc(n) || !idxB.alloc(n) || !nodeA.alloc(n) || !nodeB.alloc(n) ||
-      !lo2.alloc(n) || !hi2.alloc(n) || !pflags.alloc(n) || !pbefore.alloc(n) ||
-      !tasksA.alloc((size_t)n / 4 + 2) || !tasksB.alloc((size_t)n / 4 + 2) || !counters.alloc(4) ||
-      !bins.alloc((size_t)chunkTasks * nbins)) {
+      !lo2.alloc(n) || !hi2.alloc(n) || !pbefore.alloc(n) || !tasksA.alloc((size_t)maxOpen + 1) ||
+      !tasksB.alloc((size_t)maxOpen + 1) || !smallTasks.alloc((size_t)n / 5 + 2) || !counters.alloc(C_BUILD_COUNTERS) ||
+      !levelCount.alloc(kMaxLevels + 2) || !bins.alloc((size_t)chunkTasks * nbins)) {
     err = "out of device memory (BVH build)";
     return RG_ERR_OUT_OF_MEMORY;
   }
-  const int rootOpen = n > 4 ? 1 : 0;
-  k_initRoot<<<gridFor(n, 256), 256, 0, st>>>(n, rb.p, nodes.p, idxA.p, nodeA.p, rootOpen);
-  int h_counters[4] = {1, 0, 0, 0};  // [0] node count, [1] next task count, [2] error
-  cudaMemcpyAsync(counters.p, h_counters, sizeof(h_counters), cudaMemcpyHostToDevice, st);
-  int numTasks = rootOpen;
-  {
-    const int zero = 0;
-    cudaMemcpyAsync(tasksA.p, &zero, sizeof(int), cudaMemcpyHostToDevice, st);
-  }
+  const int rootOpen = n <= 4 ? 0 : (n > openCount ? 1 : 2);
+  cudaMemsetAsync(levelCount.p, 0, sizeof(int) * (kMaxLevels + 2), st);
+  k_initRoot<<<gridFor(n, 256), 256, 0, st>>>(n, rb.p, nodes.p, idxA.p, nodeA.p, rootOpen, counters.p, levelCount.p,
+                                              tasksA.p, smallTasks.p);
   int* curIdx = idxA.p;
   int* curNode = nodeA.p;
   int* altIdx = idxB.p;
   int* altNode = nodeB.p;
   int* curTasks = tasksA.p;
   int* nxtTasks = tasksB.p;
-  // up to 32 bins: one warp per node decides the split and resets its bins, which
-  // therefore start reset once here
-  const bool warpSplit = nbins <= 32;
-  if (warpSplit) {
-    const size_t nb = (size_t)chunkTasks * nbins;
-    k_resetBins<<<(unsigned)((nb + 255) / 256), 256, 0, st>>>(nb, bins.p);
-  }
-  // scratch of the partition's prefix sum
-  size_t scanBytes = 0;
-  cub::DeviceScan::ExclusiveSum(nullptr, scanBytes, pflags.p, pbefore.p, n, st);
-  DevBuf<unsigned char>& scanTmp = X.scanTmp;
-  if (!scanTmp.alloc(scanBytes + 16)) {
-    err = "out of device memory (BVH build)";
-    return RG_ERR_OUT_OF_MEMORY;
-  }
   float4* curLo = lo.p;
   float4* curHi = hi.p;
   float4* altLo = lo2.p;
   float4* altHi = hi2.p;
   int levels = 0;
   trace.mark("alloc tree", 0, n);
-  trace.mark("prep", 0, numTasks);
-  while (numTasks > 0) {
-    levels++;
-    const int tasksThisLevel = numTasks;
-    cudaMemsetAsync(counters.p + 1, 0, sizeof(int), st);
-    for (int c0 = 0; c0 < numTasks; c0 += chunkTasks) {
-      const int nt = std::min(chunkTasks, numTasks - c0);
-      const int prepN = warpSplit ? nt : std::max(nt, nt * nbins);
-      k_prepareLevel<<<gridFor(prepN, 256), 256, 0, st>>>(nt, curTasks + c0, nodes.p, bins.p, nbins, !warpSplit);
-      k_bin<<<gridFor(n, kBinChunk), 256, 0, st>>>(n, curNode, nodes.p, curLo, curHi, bins.p, nbins);
-      if (warpSplit)
-        k_splitWarp<<<gridFor((long long)nt * 32, 128), 128, 0, st>>>(nt, curTasks + c0, nodes.p, bins.p, nbins,
-                                                                      counters.p, nxtTasks, counters.p + 1,
-                                                                      wide ? kWideMaxLeaf : kMaxLeaf);
-      else
-        k_split<<<gridFor(nt, 128), 128, 0, st>>>(nt, curTasks + c0, nodes.p, bins.p, nbins, counters.p, nxtTasks,
-                                                   counters.p + 1, wide ? kWideMaxLeaf : kMaxLeaf);
+  if (rootOpen == 1) {
+    if (warpSplit) {  // k_splitWarp resets the bins it reads, so they start reset once here
+      const size_t nb = (size_t)chunkTasks * nbins;
+      k_resetBins<<<(unsigned)((nb + 255) / 256), 256, 0, st>>>(nb, bins.p);
     }
-    k_partitionFlags<<<gridFor(n, 256), 256, 0, st>>>(n, curNode, nodes.p, curLo, curHi, nbins, pflags.p);
-    cub::DeviceScan::ExclusiveSum(scanTmp.p, scanBytes, pflags.p, pbefore.p, n, st);
-    k_partitionScatter<<<gridFor(n, 256), 256, 0, st>>>(n, curIdx, curNode, nodes.p, curLo, curHi, pflags.p, pbefore.p,
-                                                        altIdx, altNode, altLo, altHi, counters.p + 2);
-    std::swap(curIdx, altIdx);
-    std::swap(curNode, altNode);
-    std::swap(curLo, altLo);
-    std::swap(curHi, altHi);
-    std::swap(curTasks, nxtTasks);
-    cudaMemcpyAsync(&numTasks, counters.p + 1, sizeof(int), cudaMemcpyDeviceToHost, st);
-    if (cudaStreamSynchronize(st) != cudaSuccess) {
-      err = "BVH build level failed";
-      return RG_ERR_CUDA;
+    // scratch of the partition's prefix sum
+    const auto flagsOf = [&](const int* node, const float4* l, const float4* h) {
+      return thrust::make_transform_iterator(thrust::counting_iterator<int>(0), LeftFlag{node, nodes.p, l, h, nbins});
+    };
+    size_t scanBytes = 0;
+    cub::DeviceScan::ExclusiveSum(nullptr, scanBytes, flagsOf(curNode, curLo, curHi), pbefore.p, n, st);
+    DevBuf<unsigned char>& scanTmp = X.scanTmp;
+    if (!scanTmp.alloc(scanBytes + 16)) {
+      err = "out of device memory (BVH build)";
+      return RG_ERR_OUT_OF_MEMORY;
     }
-    trace.mark("level", levels, tasksThisLevel);
-    if (levels > 200) {
-      err = "BVH build did not converge";
-      return RG_ERR_DEVICE_STATUS;
+    // The levels a balanced tree takes to reach openCount, and two, are launched without
+    // waiting (task counts stay on the device; a level without tasks copies the primitives);
+    // then the host looks at the count before each further level.
+    int ahead = 2;
+    for (long long c = n; c > openCount; c = (c + 1) / 2) ahead++;
+    int numTasks = 1;
+    while (numTasks > 0) {
+      const int most = (int)std::min<long long>(levels < 31 ? 1ll << levels : (long long)maxOpen, maxOpen);
+      const int* count = levelCount.p + levels;
+      int* nextCount = levelCount.p + levels + 1;
+      for (int c0 = 0; c0 < most; c0 += chunkTasks) {
+        const int nt = std::min(chunkTasks, most - c0);
+        k_prepareLevel<<<gridFor(warpSplit ? nt : (long long)nt * nbins, 256), 256, 0, st>>>(count, c0, nt, curTasks, nodes.p,
+                                                                                          bins.p, nbins, !warpSplit);
+        if (warpSplit) {
+          k_bin<<<gridFor(n, kBinChunk), 256, 0, st>>>(n, curNode, nodes.p, curLo, curHi, bins.p, nbins);
+          k_splitWarp<<<gridFor((long long)nt * 32, 128), 128, 0, st>>>(
+              count, c0, nt, curTasks, nodes.p, bins.p, nbins, counters.p + C_NODES, nxtTasks, nextCount, smallTasks.p,
+              counters.p + C_SMALL, wide ? kWideMaxLeaf : kMaxLeaf);
+        } else {
+          k_binAny<<<gridFor(n, kBinChunk), 256, 0, st>>>(n, curNode, nodes.p, curLo, curHi, bins.p, nbins);
+          k_split<<<gridFor(nt, 128), 128, 0, st>>>(count, c0, nt, curTasks, nodes.p, bins.p, nbins, counters.p + C_NODES,
+                                                     nxtTasks, nextCount, wide ? kWideMaxLeaf : kMaxLeaf);
+        }
+      }
+      cub::DeviceScan::ExclusiveSum(scanTmp.p, scanBytes, flagsOf(curNode, curLo, curHi), pbefore.p, n, st);
+      k_partitionScatter<<<gridFor(n, 256), 256, 0, st>>>(n, curIdx, curNode, nodes.p, curLo, curHi, nbins, pbefore.p, altIdx,
+                                                          altNode, altLo, altHi, openCount, counters.p + C_BUILD_ERROR);
+      std::swap(curIdx, altIdx);
+      std::swap(curNode, altNode);
+      std::swap(curLo, altLo);
+      std::swap(curHi, altHi);
+      std::swap(curTasks, nxtTasks);
+      levels++;
+      if (levels >= ahead) {
+        cudaMemcpyAsync(&numTasks, nextCount, sizeof(int), cudaMemcpyDeviceToHost, st);
+        if (cudaStreamSynchronize(st) != cudaSuccess) {
+          err = "BVH build level failed";
+          return RG_ERR_CUDA;
+        }
+        trace.mark("levels", levels, numTasks);
+        if (numTasks > 0 && levels >= kMaxLevels) {
+          err = "BVH build did not converge";
+          return RG_ERR_DEVICE_STATUS;
+        }
+      }
     }
   }
-  int numNodes = 0, buildErr = 0;
-  cudaMemcpyAsync(&numNodes, counters.p, sizeof(int), cudaMemcpyDeviceToHost, st);
-  cudaMemcpyAsync(&buildErr, counters.p + 2, sizeof(int), cudaMemcpyDeviceToHost, st);
-  cudaStreamSynchronize(st);
-  if (buildErr != 0) {
-    err = "BVH build scatter error " + std::to_string(buildErr);
-    return RG_ERR_DEVICE_STATUS;
-  }
+  if (warpSplit && n > 4)
+    k_subtrees<<<std::min(n / 5 + 1, 148 * 8), kSubThreads, 0, st>>>(counters.p + C_SMALL, smallTasks.p, nodes.p, curIdx,
+                                                                    curLo, curHi, nbins, counters.p + C_NODES,
+                                                                    wide ? kWideMaxLeaf : kMaxLeaf);
   ds.buildLevels = levels;
-  trace.mark("levels end", 0, n);
   if (!ds.triVerts.alloc((size_t)n * 3) || !ds.triShade.alloc((size_t)n * 3) || !ds.triOrig.alloc(n)) {
     err = "out of device memory (triangles)";
     return RG_ERR_OUT_OF_MEMORY;
@@ -1002,60 +1278,57 @@ rg_status buildDeviceBvh(DeviceScene& ds, int nbins, bool wide, cudaStream_t st,
   }
   trace.mark("alloc tris", 0, n);
   if (wide) {
-    // collapse to the 8-wide compressed layout, level by level
+    // collapse to the 8-wide layout, level by level, the task counts on the device; an inner
+    // binary node has five primitives or more, which bounds the tasks of a level
     ds.bvhWidth = 8;
-    const int maxTasks8 = numNodes + 1;
     DevBuf<int2> &ta = X.ta, &tb = X.tb;
     DevBuf<int> &order = X.order, &c8 = X.c8;
-    if (!ta.alloc(maxTasks8) || !tb.alloc(maxTasks8) || !order.alloc(n) || !c8.alloc(4)) {
+    // the node array: as allocated, or about what scenes need (0.08-0.13 nodes a triangle)
+    int cap = (int)std::max<size_t>(ds.nodes8.n / kNode8Vec, (size_t)n / 7 + 64);
+    if (!ta.alloc((size_t)n / 5 + 2) || !tb.alloc((size_t)n / 5 + 2) || !order.alloc(n) || !c8.alloc(2) ||
+        !ds.nodes8.alloc((size_t)cap * kNode8Vec)) {
       err = "out of device memory (wide BVH)";
       return RG_ERR_OUT_OF_MEMORY;
     }
-    // two passes over the levels: the first counts the 8-wide nodes, so the node
-    // array is allocated at its size (about a seventh of the binary node count)
-    int numNodes8 = 0;
-    for (int pass = 0; pass < 2; pass++) {
-      const bool countOnly = pass == 0;
-      if (!countOnly && !ds.nodes8.alloc((size_t)numNodes8 * kNode8Vec)) {
-        err = "out of device memory (wide BVH)";
-        return RG_ERR_OUT_OF_MEMORY;
-      }
-      trace.mark(countOnly ? "count wide" : "alloc wide", 0, numNodes8);
-      const int init[4] = {1, 0, 0, 0};  // [0] nodes (root preallocated) [1] triangles [2] next tasks [3] error
-      cudaMemcpyAsync(c8.p, init, sizeof(init), cudaMemcpyHostToDevice, st);
-      const int2 root = make_int2(0, 0);
-      cudaMemcpyAsync(ta.p, &root, sizeof(int2), cudaMemcpyHostToDevice, st);
-      int nt = 1;
+    int h8[2] = {0, 0}, buildErr = 0;  // nodes, triangles
+    for (int pass = 0;; pass++) {
+      cudaMemsetAsync(levelCount.p, 0, sizeof(int) * (kMaxLevels + 2), st);
+      k_initCollapse<<<1, 1, 0, st>>>(c8.p, levelCount.p, ta.p);
       int2* cur = ta.p;
       int2* nxt = tb.p;
-      int lv = 0;
-      while (nt > 0) {
-        cudaMemsetAsync(c8.p + 2, 0, sizeof(int), st);
-        k_collapse<<<gridFor(nt, 64), 64, 0, st>>>(nt, cur, nodes.p, curIdx, ds.nodes8.p, c8.p, nxt, order.p,
-                                                   numNodes8, countOnly);
-        cudaMemcpyAsync(&nt, c8.p + 2, sizeof(int), cudaMemcpyDeviceToHost, st);
+      int more = 1, lv = 0, ahead = 2;
+      for (long long c = n; c > 4; c /= 6) ahead++;
+      while (more > 0) {
+        const long long most = std::min<long long>((long long)n / 5 + 2, lv < 10 ? 1ll << (3 * lv) : (long long)n);
+        k_collapse<<<(int)std::min<long long>((most + 63) / 64, 148 * 24), 64, 0, st>>>(
+            levelCount.p + lv, cur, nodes.p, curIdx, ds.nodes8.p, c8.p, nxt, levelCount.p + lv + 1, order.p, cap);
+        std::swap(cur, nxt);
+        if (++lv < ahead) continue;
+        cudaMemcpyAsync(&more, levelCount.p + lv, sizeof(int), cudaMemcpyDeviceToHost, st);
+        cudaMemcpyAsync(h8, c8.p, sizeof(h8), cudaMemcpyDeviceToHost, st);
+        cudaMemcpyAsync(&buildErr, counters.p + C_BUILD_ERROR, sizeof(int), cudaMemcpyDeviceToHost, st);
         if (cudaStreamSynchronize(st) != cudaSuccess) {
           err = "wide BVH collapse failed";
           return RG_ERR_CUDA;
         }
-        if (!countOnly) trace.mark("collapse", lv + 1, nt);
-        std::swap(cur, nxt);
-        if (++lv > 200) {
+        trace.mark("collapse", lv, h8[0]);
+        if (buildErr != 0) {
+          err = "BVH build scatter error " + std::to_string(buildErr);
+          return RG_ERR_DEVICE_STATUS;
+        }
+        if (more > 0 && lv >= kMaxLevels) {
           err = "wide BVH collapse did not converge";
           return RG_ERR_DEVICE_STATUS;
         }
       }
-      if (countOnly) {
-        if (cudaMemcpy(&numNodes8, c8.p, sizeof(int), cudaMemcpyDeviceToHost) != cudaSuccess || numNodes8 < 1 ||
-            numNodes8 > maxTasks8) {
-          err = "wide BVH node count failed";
-          return RG_ERR_DEVICE_STATUS;
-        }
+      if (h8[0] <= cap || pass > 0) break;
+      cap = h8[0];  // more nodes than the array held: once more with the exact size
+      if (!ds.nodes8.alloc((size_t)cap * kNode8Vec)) {
+        err = "out of device memory (wide BVH)";
+        return RG_ERR_OUT_OF_MEMORY;
       }
     }
-    int h8[4];
-    cudaMemcpy(h8, c8.p, sizeof(h8), cudaMemcpyDeviceToHost);
-    if (h8[3] != 0 || h8[1] != n || h8[0] != numNodes8) {
+    if (h8[1] != n || h8[0] < 1 || h8[0] > cap) {
       err = "wide BVH collapse error (nodes " + std::to_string(h8[0]) + ", triangles " + std::to_string(h8[1]) + ")";
       return RG_ERR_DEVICE_STATUS;
     }
@@ -1071,6 +1344,17 @@ rg_status buildDeviceBvh(DeviceScene& ds, int nbins, bool wide, cudaStream_t st,
     return RG_OK;
   }
   // binary traversal layout
+  int numNodes = 0, buildErr = 0;
+  cudaMemcpyAsync(&numNodes, counters.p + C_NODES, sizeof(int), cudaMemcpyDeviceToHost, st);
+  cudaMemcpyAsync(&buildErr, counters.p + C_BUILD_ERROR, sizeof(int), cudaMemcpyDeviceToHost, st);
+  if (cudaStreamSynchronize(st) != cudaSuccess) {
+    err = "BVH build failed";
+    return RG_ERR_CUDA;
+  }
+  if (buildErr != 0) {
+    err = "BVH build scatter error " + std::to_string(buildErr);
+    return RG_ERR_DEVICE_STATUS;
+  }
   ds.bvhWidth = 2;
   DevBuf<int> &flags = X.flags, &trav = X.trav;
   if (!flags.alloc(numNodes) || !trav.alloc(numNodes)) {
