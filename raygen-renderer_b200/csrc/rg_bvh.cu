@@ -18,8 +18,6 @@
 #include <cstdlib>
 #include <climits>
 #include <cub/device/device_scan.cuh>
-#include <thrust/iterator/counting_iterator.h>
-#include <thrust/iterator/transform_iterator.h>
 #include <cuda_fp16.h>
 
 #include <cfloat>
@@ -819,33 +817,40 @@ __global__ void __launch_bounds__(kSubThreads) k_subtrees(const int* __restrict_
   }
 }
 
-// 1 for a primitive that goes to the left child of its node (the split bin, or the first half
-// of the node's range for a median split); the input of the partition's prefix sum.
-struct LeftFlag {
-  const int* primNode;
-  const BNode* nodes;
-  const float4 *bmin, *bmax;
-  int nbins;
-  __device__ __forceinline__ int operator()(int i) const {
-    const int node = primNode[i];
-    if (node < 0) return 0;
+// Partition, pass 1: flag 1 for a primitive that goes to the left child of its
+// node (the split bin, or the first half of the node's range for a median split).
+// A pass of its own: computed inside the prefix sum the flags cost more (4M primitives 66
+// against 31 + 12 us, 20k 31 against 10).
+__global__ void k_partitionFlags(int n, const int* __restrict__ primNode, const BNode* __restrict__ nodes,
+                                 const float4* __restrict__ bmin, const float4* __restrict__ bmax, int nbins,
+                                 int* __restrict__ flags) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= n) return;
+  const int node = primNode[i];
+  int flag = 0;
+  if (node >= 0) {
     const BNode& nd = nodes[node];
-    if (nd.left < 0) return 0;
-    if (nd.splitBin == -2) return (i - nd.start) < nd.count / 2 ? 1 : 0;
-    const float c = (axisOf(bmin[i], nd.axis) + axisOf(bmax[i], nd.axis)) * 0.5f;
-    return binOf(nd, c, nbins) <= nd.splitBin ? 1 : 0;
+    if (nd.left >= 0) {
+      if (nd.splitBin == -2) {
+        flag = (i - nd.start) < nd.count / 2 ? 1 : 0;
+      } else {
+        const float c = (axisOf(bmin[i], nd.axis) + axisOf(bmax[i], nd.axis)) * 0.5f;
+        flag = binOf(nd, c, nbins) <= nd.splitBin ? 1 : 0;
+      }
+    }
   }
-};
+  flags[i] = flag;
+}
 
-// Partition, after an exclusive scan of the flags into `before`: a stable
+// Partition, pass 2 (after an exclusive scan of the flags into `before`): a stable
 // scatter of each split node's primitives into its children's ranges, with their
 // bounds; primitives of closed nodes and new leaves stay where they are.  No
 // atomics, so the order (and the BVH) is the same on every run.
 __global__ void k_partitionScatter(int n, const int* __restrict__ primIdx, const int* __restrict__ primNode,
                                    const BNode* __restrict__ nodes, const float4* __restrict__ bmin,
-                                   const float4* __restrict__ bmax, int nbins, const int* __restrict__ before,
-                                   int* __restrict__ outIdx, int* __restrict__ outNode, float4* __restrict__ outMin,
-                                   float4* __restrict__ outMax, int openCount, int* err) {
+                                   const float4* __restrict__ bmax, const int* __restrict__ flags,
+                                   const int* __restrict__ before, int* __restrict__ outIdx, int* __restrict__ outNode,
+                                   float4* __restrict__ outMin, float4* __restrict__ outMax, int openCount, int* err) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
   const int node = primNode[i];
@@ -854,7 +859,7 @@ __global__ void k_partitionScatter(int n, const int* __restrict__ primIdx, const
     const BNode& nd = nodes[node];
     if (nd.left >= 0) {
       const int leftBefore = before[i] - before[nd.start];
-      const int side = LeftFlag{primNode, nodes, bmin, bmax, nbins}(i) ? 0 : 1;
+      const int side = flags[i] ? 0 : 1;
       const int rank = side == 0 ? leftBefore : (i - nd.start) - leftBefore;
       const BNode& cn = nodes[nd.left + side];
       if (rank >= cn.count) {
@@ -928,163 +933,192 @@ __global__ void k_gather(int n, const int* __restrict__ primIdx, const float4* _
 // Slots are assigned per octant: a child whose centre lies on the negative side
 // of the node centre along axis k prefers slots with bit k set, so visiting hit
 // slots in descending order of (slot XOR ray octant) is roughly front to back.
-// One task: binary node task.x becomes wide node task.y.  Nodes past maxNodes8 are counted
-// and their children followed, but not written (the host then sizes the array and repeats).
-__device__ __forceinline__ void collapseTask(int2 task, const BNode* __restrict__ nodes, const int* __restrict__ primIdx,
-                                             float4* __restrict__ nodes8, int* counters, int2* __restrict__ nextTasks,
-                                             int* nextCount, int* __restrict__ triOrder, int maxNodes8) {
-  const BNode& nd = nodes[task.x];
-  int ch[8];
-  int nc;
-  if (nd.left < 0) {
-    ch[0] = task.x;
-    nc = 1;
-  } else {
-    ch[0] = nd.left;
-    ch[1] = nd.left + 1;
-    nc = 2;
-    while (nc < 8) {
-      int best = -1;
-      float bestA = -1.0f;
-      for (int i = 0; i < nc; i++) {
-        const BNode& c = nodes[ch[i]];
-        if (c.left < 0) continue;
-        const float a = areaOf(c.bmin, c.bmax);
-        if (a > bestA) { bestA = a; best = i; }
-      }
-      if (best < 0) break;
-      const int l = nodes[ch[best]].left;
-      ch[best] = l;
-      ch[nc++] = l + 1;
-    }
-  }
-  float lo[3] = {FLT_MAX, FLT_MAX, FLT_MAX}, hi[3] = {-FLT_MAX, -FLT_MAX, -FLT_MAX};
-  float cc[8][3];
-  for (int i = 0; i < nc; i++) {
-    const BNode& c = nodes[ch[i]];
-    for (int k = 0; k < 3; k++) {
-      const float a = inflateLo(c.bmin[k]), b = inflateHi(c.bmax[k]);
-      lo[k] = fminf(lo[k], a);
-      hi[k] = fmaxf(hi[k], b);
-      cc[i][k] = 0.5f * (c.bmin[k] + c.bmax[k]);
-    }
-  }
-  // greedy octant slot assignment
-  int slotOf[8];
-  bool slotUsed[8] = {false, false, false, false, false, false, false, false};
-  bool childDone[8] = {false, false, false, false, false, false, false, false};
-  const float ctr[3] = {0.5f * (lo[0] + hi[0]), 0.5f * (lo[1] + hi[1]), 0.5f * (lo[2] + hi[2])};
-  for (int it = 0; it < nc; it++) {
-    float bestS = -FLT_MAX;
-    int bj = -1, bs = -1;
-    for (int j = 0; j < nc; j++) {
-      if (childDone[j]) continue;
-      for (int sl = 0; sl < 8; sl++) {
-        if (slotUsed[sl]) continue;
-        const float sc = (cc[j][0] - ctr[0]) * ((sl & 1) ? -1.0f : 1.0f) + (cc[j][1] - ctr[1]) * ((sl & 2) ? -1.0f : 1.0f) +
-                         (cc[j][2] - ctr[2]) * ((sl & 4) ? -1.0f : 1.0f);
-        if (sc > bestS) { bestS = sc; bj = j; bs = sl; }
-      }
-    }
-    childDone[bj] = true;
-    slotUsed[bs] = true;
-    slotOf[bj] = bs;
-  }
-  int childAt[8];
-  for (int sl = 0; sl < 8; sl++) childAt[sl] = -1;
-  for (int j = 0; j < nc; j++) childAt[slotOf[j]] = ch[j];
-  // planes of the child boxes (each widened by the inflate margin) as half values; an
-  // empty slot keeps an inverted box.  A node that is not of finite size has boxes
-  // that every ray enters.
-  // The origin of the planes is, per axis, the node's low end, centre or high end: the one
-  // closest to the planes of thin boxes (walls, floors, lamps), whose rounding matters most
-  // because rays start and end at such surfaces.
-  float org[3], ext = 0.0f;
-  for (int k = 0; k < 3; k++) {
-    const float cand[3] = {ctr[k], lo[k], hi[k]}, thin = (hi[k] - lo[k]) * (1.0f / 256.0f);
-    float best = FLT_MAX;
-    org[k] = ctr[k];
-    for (int q = 0; q < 3; q++) {
-      float cost = 0.0f;
-      for (int i = 0; i < nc; i++) {
-        const BNode& c = nodes[ch[i]];
-        cost += (fabsf(c.bmin[k] - cand[q]) + fabsf(c.bmax[k] - cand[q])) / (c.bmax[k] - c.bmin[k] + thin);
-      }
-      if (cost < best) {
-        best = cost;
-        org[k] = cand[q];
-      }
-    }
-    ext = fmaxf(ext, fmaxf(__fsub_ru(hi[k], org[k]), __fsub_ru(org[k], lo[k])));
-  }
-  const bool finite = ext < 1e30f;
-  int exponent = 0;
-  if (finite) frexpf(ext, &exponent);  // ext < 2^exponent
-  exponent = max(exponent - 15, -126);
-  const float scale = ldexpf(1.0f, exponent), toHalf = ldexpf(1.0f, -exponent);
-  __half pl[3][2][8];
-  for (int k = 0; k < 3; k++)
-    for (int sl = 0; sl < 8; sl++) {
-      pl[k][0][sl] = __float2half_rn(65504.0f);
-      pl[k][1][sl] = __float2half_rn(-65504.0f);
-    }
-  uint32_t meta[2] = {0, 0}, inner = 0;
-  int ni = 0, ntri = 0;
-  for (int sl = 0; sl < 8; sl++) {
-    const int c = childAt[sl];
-    if (c < 0) continue;
-    const BNode& cn = nodes[c];
-    for (int k = 0; k < 3; k++) {
-      pl[k][0][sl] = finite ? __float2half_rd(__fsub_rd(inflateLo(cn.bmin[k]), org[k]) * toHalf) : __float2half_rd(-INFINITY);
-      pl[k][1][sl] = finite ? __float2half_ru(__fsub_ru(inflateHi(cn.bmax[k]), org[k]) * toHalf) : __float2half_ru(INFINITY);
-    }
-    if (cn.left >= 0) {
-      inner |= 1u << sl;
-      ni++;
-    } else {
-      meta[sl >> 2] |= (uint32_t)((cn.count << 5) | ntri) << (8 * (sl & 3));
-      ntri += cn.count;
-    }
-  }
-  const int childBase = ni ? atomicAdd(&counters[0], ni) : 0;
-  const int triBase = atomicAdd(&counters[1], ntri);
-  const bool fits = task.y < maxNodes8;
-  float4* o = nodes8 + (size_t)(fits ? task.y : 0) * kNode8Vec;
-  const int sw = task.y & 7;
-  if (fits) {
-  o[0 ^ sw] = make_float4(__int_as_float(childBase), __int_as_float(triBase), __uint_as_float(meta[0]), __uint_as_float(meta[1]));
-  o[1 ^ sw] = make_float4(finite ? org[0] : 0.0f, finite ? org[1] : 0.0f, finite ? org[2] : 0.0f,
-                     __uint_as_float(__float_as_uint(scale) | inner));
-  for (int k = 0; k < 3; k++)
-    for (int h = 0; h < 2; h++) {
-      __align__(16) __half2 q[4];
-      for (int j = 0; j < 4; j++) q[j] = __halves2half2(pl[k][h][2 * j], pl[k][h][2 * j + 1]);
-      o[(2 + 2 * k + h) ^ sw] = *reinterpret_cast<const float4*>(q);
-    }
-  }
-  int k = 0, off = 0;
-  for (int sl = 0; sl < 8; sl++) {
-    const int c = childAt[sl];
-    if (c < 0) continue;
-    const BNode& cn = nodes[c];
-    if (cn.left >= 0) {
-      const int slot = atomicAdd(nextCount, 1);
-      nextTasks[slot] = make_int2(c, childBase + k);
-      k++;
-    } else {
-      for (int q = 0; q < cn.count; q++) triOrder[triBase + off + q] = primIdx[cn.start + q];
-      off += cn.count;
-    }
-  }
-}
-
-__global__ void __launch_bounds__(64) k_collapse(const int* __restrict__ count, const int2* __restrict__ tasks,
-                                                 const BNode* __restrict__ nodes, const int* __restrict__ primIdx,
-                                                 float4* __restrict__ nodes8, int* counters, int2* __restrict__ nextTasks,
-                                                 int* nextCount, int* __restrict__ triOrder, int maxNodes8) {
+// Eight lanes collapse one task (binary node task.x becomes wide node task.y), a lane per child
+// and then per slot: one thread per node took 53 us a level, the latency of its chain of
+// node reads and 8 x 8 slot scores, whatever the number of nodes.  Nodes past maxNodes8 are
+// counted and their children followed, but not written (the host then sizes the array and
+// repeats).
+__global__ void __launch_bounds__(128) k_collapse(const int* __restrict__ count, const int2* __restrict__ tasks,
+                                                  const BNode* __restrict__ nodes, const int* __restrict__ primIdx,
+                                                  float4* __restrict__ nodes8, int* counters, int2* __restrict__ nextTasks,
+                                                  int* nextCount, int* __restrict__ triOrder, int maxNodes8) {
+  constexpr unsigned kAll = 0xffffffffu;
   const int numTasks = *count;
-  for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < numTasks; t += gridDim.x * blockDim.x)
-    collapseTask(tasks[t], nodes, primIdx, nodes8, counters, nextTasks, nextCount, triOrder, maxNodes8);
+  const int lane = threadIdx.x & 7, shift = threadIdx.x & 24;  // lane of the node's eight, their place in the warp
+  auto of = [&](auto v, int l) { return __shfl_sync(kAll, v, l, 8); };
+  auto minOf = [&](float v) {
+    for (int o = 4; o > 0; o >>= 1) v = fminf(v, __shfl_xor_sync(kAll, v, o));
+    return v;
+  };
+  auto maxOf = [&](float v) {
+    for (int o = 4; o > 0; o >>= 1) v = fmaxf(v, __shfl_xor_sync(kAll, v, o));
+    return v;
+  };
+  auto sumOf = [&](float v) {
+    for (int o = 4; o > 0; o >>= 1) v += __shfl_xor_sync(kAll, v, o);
+    return v;
+  };
+  const int stride = (int)(gridDim.x * blockDim.x) >> 3;
+  // whole warps: a group past the last task goes along without one
+  for (int t0 = (int)(blockIdx.x * blockDim.x + (threadIdx.x & ~31)) >> 3; t0 < numTasks; t0 += stride) {
+    const int t = t0 + (shift >> 3);
+    const bool on = t < numTasks;
+    const int2 task = on ? tasks[t] : make_int2(0, 0);
+    // children by opening the inner child of the largest area until there are eight
+    int id = -1, left = -1, cnt = 0, first = 0;
+    float bmin[3] = {0, 0, 0}, bmax[3] = {0, 0, 0}, area = -1.0f;
+    auto load = [&](int node) {
+      const BNode& c = nodes[node];
+      id = node;
+      left = c.left;
+      cnt = c.count;
+      first = c.start;
+      for (int k = 0; k < 3; k++) {
+        bmin[k] = c.bmin[k];
+        bmax[k] = c.bmax[k];
+      }
+      area = left >= 0 ? areaOf(bmin, bmax) : -1.0f;
+    };
+    int nc = on ? 1 : 0;
+    const int rootLeft = on ? nodes[task.x].left : -1;
+    if (on) {
+      if (rootLeft < 0) {
+        if (lane == 0) load(task.x);
+      } else {
+        nc = 2;
+        if (lane < 2) load(rootLeft + lane);
+      }
+    }
+    for (int it = 0; it < 6; it++) {
+      const float best = maxOf(area);
+      const unsigned m = (__ballot_sync(kAll, area == best && best >= 0.0f) >> shift) & 0xffu;
+      if (__ballot_sync(kAll, m != 0 && nc < 8) == 0) break;
+      const int who = m ? __ffs(m) - 1 : 0;  // the first of equal areas
+      const int l = of(left, who);
+      if (m && nc < 8) {
+        if (lane == who) load(l);
+        else if (lane == nc) load(l + 1);
+        nc++;
+      }
+    }
+    // node bounds of the widened child boxes, their centre, and greedy octant slots
+    const bool mine = lane < nc;
+    float lo[3], hi[3], ctr[3], cc[3];
+    for (int k = 0; k < 3; k++) {
+      lo[k] = minOf(mine ? inflateLo(bmin[k]) : FLT_MAX);
+      hi[k] = maxOf(mine ? inflateHi(bmax[k]) : -FLT_MAX);
+      ctr[k] = 0.5f * (lo[k] + hi[k]);
+      cc[k] = 0.5f * (bmin[k] + bmax[k]);
+    }
+    int slot = -1;
+    unsigned used = 0;
+    for (int it = 0; it < 8; it++) {
+      float bestS = -INFINITY;
+      int bs = -1;
+      if (mine && slot < 0)
+        for (int sl = 0; sl < 8; sl++) {
+          if ((used >> sl) & 1u) continue;
+          const float sc = (cc[0] - ctr[0]) * ((sl & 1) ? -1.0f : 1.0f) + (cc[1] - ctr[1]) * ((sl & 2) ? -1.0f : 1.0f) +
+                           (cc[2] - ctr[2]) * ((sl & 4) ? -1.0f : 1.0f);
+          if (bs < 0 || sc > bestS) { bestS = sc; bs = sl; }
+        }
+      const bool cand = bs >= 0;
+      const float top = maxOf(cand ? bestS : -INFINITY);
+      unsigned m = (__ballot_sync(kAll, cand && bestS == top) >> shift) & 0xffu;
+      const unsigned anyCand = (__ballot_sync(kAll, cand) >> shift) & 0xffu;
+      if (__ballot_sync(kAll, anyCand != 0) == 0) break;
+      if (!m) m = anyCand;  // scores that are no numbers: any order will do
+      const int who = m ? __ffs(m) - 1 : 0;
+      const int s = of(bs, who);
+      if (m) {
+        used |= 1u << s;
+        if (lane == who) slot = s;
+      }
+    }
+    // from here a lane stands for slot `lane`
+    int from = -1;
+    for (int j = 0; j < 8; j++)
+      if (of(slot, j) == lane) from = j;
+    const bool full = from >= 0;
+    const int src = full ? from : lane;
+    const int cId = of(id, src), cLeft = of(left, src), cCnt = of(cnt, src), cFirst = of(first, src);
+    float cMin[3], cMax[3];
+    for (int k = 0; k < 3; k++) {
+      cMin[k] = of(bmin[k], src);
+      cMax[k] = of(bmax[k], src);
+    }
+    const bool inner = full && cLeft >= 0, leaf = full && cLeft < 0;
+    const unsigned innerMask = (__ballot_sync(kAll, inner) >> shift) & 0xffu;
+    const int ni = __popc(innerMask), rank = __popc(innerMask & ((1u << lane) - 1u));
+    int off = leaf ? cCnt : 0;  // triangles of the slots up to this one
+    for (int o = 1; o < 8; o <<= 1) {
+      const int up = __shfl_up_sync(kAll, off, o, 8);
+      if (lane >= o) off += up;
+    }
+    const int ntri = of(off, 7);
+    off -= leaf ? cCnt : 0;
+    int childBase = 0, triBase = 0, taskBase = 0;
+    if (lane == 0 && on) {
+      if (ni) {
+        childBase = atomicAdd(&counters[0], ni);
+        taskBase = atomicAdd(nextCount, ni);
+      }
+      triBase = atomicAdd(&counters[1], ntri);
+    }
+    childBase = of(childBase, 0);
+    triBase = of(triBase, 0);
+    taskBase = of(taskBase, 0);
+    if (on && inner) nextTasks[taskBase + rank] = make_int2(cId, childBase + rank);
+    if (on && leaf)
+      for (int q = 0; q < cCnt; q++) triOrder[triBase + off + q] = primIdx[cFirst + q];
+    // The origin of the planes is, per axis, the node's low end, centre or high end: the one
+    // closest to the planes of thin boxes (walls, floors, lamps), whose rounding matters most
+    // because rays start and end at such surfaces.
+    float org[3], ext = 0.0f;
+    for (int k = 0; k < 3; k++) {
+      const float cand[3] = {ctr[k], lo[k], hi[k]}, thin = (hi[k] - lo[k]) * (1.0f / 256.0f);
+      float best = FLT_MAX;
+      org[k] = ctr[k];
+      for (int q = 0; q < 3; q++) {
+        const float cost =
+            sumOf(full ? (fabsf(cMin[k] - cand[q]) + fabsf(cMax[k] - cand[q])) / (cMax[k] - cMin[k] + thin) : 0.0f);
+        if (cost < best) {
+          best = cost;
+          org[k] = cand[q];
+        }
+      }
+      ext = fmaxf(ext, fmaxf(__fsub_ru(hi[k], org[k]), __fsub_ru(org[k], lo[k])));
+    }
+    // planes as half values, rounded outward; an empty slot keeps an inverted box, and a node
+    // that is not of finite size has boxes that every ray enters
+    const bool finite = ext < 1e30f;
+    int exponent = 0;
+    if (finite) frexpf(ext, &exponent);  // ext < 2^exponent
+    exponent = max(exponent - 15, -126);
+    const float scale = ldexpf(1.0f, exponent), toHalf = ldexpf(1.0f, -exponent);
+    uint32_t meta = leaf ? (uint32_t)((cCnt << 5) | off) << (8 * (lane & 3)) : 0u;
+    meta |= __shfl_xor_sync(kAll, meta, 1);
+    meta |= __shfl_xor_sync(kAll, meta, 2);
+    const uint32_t meta1 = of(meta, 4);
+    if (!on || task.y >= maxNodes8) continue;
+    float4* o = nodes8 + (size_t)task.y * kNode8Vec;
+    const int sw = task.y & 7;
+    for (int k = 0; k < 3; k++)
+      for (int h = 0; h < 2; h++) {
+        __half v = __float2half_rn(h ? -65504.0f : 65504.0f);
+        if (full) {
+          if (!finite) v = h ? __float2half_ru(INFINITY) : __float2half_rd(-INFINITY);
+          else if (h) v = __float2half_ru(__fsub_ru(inflateHi(cMax[k]), org[k]) * toHalf);
+          else v = __float2half_rd(__fsub_rd(inflateLo(cMin[k]), org[k]) * toHalf);
+        }
+        reinterpret_cast<__half*>(o + ((2 + 2 * k + h) ^ sw))[lane] = v;
+      }
+    if (lane == 0) {
+      o[0 ^ sw] = make_float4(__int_as_float(childBase), __int_as_float(triBase), __uint_as_float(meta), __uint_as_float(meta1));
+      o[1 ^ sw] = make_float4(finite ? org[0] : 0.0f, finite ? org[1] : 0.0f, finite ? org[2] : 0.0f,
+                              __uint_as_float(__float_as_uint(scale) | innerMask));
+    }
+  }
 }
 
 __global__ void k_initCollapse(int* counters, int* levelCount, int2* tasks) {
@@ -1120,7 +1154,7 @@ struct BvhScratch {
   DevBuf<float2> uvTmp;
   DevBuf<uint32_t> rb;
   DevBuf<BNode> nodes;
-  DevBuf<int> idxA, idxB, nodeA, nodeB, tasksA, tasksB, smallTasks, counters, levelCount, pbefore;
+  DevBuf<int> idxA, idxB, nodeA, nodeB, tasksA, tasksB, smallTasks, counters, levelCount, pflags, pbefore;
   DevBuf<BinData> bins;
   DevBuf<unsigned char> scanTmp, tmp;
   DevBuf<int2> ta, tb;
@@ -1172,12 +1206,12 @@ rg_status buildDeviceBvh(DeviceScene& ds, int nbins, bool wide, cudaStream_t st,
   DevBuf<BNode>& nodes = X.nodes;
   DevBuf<int> &idxA = X.idxA, &idxB = X.idxB, &nodeA = X.nodeA, &nodeB = X.nodeB, &tasksA = X.tasksA,
   &tasksB = X.tasksB, &smallTasks = X.smallTasks, &counters = X.counters, &levelCount = X.levelCount,
-  &pbefore = X.pbefore;
+  &pflags = X.pflags, &pbefore = X.pbefore;
   DevBuf<BinData>& bins = X.bins;
   trace.mark("prep kern", 0, n);
   constexpr int kMaxLevels = 200;
   if (!nodes.alloc(maxNodes) || !idxA.alloc(n) || !idxB.alloc(n) || !nodeA.alloc(n) || !nodeB.alloc(n) ||
-      !lo2.alloc(n) || !hi2.alloc(n) || !pbefore.alloc(n) || !tasksA.alloc((size_t)maxOpen + 1) ||
+      !lo2.alloc(n) || !hi2.alloc(n) || !pflags.alloc(n) || !pbefore.alloc(n) || !tasksA.alloc((size_t)maxOpen + 1) ||
       !tasksB.alloc((size_t)maxOpen + 1) || !smallTasks.alloc((size_t)n / 5 + 2) || !counters.alloc(C_BUILD_COUNTERS) ||
       !levelCount.alloc(kMaxLevels + 2) || !bins.alloc((size_t)chunkTasks * nbins)) {
     err = "out of device memory (BVH build)";
@@ -1205,11 +1239,8 @@ rg_status buildDeviceBvh(DeviceScene& ds, int nbins, bool wide, cudaStream_t st,
       k_resetBins<<<(unsigned)((nb + 255) / 256), 256, 0, st>>>(nb, bins.p);
     }
     // scratch of the partition's prefix sum
-    const auto flagsOf = [&](const int* node, const float4* l, const float4* h) {
-      return thrust::make_transform_iterator(thrust::counting_iterator<int>(0), LeftFlag{node, nodes.p, l, h, nbins});
-    };
     size_t scanBytes = 0;
-    cub::DeviceScan::ExclusiveSum(nullptr, scanBytes, flagsOf(curNode, curLo, curHi), pbefore.p, n, st);
+    cub::DeviceScan::ExclusiveSum(nullptr, scanBytes, pflags.p, pbefore.p, n, st);
     DevBuf<unsigned char>& scanTmp = X.scanTmp;
     if (!scanTmp.alloc(scanBytes + 16)) {
       err = "out of device memory (BVH build)";
@@ -1240,8 +1271,9 @@ rg_status buildDeviceBvh(DeviceScene& ds, int nbins, bool wide, cudaStream_t st,
                                                      nxtTasks, nextCount, wide ? kWideMaxLeaf : kMaxLeaf);
         }
       }
-      cub::DeviceScan::ExclusiveSum(scanTmp.p, scanBytes, flagsOf(curNode, curLo, curHi), pbefore.p, n, st);
-      k_partitionScatter<<<gridFor(n, 256), 256, 0, st>>>(n, curIdx, curNode, nodes.p, curLo, curHi, nbins, pbefore.p, altIdx,
+      k_partitionFlags<<<gridFor(n, 256), 256, 0, st>>>(n, curNode, nodes.p, curLo, curHi, nbins, pflags.p);
+      cub::DeviceScan::ExclusiveSum(scanTmp.p, scanBytes, pflags.p, pbefore.p, n, st);
+      k_partitionScatter<<<gridFor(n, 256), 256, 0, st>>>(n, curIdx, curNode, nodes.p, curLo, curHi, pflags.p, pbefore.p, altIdx,
                                                           altNode, altLo, altHi, openCount, counters.p + C_BUILD_ERROR);
       std::swap(curIdx, altIdx);
       std::swap(curNode, altNode);
@@ -1300,7 +1332,7 @@ rg_status buildDeviceBvh(DeviceScene& ds, int nbins, bool wide, cudaStream_t st,
       for (long long c = n; c > 4; c /= 6) ahead++;
       while (more > 0) {
         const long long most = std::min<long long>((long long)n / 5 + 2, lv < 10 ? 1ll << (3 * lv) : (long long)n);
-        k_collapse<<<(int)std::min<long long>((most + 63) / 64, 148 * 24), 64, 0, st>>>(
+        k_collapse<<<(int)std::min<long long>((most + 15) / 16, 148 * 16), 128, 0, st>>>(
             levelCount.p + lv, cur, nodes.p, curIdx, ds.nodes8.p, c8.p, nxt, levelCount.p + lv + 1, order.p, cap);
         std::swap(cur, nxt);
         if (++lv < ahead) continue;
