@@ -785,7 +785,11 @@ __device__ __forceinline__ void traverseWave8(const DevScene& S0, const DevJob* 
   __shared__ uint2 sStack[kSharedStack > 0 ? kSharedStack : 1][kTraceBlock];
   uint2 lStack[kStack8 - kSharedStack];
   // triangle queue: entries [head, tail) modulo kTriQueue, head and tail alike in all lanes
-  __shared__ int2 sTri[kTraceWarps][kTriQueue];  // (triangle, owner lane)
+  __shared__ int2 sTri[kTraceWarps][kTriQueue];  // (triangle, owner lane | the owner's node step << 5)
+  // The node step that found the closest hit so far.  Of equal distances the triangle found
+  // first is the hit, as if each were tested when found, although a queued triangle may be
+  // tested after one found later.
+  __shared__ int sStep[ANY ? 1 : kTraceBlock];
   __shared__ unsigned sHits[kTraceWarps][32];  // per owner: the batch entries that hit
   int head = 0, tail = 0;
   int qEnd = 0;  // queue position after this lane's last entry
@@ -842,6 +846,7 @@ __device__ __forceinline__ void traverseWave8(const DevScene& S0, const DevJob* 
           }
           prim = -1;
           hu = hv = 0.0f;
+          if (!ANY) sStep[threadIdx.x] = 0;
           occluded = false;
           inv = safeInv(d);
           oct = rayOctant(inv);
@@ -905,7 +910,7 @@ __device__ __forceinline__ void traverseWave8(const DevScene& S0, const DevJob* 
             asm volatile("prefetch.global.L1 [%0];" ::"l"(nodesP + (size_t)nnode * kNode8Vec));
         }
       }
-      // ---- while most lanes hold triangles, each tests one of its own: the warp is full as it is
+      // ---- while many lanes hold triangles, each tests one of its own: the warp is full as it is
       while (__popc(__ballot_sync(kAll, tMask != 0)) >= (ANY ? kDirectAny : kDirectClosest)) {
         if (tMask) {
           const int tk = tBase + __ffs(tMask) - 1;
@@ -932,6 +937,7 @@ __device__ __forceinline__ void traverseWave8(const DevScene& S0, const DevJob* 
                 hu = h.u;
                 hv = h.v;
                 prim = tk;
+                sStep[threadIdx.x] = steps;
               }
             }
           }
@@ -952,7 +958,7 @@ __device__ __forceinline__ void traverseWave8(const DevScene& S0, const DevJob* 
           int at = tail + incl - n;
           qEnd = tail + incl;
           do {
-            sTri[warp][at & (kTriQueue - 1)] = make_int2(tBase + __ffs(tMask) - 1, lane);
+            sTri[warp][at & (kTriQueue - 1)] = make_int2(tBase + __ffs(tMask) - 1, lane | (steps << 5));
             tMask &= tMask - 1u;
             at++;
           } while (tMask);
@@ -966,7 +972,7 @@ __device__ __forceinline__ void traverseWave8(const DevScene& S0, const DevJob* 
         const int n = min(queued, 32);
         const bool mine = lane < n;
         const int2 entry = sTri[warp][(head + (mine ? lane : 0)) & (kTriQueue - 1)];
-        const int tk = entry.x, own = entry.y;
+        const int tk = entry.x, own = entry.y & 31;
         const V3 ro = v3(__shfl_sync(kAll, o.x, own), __shfl_sync(kAll, o.y, own), __shfl_sync(kAll, o.z, own));
         const V3 rd = v3(__shfl_sync(kAll, d.x, own), __shfl_sync(kAll, d.y, own), __shfl_sync(kAll, d.z, own));
         const float4* base = MULTI ? reinterpret_cast<const float4*>(
@@ -983,7 +989,7 @@ __device__ __forceinline__ void traverseWave8(const DevScene& S0, const DevJob* 
             const float4 a = ldTri4(tp), c = ldTri4(tp + 2);
             tris++;
             if (ANY) hit = mtAny(ro, rd, xyz(a), xyz(b), xyz(c), h.t);
-            else hit = mtClosest(ro, rd, xyz(a), xyz(b), xyz(c), h);
+            else hit = mtClosest<true>(ro, rd, xyz(a), xyz(b), xyz(c), h);
           }
         }
         head += n;
@@ -1001,13 +1007,15 @@ __device__ __forceinline__ void traverseWave8(const DevScene& S0, const DevJob* 
               tMask = 0;
             }
           } else {
-            int best = -1;
-            while (__any_sync(kAll, m != 0)) {  // in queue order: the first of equal distances stays
+            int best = -1, bestStep = m ? sStep[threadIdx.x] : 0;
+            while (__any_sync(kAll, m != 0)) {
               const int k = m ? __ffs(m) - 1 : lane;
               const float t = __shfl_sync(kAll, h.t, k);
-              if (m && t < tmax) {
+              const int step = __shfl_sync(kAll, entry.y, k) >> 5;
+              if (m && (t < tmax || (t == tmax && step < bestStep))) {
                 tmax = t;
                 best = k;
+                bestStep = step;
               }
               m &= m - 1u;
             }
@@ -1018,6 +1026,7 @@ __device__ __forceinline__ void traverseWave8(const DevScene& S0, const DevJob* 
               hu = u;
               hv = v;
               prim = p;
+              sStep[threadIdx.x] = bestStep;
             }
           }
         }

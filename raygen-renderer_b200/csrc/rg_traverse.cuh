@@ -61,7 +61,9 @@ struct ClosestHit {
 };
 
 // RenderMeshTriangle::intersectsRay(ray, info): raycommon.cpp:200-235
-// (dot / cross in the fixed FMA form of dot_f / cross_f, as in the oracle)
+// (dot / cross in the fixed FMA form of dot_f / cross_f, as in the oracle).  UP_TO: a hit at
+// exactly h.t counts too (the caller decides between equal distances).
+template <bool UP_TO = false>
 __device__ __forceinline__ bool mtClosest(V3 o, V3 d, V3 p1, V3 e1, V3 e2, ClosestHit& h) {
   const V3 pvec = cross_f(d, e2);
   const float det = dot_f(e1, pvec);
@@ -75,7 +77,7 @@ __device__ __forceinline__ bool mtClosest(V3 o, V3 d, V3 p1, V3 e1, V3 e2, Close
   if (v < 0.0f || __fadd_rn(u, v) > 1.0f) return false;
   const float t = __fmul_rn(dot_f(e2, qvec), invDet);
   if (t < 0.0f) return false;
-  if (t >= h.t) return false;
+  if (UP_TO ? t > h.t : t >= h.t) return false;
   h.t = t;
   h.u = u;
   h.v = v;
