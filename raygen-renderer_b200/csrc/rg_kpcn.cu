@@ -16,9 +16,10 @@
 //                  producer thread and four epilogue warps); B = weights;
 //   backward data  the same with the gradient, mirrored taps and transposed
 //                  weights, the ReLU mask of the layer input in the epilogue;
-//   backward wt.   rows = (tap, input channel), K = pixels (a chunk of 512
-//                  per CTA, 128 at a time), B = the output gradient;
-//                  per-chunk partials reduced in chunk order (deterministic).
+//   backward wt.   rows = (tap, input channel), K = pixels (a chunk of 512 or
+//                  more per CTA, 128 at a time), B = the output gradient;
+//                  per-chunk partials of all layers are reduced in chunk order
+//                  (deterministic) by the kernel that applies Adam and repacks.
 // Activations and gradients are stored BF16 (NHWC, channels contiguous),
 // master weights and Adam moments FP32.  Softmax, kernel application, loss,
 // bias gradients and Adam run on the CUDA cores.
@@ -36,6 +37,7 @@
 #include <mutex>
 #include <random>
 #include <string>
+#include <type_traits>
 #include <vector>
 
 #include "raygen_b200.h"
@@ -123,14 +125,6 @@ __host__ __device__ constexpr int layerOffset(int l) {
   return o;
 }
 constexpr int kNumParams = layerOffset(kLayers);
-
-// (b, y, x) of pixel p in a batch of H x W images, neighbour at (dy, dx) or -1
-__device__ __forceinline__ int neighbor(int p, int dy, int dx, int H, int W) {
-  const int x = p % W, t = p / W, y = t % H, b = t / H;
-  const int yy = y + dy, xx = x + dx;
-  if (yy < 0 || yy >= H || xx < 0 || xx >= W) return -1;
-  return (b * H + yy) * W + xx;
-}
 
 __device__ __forceinline__ int clampNeighbor(int p, int dy, int dx, int H, int W) {
   const int x = p % W, t = p / W, y = t % H, b = t / H;
@@ -411,16 +405,38 @@ __global__ void __launch_bounds__(kConvThreads) k_convStrip(const __grid_constan
   if (warp == 0) tc::tmemFree(tmem, 64);
 }
 
-// Backward weights: partial[chunk][m = (t, ci)][co] = sum over the chunk's
-// pixels q of X[q + off(t)][ci] * G[q][co].  Grid: (M tiles of 128 rows,
-// pixel chunks).  Rows beyond 9 * CIN are zero.
+// Pixels per backward-weight CTA: kChunk, or so many that a batch has at most kMaxChunks
+// chunks (one round of CTAs), which also bounds the partial sums kept.
+constexpr int kMaxChunks = 256;
+__host__ __device__ constexpr int chunkPixels(int P) {
+  return P <= kChunk * kMaxChunks ? kChunk : (P / kMaxChunks + kSub) / kSub * kSub;
+}
+__host__ __device__ constexpr int chunksFor(int P) { return (P + chunkPixels(P) - 1) / chunkPixels(P); }
+// Partial sums of one chunk: per layer the weights (m = (t, ci), co), then the biases.
+constexpr int kPartialFloats = kNumParams;
+
+// Shared-memory layout of the backward-weight operands: K-major core matrices (8 rows x 16
+// bytes) whose K neighbours lie 144 bytes apart and whose row groups 2336: a warp's stores of
+// pixel pairs then fall on 32 different banks (with the dense 128-byte spacing they met
+// four- and eight-fold).
+constexpr uint32_t kWgLbo = 144, kWgSbo = (kSub / 8) * kWgLbo + 32;
+__device__ __forceinline__ uint32_t wgOffset(int row, int k) {  // byte of element (row, k), k even
+  return (uint32_t)(row >> 3) * kWgSbo + (uint32_t)(k >> 3) * kWgLbo + (uint32_t)(row & 7) * 16u + (uint32_t)(k & 7) * 2u;
+}
+
+// Backward weights: partial[chunk][layer][m = (t, ci)][co] = sum over the chunk's
+// pixels q of X[q + off(t)][ci] * G[q][co], and from the first tile the bias sums of G.
+// Grid: (M tiles of 128 rows, pixel chunks).  Rows beyond 9 * CIN are zero.  Bound by
+// staging: pixels are the K dimension, so the channels-last rows are transposed on the way
+// to shared memory, as pairs of pixels in one 32-bit store.
 template <int CIN>
-__global__ void __launch_bounds__(128) k_convBwdWeight(int B, int H, int W, const __nv_bfloat16* __restrict__ X,
+__global__ void __launch_bounds__(128) k_convBwdWeight(int B, int H, int W, int chunkPix, const __nv_bfloat16* __restrict__ X,
                                                        const __nv_bfloat16* __restrict__ G, float* __restrict__ partial,
                                                        int* __restrict__ err) {
   constexpr int M = 9 * CIN;
-  __shared__ __align__(1024) unsigned char sA[128 * kSub * 2];
-  __shared__ __align__(1024) unsigned char sB[kC * kSub * 2];
+  __shared__ __align__(128) unsigned char sA[128 / 8 * kWgSbo];
+  __shared__ __align__(128) unsigned char sB[kC / 8 * kWgSbo];
+  __shared__ float sRed[4][kC];
   __shared__ uint64_t bar;
   __shared__ uint32_t tbase;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
@@ -434,69 +450,80 @@ __global__ void __launch_bounds__(128) k_convBwdWeight(int B, int H, int W, cons
   const uint32_t idesc = tc::instrDescBf16(128, kC);
   uint32_t phase = 0;
   bool ok = true;
-  for (int sub = 0; sub < kChunk / kSub; ++sub) {
-    const int q0 = chunk * kChunk + sub * kSub;
-    if (q0 >= P) break;
-    // thread tid stages pixel q = q0 + tid: its column in A (all rows of this tile) and in B
-    const int q = q0 + tid;
-    const int kcol = tid;
-    auto put = [&](unsigned char* base, int row, __nv_bfloat16 val) {
-      *reinterpret_cast<__nv_bfloat16*>(base + tc::chunkOffset(row, kcol >> 3, kSub) + (kcol & 7) * 2) = val;
-    };
+  float biasSum = 0.0f;  // channel `lane`, pixels 32 warp .. + 31 of each step
+  // a lane pair holds the two channel halves of one pixel pair
+  const int kpix = (tid >> 1) * 2, half = tid & 1;
+  // rows r0 + half * N / 2 .. of pixels (a, b), N / 2 channels from each pixel's half, both masked
+  auto stage = [&](unsigned char* base, int r0, const __nv_bfloat16* a, const __nv_bfloat16* b, auto n) {
+    constexpr int N2 = decltype(n)::value / 2;
+    uint4 va[N2 / 8], vb[N2 / 8];
+#pragma unroll
+    for (int j = 0; j < N2 / 8; ++j) {
+      va[j] = a ? reinterpret_cast<const uint4*>(a + half * N2)[j] : make_uint4(0, 0, 0, 0);
+      vb[j] = b ? reinterpret_cast<const uint4*>(b + half * N2)[j] : make_uint4(0, 0, 0, 0);
+    }
+#pragma unroll
+    for (int j = 0; j < N2 / 8; ++j) {
+      const uint32_t wa[4] = {va[j].x, va[j].y, va[j].z, va[j].w}, wb[4] = {vb[j].x, vb[j].y, vb[j].z, vb[j].w};
+#pragma unroll
+      for (int k = 0; k < 4; ++k) {
+        const int row = r0 + half * N2 + j * 8 + 2 * k;
+        *reinterpret_cast<uint32_t*>(base + wgOffset(row, kpix)) = __byte_perm(wa[k], wb[k], 0x5410);
+        *reinterpret_cast<uint32_t*>(base + wgOffset(row + 1, kpix)) = __byte_perm(wa[k], wb[k], 0x7632);
+      }
+    }
+  };
+  const int end = min(P, (chunk + 1) * chunkPix);
+  for (int q0 = chunk * chunkPix, sub = 0; q0 < end; q0 += kSub, ++sub) {
+    // this thread's two pixels
+    const int qa = q0 + kpix, qb = qa + 1;
+    const int xa = qa % W, ya = (qa / W) % H, xb = qb % W, yb = (qb / W) % H;
     for (int r = 0; r < 128; r += CIN) {  // one tap (CIN rows) at a time
-      const int m = m0 + r, t = m / CIN;
-      __align__(16) __nv_bfloat16 xv[CIN];
-#pragma unroll
-      for (int j = 0; j < CIN; ++j) xv[j] = __float2bfloat16_rn(0.0f);
-      if (m < M && q < P) {
-        const int n = neighbor(q, t / 3 - 1, t % 3 - 1, H, W);
-        if (n >= 0) {
-          const uint4* src = reinterpret_cast<const uint4*>(X + (size_t)n * CIN);
-#pragma unroll
-          for (int j = 0; j < CIN / 8; ++j) reinterpret_cast<uint4*>(xv)[j] = src[j];
-        }
+      const int m = m0 + r, t = m / CIN, dy = t / 3 - 1, dx = t % 3 - 1;
+      const __nv_bfloat16 *pa = nullptr, *pb = nullptr;
+      if (m < M) {
+        if (qa < end && ya + dy >= 0 && ya + dy < H && xa + dx >= 0 && xa + dx < W) pa = X + (size_t)(qa + dy * W + dx) * CIN;
+        if (qb < end && yb + dy >= 0 && yb + dy < H && xb + dx >= 0 && xb + dx < W) pb = X + (size_t)(qb + dy * W + dx) * CIN;
       }
-#pragma unroll
-      for (int j = 0; j < CIN; ++j) put(sA, r + j, xv[j]);
+      stage(sA, r, pa, pb, std::integral_constant<int, CIN>());
     }
-    {
-      __align__(16) __nv_bfloat16 gv[kC];
-#pragma unroll
-      for (int j = 0; j < kC; ++j) gv[j] = __float2bfloat16_rn(0.0f);
-      if (q < P) {
-        const uint4* src = reinterpret_cast<const uint4*>(G + (size_t)q * kC);
-#pragma unroll
-        for (int j = 0; j < 4; ++j) reinterpret_cast<uint4*>(gv)[j] = src[j];
-      }
-#pragma unroll
-      for (int j = 0; j < kC; ++j) put(sB, j, gv[j]);
-    }
+    stage(sB, 0, qa < end ? G + (size_t)qa * kC : nullptr, qb < end ? G + (size_t)qb * kC : nullptr,
+          std::integral_constant<int, kC>());
     tc::fenceProxyAsync();
     __syncthreads();
     tc::fenceAfterSync();
     if (tid == 0) {
       const uint32_t aBase = tc::smemAddr(sA), bBase = tc::smemAddr(sB);
       for (int s = 0; s < kSub / 16; ++s)
-        tc::mmaBf16(tmem, tc::smemDesc(aBase + s * 256, 128, (kSub / 8) * 128),
-                    tc::smemDesc(bBase + s * 256, 128, (kSub / 8) * 128), idesc, sub > 0 || s > 0);
+        tc::mmaBf16(tmem, tc::smemDesc(aBase + s * 2 * kWgLbo, kWgLbo, kWgSbo), tc::smemDesc(bBase + s * 2 * kWgLbo, kWgLbo, kWgSbo),
+                    idesc, sub > 0 || s > 0);
       tc::commit(&bar);
     }
+    if (mt == 0)
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        const uint4 v = *reinterpret_cast<const uint4*>(sB + wgOffset(lane, warp * 32 + j * 8));
+        const uint32_t w[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+          biasSum += __uint_as_float(w[k] << 16);
+          biasSum += __uint_as_float(w[k] & 0xffff0000u);
+        }
+      }
     ok = __syncthreads_and(tc::mbarWait(&bar, phase)) != 0;
     phase ^= 1u;
     tc::fenceAfterSync();
     if (!ok) break;
   }
+  if (mt == 0) sRed[warp][lane] = biasSum;
   if (ok) {
     float v[32];
     tc::tmemLoad32(tmem + ((uint32_t)(warp * 32) << 16), v);
     const int m = m0 + warp * 32 + lane;
-    // a chunk that starts past the end of the batch contributes zeros
-    const bool any = chunk * kChunk < P;
     if (m < M) {
-      float4* dst = reinterpret_cast<float4*>(partial + ((size_t)chunk * M + m) * kC);
+      float4* dst = reinterpret_cast<float4*>(partial + (size_t)chunk * kPartialFloats + (size_t)m * kC);
 #pragma unroll
-      for (int j = 0; j < kC; j += 4)
-        dst[j / 4] = any ? make_float4(v[j], v[j + 1], v[j + 2], v[j + 3]) : make_float4(0.f, 0.f, 0.f, 0.f);
+      for (int j = 0; j < kC; j += 4) dst[j / 4] = make_float4(v[j], v[j + 1], v[j + 2], v[j + 3]);
     }
   } else {
     if (tid == 0) atomicCAS(err, 0, tc::kErrTcTimeout);
@@ -504,36 +531,9 @@ __global__ void __launch_bounds__(128) k_convBwdWeight(int B, int H, int W, cons
   }
   tc::fenceBeforeSync();
   __syncthreads();
+  if (mt == 0 && tid < kC)
+    partial[(size_t)chunk * kPartialFloats + (size_t)M * kC + tid] = ((sRed[0][tid] + sRed[1][tid]) + sRed[2][tid]) + sRed[3][tid];
   if (warp == 0) tc::tmemFree(tmem, 32);
-}
-
-// grad W[co][t][ci] = sum over chunks (in order) of partial[chunk][(t, ci)][co].
-__global__ void k_reduceWeightGrad(int M, int chunks, const float* __restrict__ partial, float* __restrict__ gradW) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;  // over M * 32
-  if (i >= M * kC) return;
-  const int co = i / M, m = i % M;
-  float s = 0.0f;
-  for (int c = 0; c < chunks; ++c) s += partial[((size_t)c * M + m) * kC + co];
-  gradW[(size_t)co * M + m] = s;
-}
-
-// grad b[co] = sum_q G[q][co]: per-chunk partials, then an in-order reduction.
-__global__ void k_biasPartial(int P, const __nv_bfloat16* __restrict__ G, float* __restrict__ partial) {
-  const int chunk = blockIdx.x, co = threadIdx.x & 31, lane4 = threadIdx.x >> 5;  // 128 threads: 4 pixel lanes
-  __shared__ float acc[4][kC];
-  float s = 0.0f;
-  for (int q = chunk * kChunk + lane4; q < min(P, (chunk + 1) * kChunk); q += 4) s += __bfloat162float(G[(size_t)q * kC + co]);
-  acc[lane4][co] = s;
-  __syncthreads();
-  if (lane4 == 0) partial[(size_t)chunk * kC + co] = ((acc[0][co] + acc[1][co]) + acc[2][co]) + acc[3][co];
-}
-
-__global__ void k_reduceBiasGrad(int chunks, const float* __restrict__ partial, float* __restrict__ gradB) {
-  const int co = threadIdx.x;
-  if (co >= kC) return;
-  float s = 0.0f;
-  for (int c = 0; c < chunks; ++c) s += partial[(size_t)c * kC + co];
-  gradB[co] = s;
 }
 
 // Softmax + 5 x 5 kernel application.  TRAIN: also the relMSE loss and its
@@ -588,21 +588,59 @@ __global__ void k_head(int B, int H, int W, const float* __restrict__ Z, const f
   }
 }
 
-// Adam (Kingma & Ba 2015) on the FP32 master parameters.
-// Adam; the step number t = state[1] + 1 is read on the device so that a
-// captured training step can be replayed.
-__global__ void k_adam(int n, float* __restrict__ p, const float* __restrict__ g, float* __restrict__ m,
-                       float* __restrict__ v, float lr, float b1, float b2, const int* __restrict__ state, float eps) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n) return;
-  const float t = (float)(state[1] + 1);
-  const float c1 = 1.0f - powf(b1, t), c2 = 1.0f - powf(b2, t);
-  const float gi = g[i];
-  const float mi = b1 * m[i] + (1.0f - b1) * gi, vi = b2 * v[i] + (1.0f - b2) * gi * gi;
-  m[i] = mi;
-  v[i] = vi;
-  p[i] -= lr * (mi / c1) / (sqrtf(vi / c2) + eps);
+// Where the parameters of a layer lie, and its BF16 copies.
+struct PackTargets {
+  __nv_bfloat16* wf[kLayers];
+  __nv_bfloat16* wt[kLayers];
+};
+
+// BF16 copies of weight (co, m = (t, ci)) of a layer: the forward layout [co][(t, ci)] and the
+// transposed backward-data layout [ci][(t, co)] (32-channel inputs only).
+__device__ __forceinline__ void packWeight(const PackTargets& T, int layer, int co, int m, float v) {
+  const int cin = cinOf(layer);
+  const __nv_bfloat16 b = __float2bfloat16_rn(v);
+  T.wf[layer][co * 9 * cin + m] = b;
+  if (layer > 0) T.wt[layer][(size_t)(m % cin) * (9 * kC) + (m / cin) * kC + co] = b;
 }
+
+// One block per row m = (t, ci) of a layer (and one per layer for the biases): the gradient is
+// the sum of the chunks' partial sums in order, a quarter of them per warp, the quarters added
+// in order (deterministic).  UPDATE: Adam (Kingma & Ba 2015) on the FP32 master parameters and
+// their BF16 copies, in the same pass (20 launches of 100-250 us a step before); the step
+// number state[1] + 1 is read on the device so that a captured training step can be replayed.
+template <bool UPDATE>
+__global__ void __launch_bounds__(128) k_gradUpdate(int chunks, const float* __restrict__ partial, float* __restrict__ grad,
+                                                    float* __restrict__ params, float* __restrict__ m1, float* __restrict__ v1,
+                                                    float lr, float b1, float b2, const int* __restrict__ state, float eps,
+                                                    PackTargets T) {
+  int layer = 0, m = blockIdx.x;  // row of the layer: 9 cin weight rows, then the bias row
+  while (m > 9 * cinOf(layer)) m -= 9 * cinOf(layer++) + 1;
+  const int M = 9 * cinOf(layer), lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  // the layer's partial sums start where its parameters do: M rows of 32, then 32 biases
+  const float* src = partial + layerOffset(layer) + (size_t)m * kC + lane;
+  const int per = (chunks + 3) / 4, c1 = min(chunks, (warp + 1) * per);
+  float s = 0.0f;
+#pragma unroll 8
+  for (int c = warp * per; c < c1; ++c) s += src[(size_t)c * kPartialFloats];
+  __shared__ float sum[4][32];
+  sum[warp][lane] = s;
+  __syncthreads();
+  if (warp != 0) return;
+  const float g = ((sum[0][lane] + sum[1][lane]) + sum[2][lane]) + sum[3][lane];
+  const int i = layerOffset(layer) + (m < M ? lane * M + m : M * kC + lane);
+  grad[i] = g;
+  if (UPDATE) {
+    const float t = (float)(state[1] + 1);
+    const float k1 = 1.0f - powf(b1, t), k2 = 1.0f - powf(b2, t);
+    const float mi = b1 * m1[i] + (1.0f - b1) * g, vi = b2 * v1[i] + (1.0f - b2) * g * g;
+    m1[i] = mi;
+    v1[i] = vi;
+    const float pv = params[i] - lr * (mi / k1) / (sqrtf(vi / k2) + eps);
+    params[i] = pv;
+    if (m < M) packWeight(T, layer, lane, m, pv);
+  }
+}
+constexpr int kUpdateRows = 9 * (16 + 5 * 32) + kLayers;
 
 // One training example on the device: features, noisy radiance, reference.
 struct ExampleRef {
@@ -634,19 +672,13 @@ __global__ void k_stepEnd(int* __restrict__ state, const float* __restrict__ los
   state[1]++;
 }
 
-// Master FP32 weights -> BF16 forward layout [co][(t, ci)] and the transposed
-// backward-data layout [ci][(t, co)] (32-channel inputs only).
-__global__ void k_packWeights(const float* __restrict__ params, __nv_bfloat16* __restrict__ wf,
-                              __nv_bfloat16* __restrict__ wt, int layer) {
-  const int cin = layer == 0 ? 16 : 32;
-  const int n = kC * 9 * cin;
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n) return;
-  const float* W = params + layerOffset(layer);
-  const int co = i / (9 * cin), rem = i % (9 * cin), t = rem / cin, ci = rem % cin;
-  const __nv_bfloat16 b = __float2bfloat16_rn(W[i]);
-  wf[i] = b;
-  if (wt) wt[(size_t)ci * (9 * kC) + t * kC + co] = b;
+// BF16 copies of all master weights (after they were set from outside).
+__global__ void k_packWeights(const float* __restrict__ params, PackTargets T) {
+  int layer = 0, m = blockIdx.x * 4 + (threadIdx.x >> 5);
+  while (layer < kLayers && m >= 9 * cinOf(layer)) m -= 9 * cinOf(layer++);
+  if (layer >= kLayers) return;
+  const int co = threadIdx.x & 31;
+  packWeight(T, layer, co, m, params[layerOffset(layer) + co * 9 * cinOf(layer) + m]);
 }
 
 }  // namespace
@@ -745,7 +777,9 @@ struct KpcnNet {
   // work buffers for P pixels
   size_t cap = 0;
   DevBuf<__nv_bfloat16> X0, act[kLayers - 1], gA, gB;
-  DevBuf<float> Z, partial, bpartial, loss;
+  DevBuf<float> Z, partial, loss;
+  cudaStream_t side = nullptr;             // backward weights beside the next layer's data gradient
+  cudaEvent_t ready = nullptr, used[2] = {nullptr, nullptr};
   DevBuf<float4> noisy, ref, out;
   DevBuf<int> err;
   ~KpcnNet() {
@@ -753,19 +787,21 @@ struct KpcnNet {
     for (auto* p : exX) cudaFree(p);
     for (auto* p : exNoisy) cudaFree(p);
     for (auto* p : exRef) cudaFree(p);
+    if (ready) cudaEventDestroy(ready);
+    for (auto e : used)
+      if (e) cudaEventDestroy(e);
+    if (side) cudaStreamDestroy(side);
     if (st) cudaStreamDestroy(st);
   }
 };
 
 namespace {
 
-int chunksFor(size_t P) { return (int)((P + kChunk - 1) / kChunk); }
-
 bool ensureWork(KpcnNet& n, size_t P) {
   if (P <= n.cap) return true;
-  const int ch = chunksFor(P);
+  const size_t ch = std::min<size_t>((P + kChunk - 1) / kChunk, kMaxChunks);  // of any batch up to P
   bool ok = n.X0.alloc(P * 16) && n.gA.alloc(P * kC) && n.gB.alloc(P * kC) && n.Z.alloc(P * kC) &&
-            n.partial.alloc((size_t)ch * 9 * kC * kC) && n.bpartial.alloc((size_t)ch * kC) && n.loss.alloc(1) &&
+            n.partial.alloc(ch * kPartialFloats) && n.loss.alloc(1) &&
             n.noisy.alloc(P) && n.ref.alloc(P) && n.out.alloc(P) && n.err.alloc(1);
   for (int l = 0; l < kLayers - 1; ++l) ok = ok && n.act[l].alloc(P * kC);
   if (ok) {
@@ -784,12 +820,16 @@ void setSmem(K kernel, size_t bytes) {
   cudaFuncSetAttribute(kernel, cudaFuncAttributePreferredSharedMemoryCarveout, (int)cudaSharedmemCarveoutMaxShared);
 }
 
-void packWeights(KpcnNet& n) {
+PackTargets packTargets(KpcnNet& n) {
+  PackTargets T;
   for (int l = 0; l < kLayers; ++l) {
-    const int cnt = layerWeights(l);
-    k_packWeights<<<(cnt + 255) / 256, 256, 0, n.st>>>(n.params.p, n.wf[l].p, l > 0 ? n.wt[l].p : nullptr, l);
+    T.wf[l] = n.wf[l].p;
+    T.wt[l] = l > 0 ? n.wt[l].p : nullptr;
   }
+  return T;
 }
+
+void packWeights(KpcnNet& n) { k_packWeights<<<(kUpdateRows + 3) / 4, 128, 0, n.st>>>(n.params.p, packTargets(n)); }
 
 // Resident CTAs per SM of a strip-convolution kernel, from its shared memory,
 // registers, threads and tensor-memory columns (64 per CTA).  The runtime's
@@ -905,26 +945,30 @@ void forward(KpcnNet& n, int B, int H, int W, const float4* noisy = nullptr, flo
                                 n.Z.p);
 }
 
-// Head gradient must be in gA; fills n.grad.
+// Head gradient must be in gA; fills n.partial.  A layer's weight gradient runs on the side
+// stream beside the data gradient of the same layer: both read G, which the data gradient two
+// layers on overwrites.
 void backward(KpcnNet& n, int B, int H, int W) {
-  const size_t P = (size_t)B * H * W;
-  const int ch = chunksFor(P);
+  const int P = B * H * W, ch = chunksFor(P), cp = chunkPixels(P);
   __nv_bfloat16* G = n.gA.p;
   __nv_bfloat16* Gn = n.gB.p;
   for (int l = kLayers - 1; l >= 0; --l) {
     const __nv_bfloat16* in = l == 0 ? n.X0.p : n.act[l - 1].p;
-    const int M = 9 * cinOf(l);
-    const dim3 g((M + 127) / 128, ch);
-    if (l == 0) k_convBwdWeight<16><<<g, 128, 0, n.st>>>(B, H, W, in, G, n.partial.p, n.err.p);
-    else k_convBwdWeight<32><<<g, 128, 0, n.st>>>(B, H, W, in, G, n.partial.p, n.err.p);
-    k_reduceWeightGrad<<<(M * kC + 255) / 256, 256, 0, n.st>>>(M, ch, n.partial.p, n.grad.p + layerOffset(l));
-    k_biasPartial<<<ch, 128, 0, n.st>>>((int)P, G, n.bpartial.p);
-    k_reduceBiasGrad<<<1, 32, 0, n.st>>>(ch, n.bpartial.p, n.grad.p + layerOffset(l) + layerWeights(l));
+    const dim3 g((9 * cinOf(l) + 127) / 128, ch);
+    float* part = n.partial.p + layerOffset(l);
+    cudaEventRecord(n.ready, n.st);  // G of this layer is there
+    cudaStreamWaitEvent(n.side, n.ready, 0);
+    if (l == 0) k_convBwdWeight<16><<<g, 128, 0, n.side>>>(B, H, W, cp, in, G, part, n.err.p);
+    else k_convBwdWeight<32><<<g, 128, 0, n.side>>>(B, H, W, cp, in, G, part, n.err.p);
+    cudaEventRecord(n.used[l & 1], n.side);
     if (l > 0) {
+      if (l < kLayers - 1) cudaStreamWaitEvent(n.st, n.used[(l + 1) & 1], 0);  // Gn was layer l + 1's G
       launchConv<32, false, true>(n, B, H, W, G, n.wt[l].p, nullptr, in, Gn, nullptr);
       std::swap(G, Gn);
     }
   }
+  cudaStreamWaitEvent(n.st, n.used[0], 0);
+  cudaStreamWaitEvent(n.st, n.used[1], 0);
 }
 
 rg_status setPipeWaitLimit(uint32_t polls) {
@@ -966,7 +1010,12 @@ bool initNet(KpcnNet& n, uint32_t seed) {
   int dev = 0;
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&n.numSMs, cudaDevAttrMultiProcessorCount, dev);
-  if (cudaStreamCreateWithFlags(&n.st, cudaStreamNonBlocking) != cudaSuccess) return false;
+  if (cudaStreamCreateWithFlags(&n.st, cudaStreamNonBlocking) != cudaSuccess ||
+      cudaStreamCreateWithFlags(&n.side, cudaStreamNonBlocking) != cudaSuccess ||
+      cudaEventCreateWithFlags(&n.ready, cudaEventDisableTiming) != cudaSuccess ||
+      cudaEventCreateWithFlags(&n.used[0], cudaEventDisableTiming) != cudaSuccess ||
+      cudaEventCreateWithFlags(&n.used[1], cudaEventDisableTiming) != cudaSuccess)
+    return false;
   n.rng.seed(seed);
   bool ok = n.params.alloc(kNumParams) && n.grad.alloc(kNumParams) && n.m.alloc(kNumParams) && n.v.alloc(kNumParams);
   for (int l = 0; l < kLayers && ok; ++l) {
@@ -1211,9 +1260,9 @@ rg_status rg_denoiser_train(rg_denoiser* d, int32_t steps, int32_t batch, float 
     rg::k_head<true><<<(unsigned)((P + 255) / 256), 256, 0, n.st>>>(B, H, W, n.Z.p, n.noisy.p, n.ref.p, nullptr, n.gA.p,
                                                                      n.loss.p);
     rg::backward(n, B, H, W);
-    rg::k_adam<<<(rg::kNumParams + 255) / 256, 256, 0, n.st>>>(rg::kNumParams, n.params.p, n.grad.p, n.m.p, n.v.p, lr,
-                                                               0.9f, 0.999f, n.state.p, 1e-8f);
-    rg::packWeights(n);
+    rg::k_gradUpdate<true><<<rg::kUpdateRows, 128, 0, n.st>>>(rg::chunksFor((int)P), n.partial.p, n.grad.p, n.params.p, n.m.p,
+                                                              n.v.p, lr, 0.9f, 0.999f, n.state.p, 1e-8f,
+                                                              rg::packTargets(n));
     rg::k_stepEnd<<<1, 1, 0, n.st>>>(n.state.p, n.loss.p, n.lossHist.p);
     RG_CUDA_CHECK(cudaStreamEndCapture(n.st, &g));
     const cudaError_t ie = cudaGraphInstantiate(&n.trainGraph, g, 0);
@@ -1267,6 +1316,8 @@ rg_status rg_denoiser_gradients(rg_denoiser* d, int32_t count, int32_t w, int32_
   rg::k_head<true><<<(unsigned)((P + 255) / 256), 256, 0, n.st>>>(count, h, w, n.Z.p, n.noisy.p, n.ref.p, nullptr, n.gA.p,
                                                                    n.loss.p);
   rg::backward(n, count, h, w);
+  rg::k_gradUpdate<false><<<rg::kUpdateRows, 128, 0, n.st>>>(rg::chunksFor((int)P), n.partial.p, n.grad.p, nullptr, nullptr,
+                                                             nullptr, 0.0f, 0.0f, 0.0f, nullptr, 0.0f, rg::PackTargets{});
   const rg_status rs = rg::checkErr(n, "learned denoiser gradients");
   if (rs != RG_OK) return rs;
   RG_CUDA_CHECK(cudaMemcpy(grad, n.grad.p, sizeof(float) * rg::kNumParams, cudaMemcpyDeviceToHost));
