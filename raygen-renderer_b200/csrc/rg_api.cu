@@ -280,22 +280,20 @@ void buildMedia(const rg_scene_desc* d, const Mat4& view, MediaTables& T) {
 using namespace rg;
 
 // Buffers of the ray-batch queries, kept between calls: allocating and freeing them took a
-// third of a 1000-ray query.  Inputs and outputs lie in one device array each, so a batch of
-// up to kSmall rays is one copy in and one out through a page-locked array (a larger one is
-// copied from and to the caller's arrays).  More than 64 MB are given back after the call.
+// third of a 1000-ray query.  One device array holds the inputs, the query's error word and
+// the outputs, in this order, so a batch of up to kSmall rays is one copy in (its error word
+// zero), the kernel, and one copy out, through a page-locked array; a larger one is copied
+// from and to the caller's arrays.  More than 64 MB are given back after the call.
 struct QueryBuffers {
-  static constexpr int kSmall = 8192;
-  static constexpr size_t kHostBytes = (size_t)kSmall * 28 + 16;  // 7 floats in; 4 words and the error word out
-  DevBuf<float> in;   // rays (6 n), tmax (n)
-  DevBuf<float> out;  // the error word, then t, u, v (3 n) and triangle (n), or a byte per ray
+  static constexpr int kSmall = 16384;
+  static constexpr size_t kHostBytes = (size_t)kSmall * 44 + 16;  // 7 floats in, the error word, 4 words out
+  DevBuf<float> io;
   unsigned char* host = nullptr;
   ~QueryBuffers() {
     if (host) cudaFreeHost(host);
   }
   void trim() {
-    if (in.bytes() + out.bytes() <= (size_t(64) << 20)) return;
-    in.release();
-    out.release();
+    if (io.bytes() > (size_t(64) << 20)) io.release();
   }
 };
 
@@ -1777,42 +1775,43 @@ rg_status rg_get_view_matrix(rg_handle* h, float* m16) {
   return RG_OK;
 }
 
-// One batch query: `rays` (and `tmax`) in, `launch(in, out)` on h->stream, then the results
-// at word 1 of the output array in two parts (host array, bytes).
+// One batch query: `rays` (and `tmax`) in, `launch(scene, in, out)` on h->stream, then the
+// results in two parts (host array, bytes).
 static rg_status runQuery(rg_handle* h, const float* rays, const float* tmax, int n, size_t outWords,
-                          const std::function<void(const float*, float*)>& launch, void* out0, size_t bytes0, void* out1,
-                          size_t bytes1) {
+                          const std::function<void(const DevScene&, const float*, float*)>& launch, void* out0, size_t bytes0,
+                          void* out1, size_t bytes1) {
   QueryBuffers& b = h->query;
   const size_t inWords = (size_t)n * (tmax ? 7 : 6);
-  if (!b.in.alloc(inWords) || !b.out.alloc(1 + outWords)) {
-    b.trim();
-    return RG_ERR_OUT_OF_MEMORY;
-  }
+  if (!b.io.alloc(inWords + 1 + outWords)) return RG_ERR_OUT_OF_MEMORY;
   const bool small = n <= QueryBuffers::kSmall && b.host;
   cudaStream_t st = h->stream;
+  float* error = b.io.p + inWords;
+  DevScene S = h->dscene;
+  S.error = reinterpret_cast<int*>(error);  // this query's flag only
   int derr = 0;
-  RG_CUDA_CHECK(cudaMemsetAsync(h->error.p, 0, sizeof(int), st));  // this query's flag only
   if (small) {
     std::memcpy(b.host, rays, sizeof(float) * 6 * n);
     if (tmax) std::memcpy(b.host + sizeof(float) * 6 * n, tmax, sizeof(float) * n);
-    RG_CUDA_CHECK(cudaMemcpyAsync(b.in.p, b.host, sizeof(float) * inWords, cudaMemcpyHostToDevice, st));
+    std::memcpy(b.host + sizeof(float) * inWords, &derr, sizeof(int));
+    RG_CUDA_CHECK(cudaMemcpyAsync(b.io.p, b.host, sizeof(float) * (inWords + 1), cudaMemcpyHostToDevice, st));
   } else {
-    RG_CUDA_CHECK(copyToDevice(b.in.p, rays, sizeof(float) * 6 * n, st));
-    if (tmax) RG_CUDA_CHECK(copyToDevice(b.in.p + (size_t)6 * n, tmax, sizeof(float) * n, st));
+    RG_CUDA_CHECK(cudaMemsetAsync(error, 0, sizeof(int), st));
+    RG_CUDA_CHECK(copyToDevice(b.io.p, rays, sizeof(float) * 6 * n, st));
+    if (tmax) RG_CUDA_CHECK(copyToDevice(b.io.p + (size_t)6 * n, tmax, sizeof(float) * n, st));
   }
-  launch(b.in.p, b.out.p + 1);
-  RG_CUDA_CHECK(cudaMemcpyAsync(b.out.p, h->error.p, sizeof(int), cudaMemcpyDeviceToDevice, st));
+  launch(S, b.io.p, error + 1);
   if (small) {
-    RG_CUDA_CHECK(cudaMemcpyAsync(b.host, b.out.p, sizeof(int) + bytes0 + bytes1, cudaMemcpyDeviceToHost, st));
+    unsigned char* o = b.host + sizeof(float) * inWords;
+    RG_CUDA_CHECK(cudaMemcpyAsync(o, error, sizeof(int) + bytes0 + bytes1, cudaMemcpyDeviceToHost, st));
     RG_CUDA_CHECK(cudaStreamSynchronize(st));
-    std::memcpy(&derr, b.host, sizeof(int));
-    std::memcpy(out0, b.host + sizeof(int), bytes0);
-    if (bytes1) std::memcpy(out1, b.host + sizeof(int) + bytes0, bytes1);
+    std::memcpy(&derr, o, sizeof(int));
+    std::memcpy(out0, o + sizeof(int), bytes0);
+    if (bytes1) std::memcpy(out1, o + sizeof(int) + bytes0, bytes1);
   } else {
-    const unsigned char* o = reinterpret_cast<const unsigned char*>(b.out.p + 1);
+    const unsigned char* o = reinterpret_cast<const unsigned char*>(error + 1);
     RG_CUDA_CHECK(copyToHost(out0, o, bytes0, st));
     if (bytes1) RG_CUDA_CHECK(copyToHost(out1, o + bytes0, bytes1, st));
-    RG_CUDA_CHECK(copyToHost(&derr, b.out.p, sizeof(int), st));
+    RG_CUDA_CHECK(copyToHost(&derr, error, sizeof(int), st));
     b.trim();
   }
   if (derr) {
@@ -1829,8 +1828,8 @@ rg_status rg_trace_closest(rg_handle* h, const float* rays, int32_t n, float* ou
   if (n == 0) return RG_OK;
   return runQuery(
       h, rays, nullptr, n, (size_t)n * 4,
-      [&](const float* in, float* out) {
-        launchQueryClosest(h->dscene, in, n, out, reinterpret_cast<int*>(out + (size_t)3 * n), h->stream);
+      [&](const DevScene& S, const float* in, float* out) {
+        launchQueryClosest(S, in, n, out, reinterpret_cast<int*>(out + (size_t)3 * n), h->stream);
       },
       out_tuv, sizeof(float) * 3 * n, out_prim, sizeof(int) * n);
 }
@@ -1844,8 +1843,8 @@ rg_status rg_trace_any(rg_handle* h, const float* rays, const float* tmax, int32
   const uint32_t occ = occs[predicate];
   return runQuery(
       h, rays, tmax, n, ((size_t)n + 3) / 4,
-      [&](const float* in, float* o) {
-        launchQueryAny(h->dscene, in, in + (size_t)6 * n, n, occ, reinterpret_cast<uint8_t*>(o), h->stream);
+      [&](const DevScene& S, const float* in, float* o) {
+        launchQueryAny(S, in, in + (size_t)6 * n, n, occ, reinterpret_cast<uint8_t*>(o), h->stream);
       },
       out, n, nullptr, 0);
 }

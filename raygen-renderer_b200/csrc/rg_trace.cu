@@ -1866,6 +1866,121 @@ __global__ void k_queryAny(DevScene S, const float* __restrict__ rays, const flo
   out[i] = traceAny(S, o, d, tmax[i], occ, nodes, tris) ? 1 : 0;
 }
 
+// Small batches on the 8-wide BVH: a warp per ray.  Such a batch takes as long as its longest
+// ray, a chain of dependent reads, and 32 unrelated rays in one warp wait for one another on
+// top: 1000 rays on 20k triangles took 65 us.  Eight lanes read and test a node's children in
+// one go, and all the node's triangles are tested at once, a lane each; the first of the
+// nearest in triangle order is the hit, as one after another.
+template <bool ANY>
+__global__ void __launch_bounds__(128) k_queryWarp(DevScene S, const float* __restrict__ rays, const float* __restrict__ tmaxIn,
+                                                   int n, uint32_t occ, float* __restrict__ tuv, int* __restrict__ prim,
+                                                   uint8_t* __restrict__ out) {
+  constexpr unsigned kAll = 0xffffffffu;
+  __shared__ uint2 sStack[4][kStack8];  // node groups (child base, hit bits | inner mask << 8)
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, i = blockIdx.x * 4 + warp;
+  if (i >= n) return;
+  const float* r = rays + (size_t)i * 6;
+  const V3 o = v3(r[0], r[1], r[2]), d = v3(r[3], r[4], r[5]);
+  float tmax = ANY ? tmaxIn[i] : kMaxRayDistance, hu = 0.0f, hv = 0.0f;
+  int hit = -1;
+  bool occluded = false;
+  const V3 inv = safeInv(d);
+  const uint32_t oct = rayOctant(inv);
+  const int child = lane & 7;
+  int sp = 0, steps = 0, node = S.numTris > 0 ? 0 : -1;
+  while (node >= 0) {
+    if (node >= S.numNodes8 || ++steps > c_traversalStepCap) {
+      if (lane == 0) atomicCAS(S.error, 0, kErrTraversalSteps);
+      break;
+    }
+    const char* at = reinterpret_cast<const char*>(S.nodes8 + (size_t)node * kNode8Vec);
+    const uint32_t sw = ((uint32_t)node & 7u) * 16u;
+    const float4 h = ldNode4(reinterpret_cast<const float4*>(at + (0u ^ sw))), g = ldNode4(reinterpret_cast<const float4*>(at + (16u ^ sw)));
+    float pl[3][2];  // this child's near and far plane per axis
+#pragma unroll
+    for (int k = 0; k < 3; k++)
+#pragma unroll
+      for (int f = 0; f < 2; f++) {
+        const uint32_t w = (32u + 32u * k) ^ (16u * (f ^ ((oct >> k) & 1u)));
+        pl[k][f] = __half2float(__ldg(reinterpret_cast<const __half*>(at + (w ^ sw)) + child));
+      }
+    const uint32_t pack = __float_as_uint(g.w), m0 = __float_as_uint(h.z), m1 = __float_as_uint(h.w);
+    const float scale = __uint_as_float(pack & 0x7f800000u);
+    const V3 Sc = v3(scale * inv.x, scale * inv.y, scale * inv.z);
+    const V3 C = v3((g.x - o.x) * inv.x, (g.y - o.y) * inv.y, (g.z - o.z) * inv.z);
+    const float tmin = fmax3f(fmaf(pl[0][0], Sc.x, C.x), fmaf(pl[1][0], Sc.y, C.y), fmaf(pl[2][0], Sc.z, C.z));
+    const float tfar = fmin3f(fmaf(pl[0][1], Sc.x, C.x), fmaf(pl[1][1], Sc.y, C.y), fmaf(pl[2][1], Sc.z, C.z));
+    const unsigned hits = __ballot_sync(kAll, fmaxf(tmin, 0.0f) <= fminf(tfar, tmax)) & 0xffu;
+    const uint32_t imask = pack & 0xffu;
+    // triangles of the hit leaves: a lane each
+    const uint32_t meta = ((child & 4 ? m1 : m0) >> (8 * (child & 3))) & 0xffu;
+    const uint32_t run = (hits >> child) & 1u ? bitRun(meta, meta >> 5) : 0u;
+    const uint32_t mask = __reduce_or_sync(kAll, run);
+    if (mask) {
+      const int tk = __float_as_int(h.y) + lane;
+      bool got = false;
+      ClosestHit c;
+      c.t = tmax;
+      c.u = c.v = 0.0f;
+      if ((mask >> lane) & 1u) {
+        const float4* tp = S.triVerts + (size_t)tk * 3;
+        const float4 a = ldTri4(tp), b = ldTri4(tp + 1), e = ldTri4(tp + 2);
+        if (ANY) got = (__float_as_uint(b.w) & occ) && mtAny(o, d, xyz(a), xyz(b), xyz(e), tmax);
+        else got = mtClosest(o, d, xyz(a), xyz(b), xyz(e), c);
+      }
+      const unsigned any = __ballot_sync(kAll, got);
+      if (ANY) {
+        if (any) {
+          occluded = true;
+          break;
+        }
+      } else if (any) {
+        // t >= 0, and -0 = +0: the order of the bits is the order of the distances
+        const uint32_t bits = got ? __float_as_uint(c.t + 0.0f) : 0xffffffffu;
+        const uint32_t least = __reduce_min_sync(kAll, bits);  // by every lane: not behind a condition
+        const int best = __ffs(__ballot_sync(kAll, got && bits == least)) - 1;
+        tmax = __shfl_sync(kAll, c.t, best);
+        hu = __shfl_sync(kAll, c.u, best);
+        hv = __shfl_sync(kAll, c.v, best);
+        hit = __float_as_int(h.y) + best;
+      }
+    }
+    // the nearest hit inner child next (descending slot ^ octant), the others put aside
+    uint32_t x = hits & imask;
+    if (oct & 1u) x = ((x & 0x55u) << 1) | ((x >> 1) & 0x55u);
+    if (oct & 2u) x = ((x & 0x33u) << 2) | ((x >> 2) & 0x33u);
+    if (oct & 4u) x = ((x & 0x0fu) << 4) | ((x >> 4) & 0x0fu);
+    uint2 grp = make_uint2((uint32_t)__float_as_int(h.x), x | (imask << 8));
+    if (x == 0) {
+      if (sp == 0) break;
+      __syncwarp();
+      grp = sStack[warp][--sp];
+    }
+    const int pos = 31 - __clz(grp.y & 0xffu);
+    grp.y &= ~(1u << pos);
+    const int slot = pos ^ (int)oct;
+    node = (int)grp.x + __popc((grp.y >> 8) & ((1u << slot) - 1u));
+    if (grp.y & 0xffu) {
+      if (sp < kStack8) {
+        __syncwarp();
+        if (lane == 0) sStack[warp][sp] = grp;
+        sp++;
+      } else if (lane == 0) {
+        atomicCAS(S.error, 0, kErrStackOverflow);
+      }
+    }
+  }
+  if (lane != 0) return;
+  if (ANY) {
+    out[i] = occluded ? 1 : 0;
+  } else {
+    tuv[(size_t)i * 3] = tmax;
+    tuv[(size_t)i * 3 + 1] = hu;
+    tuv[(size_t)i * 3 + 2] = hv;
+    prim[i] = hit >= 0 ? S.triOrig[hit] : -1;
+  }
+}
+
 // Medium field queries (rg_medium_eval / rg_medium_bend).  The scene copy
 // sits in the job table so the field functions read it from global memory.
 __global__ void k_mediumEval(const DevJob* __restrict__ jobs, int medium, const float* __restrict__ pts, int n,
@@ -2047,12 +2162,28 @@ void launchProbeSampling(int which, const float* in, int n, float* out, cudaStre
   k_probeSampling<<<(n + 127) / 128, 128, 0, st>>>(which, in, n, out);
 }
 
+// Rays up to which a query takes a warp each (whole closest-hit calls on 20k triangles, warp
+// against thread per ray: 100 rays 40 / 55 us, 1000 57 / 90, 5000 61 / 98, 20000 145 / 170,
+// 50000 263 / 265, 100000 447 / 394).
+#ifndef RG_QUERY_WARP
+#define RG_QUERY_WARP 32768
+#endif
+constexpr int kQueryWarp = RG_QUERY_WARP;
+
 void launchQueryClosest(const DevScene& S, const float* rays, int n, float* tuv, int* prim, cudaStream_t st) {
-  if (n > 0) k_queryClosest<<<(n + 127) / 128, 128, 0, st>>>(S, rays, n, tuv, prim);
+  if (n <= 0) return;
+  if (S.bvhWidth == 8 && n <= kQueryWarp)
+    k_queryWarp<false><<<(n + 3) / 4, kTraceBlock, 0, st>>>(S, rays, nullptr, n, 0u, tuv, prim, nullptr);
+  else
+    k_queryClosest<<<(n + 127) / 128, 128, 0, st>>>(S, rays, n, tuv, prim);
 }
 void launchQueryAny(const DevScene& S, const float* rays, const float* tmax, int n, uint32_t occ, uint8_t* out,
                     cudaStream_t st) {
-  if (n > 0) k_queryAny<<<(n + 127) / 128, 128, 0, st>>>(S, rays, tmax, n, occ, out);
+  if (n <= 0) return;
+  if (S.bvhWidth == 8 && n <= kQueryWarp)
+    k_queryWarp<true><<<(n + 3) / 4, kTraceBlock, 0, st>>>(S, rays, tmax, n, occ, nullptr, nullptr, out);
+  else
+    k_queryAny<<<(n + 127) / 128, 128, 0, st>>>(S, rays, tmax, n, occ, out);
 }
 void launchMediumQuery(const DevJob* jobs, int medium, bool bend, const float* in, int n, float* out, cudaStream_t st) {
   if (n <= 0) return;

@@ -27,9 +27,10 @@ def in_pieces(r, rays, step=5000):
     return np.concatenate([p[0] for p in parts]), np.concatenate([p[1] for p in parts])
 
 
-# 24 bytes a ray in, 12 and 4 out: one ray; the small-batch limit; around 3 MB in (131072) and
-# 3 MB of t, u, v (262144) with and without a ragged chunk; several chunks a worker
-@pytest.mark.parametrize("n", [1, 8192, 8193, 131071, 131072, 131073, 262144, 700001])
+# 24 bytes a ray in, 12 and 4 out: one ray; the small-batch limit (16384); the limit of a warp per
+# ray (32768; the pieces compared with are below it); around 3 MB in (131072) and 3 MB of t, u, v
+# (262144) with and without a ragged chunk; several chunks a worker
+@pytest.mark.parametrize("n", [1, 16384, 16385, 32768, 32769, 131071, 131072, 131073, 262144, 700001])
 def test_query_sizes(rg, n):
     r = renderer(rg)
     rays = rays_of(n, n)
