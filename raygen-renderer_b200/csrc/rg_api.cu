@@ -480,8 +480,8 @@ namespace {
 
 DevRender makeRender(const rg_handle* h) { return makeRenderParams(h->st, h->camera); }
 
-// Shade / accumulate blocks per SM of grid (two of 256 threads are resident at 119
-// registers; the rest follow in grid-stride windows); build-time overridable (-D).
+// Shade / accumulate blocks per SM of grid (two shade blocks are resident, so a multiple of
+// two); build-time overridable (-D).
 #ifndef RG_SHADE_BLOCKS_PER_SM
 #define RG_SHADE_BLOCKS_PER_SM 4
 #endif

@@ -1122,19 +1122,32 @@ void launchTriMaterial(const DevScene& S, int n, int* triMat, cudaStream_t st) {
 // cone / path emission, heat haze) and volume-light NEE.  Scenes without
 // those features run a smaller kernel (instruction fetch is this kernel's
 // main stall).
-// Two blocks per SM (128 registers) for every variant: left to itself the compiler gave the
-// multi-job kernel 173-222 registers, which is one block (24 jobs through the server: 64 -> 53
-// ms of device time, with 0-100 bytes of spills).  Three blocks (80 registers) spill more
-// than they hide: 43.3 -> 53.3 ms on the 4M-triangle scene.
+// Block shape of the shade kernel: two blocks of 448 threads per SM (72 registers, 28 warps), two
+// rays per thread, so windows of 896 rays.  The kernel waits for its gathers: with two blocks of
+// 256 threads (128 registers, 16 warps) it issued in 30% of the cycles, and the warps are worth
+// the spills that the bound costs (140 - 1200 bytes).  Shade of 4M triangles 1080p 32 spp / 1M in
+// fog / 150k triangles / the cube room: 2 x 256 43.2 / 33.3 / 3.00 / 0.473 ms, 2 x 320 37.6 / 31.6 /
+// 2.71 / 0.432, 2 x 384 36.3 / 31.5 / 2.58 / 0.433, 2 x 448 36.0 / 29.9 / 2.53 / 0.427, 2 x 512
+// 36.2 / 29.5 / 2.54 / 0.456, 1 x 1024 37.6 / 28.2 / 2.68 / 0.460, 3 x 256 37.9 / 34.4 / 2.61 /
+// 0.429; the grid has to be a multiple of the resident blocks (3 x 256 in a grid of 4 per SM: 53).
+// Unbounded, the multi-job kernel took 173-222 registers, one block of 256 per SM (24 jobs
+// through the server 64 ms of device time, 51 now).
+#ifndef RG_SHADE_BLOCK
+#define RG_SHADE_BLOCK 448
+#endif
 #ifndef RG_SHADE_MIN_BLOCKS
 #define RG_SHADE_MIN_BLOCKS 2
 #endif
+#ifndef RG_SHADE_PER
+#define RG_SHADE_PER 2
+#endif
+constexpr int kShadeBlock = RG_SHADE_BLOCK;
 template <bool MULTI, bool ENV, int MEDL>
-__global__ void __launch_bounds__(256, RG_SHADE_MIN_BLOCKS) k_shade(DevScene S0, DevRender R0, const DevJob* __restrict__ jobs, DevQueues Q,
+__global__ void __launch_bounds__(kShadeBlock, RG_SHADE_MIN_BLOCKS) k_shade(DevScene S0, DevRender R0, const DevJob* __restrict__ jobs, DevQueues Q,
                                                int iter) {
   const int count = Q.counters[iter * kCountersPerIter + C_RAYS];
   const int inB = iter & 1, outB = (iter + 1) & 1;
-  // Each block iteration takes 512 consecutive queue entries (two per thread)
+  // Each block iteration takes kWin consecutive queue entries (two per thread)
   // and shades them grouped by the branch their hit takes (a counting sort in
   // shared memory), so that a warp mostly runs one lobe: incoherent bounces
   // otherwise leave a third of the lanes active and the kernel waiting on
@@ -1142,7 +1155,7 @@ __global__ void __launch_bounds__(256, RG_SHADE_MIN_BLOCKS) k_shade(DevScene S0,
   // 3 mirror, 4 refraction, 5 transparency, 6 mixed lobes, 7 miss.  The bins and
   // the order are double buffered by iteration, which leaves three block
   // barriers per iteration.
-  constexpr int kBins = 8, kPer = 2, kWin = 256 * kPer;
+  constexpr int kBins = 8, kPer = RG_SHADE_PER, kWin = kShadeBlock * kPer;
   __shared__ int sBin[2][kBins];
   __shared__ int sOrder[2][kWin];
   if (threadIdx.x < 2 * kBins) sBin[threadIdx.x / kBins][threadIdx.x % kBins] = 0;
@@ -1153,7 +1166,7 @@ __global__ void __launch_bounds__(256, RG_SHADE_MIN_BLOCKS) k_shade(DevScene S0,
       int key[kPer], rank[kPer];
 #pragma unroll
       for (int h = 0; h < kPer; ++h) {
-        const int q0 = base + h * 256 + threadIdx.x;
+        const int q0 = base + h * kShadeBlock + threadIdx.x;
         key[h] = kBins - 1;
         if (q0 < count) {
           const int prim0 = __float_as_int(Q.hits[q0].w);
@@ -1181,11 +1194,11 @@ __global__ void __launch_bounds__(256, RG_SHADE_MIN_BLOCKS) k_shade(DevScene S0,
       }
       __syncthreads();
 #pragma unroll
-      for (int h = 0; h < kPer; ++h) sOrder[buf][sBin[buf][key[h]] + rank[h]] = base + h * 256 + threadIdx.x;
+      for (int h = 0; h < kPer; ++h) sOrder[buf][sBin[buf][key[h]] + rank[h]] = base + h * kShadeBlock + threadIdx.x;
       __syncthreads();
     }
     for (int h = 0; h < kPer; ++h) {
-      const int q = sOrder[buf][threadIdx.x + h * 256];
+      const int q = sOrder[buf][threadIdx.x + h * kShadeBlock];
       const bool valid = q < count;
       Shadow shA, shB, shE, shV;  // area light / point light / environment / volume light
       shA.on = false;
@@ -2037,20 +2050,20 @@ void launchExtend(const DevScene* single, const DevJob* jobs, int width, const D
 void launchShade(const DevScene* single, const DevRender* singleR, const DevJob* jobs, const DevQueues& Q, int iter,
                  int grid, cudaStream_t st, int multiMediaLevel) {
   if (!single) {
-    if (multiMediaLevel >= 2) k_shade<true, true, 2><<<grid, 256, 0, st>>>(DevScene{}, DevRender{}, jobs, Q, iter);
-    else k_shade<true, true, 1><<<grid, 256, 0, st>>>(DevScene{}, DevRender{}, jobs, Q, iter);
+    if (multiMediaLevel >= 2) k_shade<true, true, 2><<<grid, kShadeBlock, 0, st>>>(DevScene{}, DevRender{}, jobs, Q, iter);
+    else k_shade<true, true, 1><<<grid, kShadeBlock, 0, st>>>(DevScene{}, DevRender{}, jobs, Q, iter);
     return;
   }
   const bool env = single->envOn != 0;
   const int ml = single->mediaLevel;
   if (!env) {
-    if (ml == 0) k_shade<false, false, 0><<<grid, 256, 0, st>>>(*single, *singleR, jobs, Q, iter);
-    else if (ml == 1) k_shade<false, false, 1><<<grid, 256, 0, st>>>(*single, *singleR, jobs, Q, iter);
-    else k_shade<false, false, 2><<<grid, 256, 0, st>>>(*single, *singleR, jobs, Q, iter);
+    if (ml == 0) k_shade<false, false, 0><<<grid, kShadeBlock, 0, st>>>(*single, *singleR, jobs, Q, iter);
+    else if (ml == 1) k_shade<false, false, 1><<<grid, kShadeBlock, 0, st>>>(*single, *singleR, jobs, Q, iter);
+    else k_shade<false, false, 2><<<grid, kShadeBlock, 0, st>>>(*single, *singleR, jobs, Q, iter);
   } else {
-    if (ml == 0) k_shade<false, true, 0><<<grid, 256, 0, st>>>(*single, *singleR, jobs, Q, iter);
-    else if (ml == 1) k_shade<false, true, 1><<<grid, 256, 0, st>>>(*single, *singleR, jobs, Q, iter);
-    else k_shade<false, true, 2><<<grid, 256, 0, st>>>(*single, *singleR, jobs, Q, iter);
+    if (ml == 0) k_shade<false, true, 0><<<grid, kShadeBlock, 0, st>>>(*single, *singleR, jobs, Q, iter);
+    else if (ml == 1) k_shade<false, true, 1><<<grid, kShadeBlock, 0, st>>>(*single, *singleR, jobs, Q, iter);
+    else k_shade<false, true, 2><<<grid, kShadeBlock, 0, st>>>(*single, *singleR, jobs, Q, iter);
   }
 }
 void launchConnect(const DevScene* single, const DevJob* jobs, int width, const DevQueues& Q, int iter, int which,
