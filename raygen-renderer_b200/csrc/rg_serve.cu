@@ -146,7 +146,7 @@ struct rg_server {
   DevSegment* hostSegs = nullptr;
   DevWave* hostWave = nullptr;
   // wave graphs: [0] homogeneous media only, [1] procedural media and volume lights
-  cudaGraphExec_t graph[2] = {nullptr, nullptr};
+  cudaGraphExec_t graph[3] = {nullptr, nullptr, nullptr};
   int maxIter = 12;
   // statistics
   std::vector<double> latencies;
@@ -213,7 +213,9 @@ bool allocServer(rg_server* s) {
 
 // Capture the multi-job wave (generate, bounce loop, accumulate) once per
 // kernel set: graph[0] with the homogeneous-media shade kernel, graph[1] with
-// the procedural-media kernel and the volume-light shadow queue.
+// the procedural-media kernel and the volume-light shadow queue, graph[2] for
+// waves whose jobs have area lights only: no media, environment or point
+// lights, so neither their code in the shade kernel nor their shadow queues.
 bool captureGraph(rg_server* s) {
   const DevQueues Q = serverQueues(s);
   // traversal: persistent warps, blocks per SM up to the occupancy limit
@@ -221,14 +223,14 @@ bool captureGraph(rg_server* s) {
   const int ext = s->numSMs * (tb > 0 ? std::min(tb, residentBlocks(0, 8)) : residentBlocks(0, 8));
   const int conn = s->numSMs * (tb > 0 ? std::min(tb, residentBlocks(1, 8)) : residentBlocks(1, 8));
   const int shadeGrid = s->numSMs * (s->cfg.shade_blocks_per_sm > 0 ? s->cfg.shade_blocks_per_sm : 4);
-  for (int k = 0; k < 2; k++) {
-    const bool procedural = k == 1;
+  for (int k = 0; k < 3; k++) {
+    const bool procedural = k == 1, plain = k == 2;
     cudaGraph_t g;
     if (cudaStreamBeginCapture(s->stream, cudaStreamCaptureModeThreadLocal) != cudaSuccess) return false;
     auto connects = [&](int it, cudaStream_t cs) {
       launchConnect(nullptr, s->jobTable.p, 8, Q, it, 0, conn, cs);
-      launchConnect(nullptr, s->jobTable.p, 8, Q, it, 1, conn, cs);
-      launchConnect(nullptr, s->jobTable.p, 8, Q, it, 2, conn, cs);
+      if (!plain) launchConnect(nullptr, s->jobTable.p, 8, Q, it, 1, conn, cs);
+      if (!plain) launchConnect(nullptr, s->jobTable.p, 8, Q, it, 2, conn, cs);
       if (procedural) launchConnect(nullptr, s->jobTable.p, 8, Q, it, 3, conn, cs);
     };
     launchGenerate(s->jobTable.p, s->waveSlot.p, Q, shadeGrid * 2, s->stream);
@@ -243,7 +245,7 @@ bool captureGraph(rg_server* s) {
       }
       launchExtend(nullptr, s->jobTable.p, 8, Q, it, ext, s->stream);
       if (it > 0) cudaStreamWaitEvent(s->stream, s->join, 0);
-      launchShade(nullptr, nullptr, s->jobTable.p, Q, it, shadeGrid, s->stream, procedural ? 2 : 1);
+      launchShade(nullptr, nullptr, s->jobTable.p, Q, it, shadeGrid, s->stream, procedural ? 2 : (plain ? 0 : 1));
     }
     if (Q.maxIter > 0) connects(Q.maxIter - 1, s->stream);
     launchAccumulate(s->jobTable.p, s->waveSlot.p, Q, shadeGrid, s->stream);
@@ -514,8 +516,13 @@ void serverLoop(rg_server* s) {
       cudaEventRecord(e0, st);
       // the procedural-media kernel only for waves that hold such a job
       bool procedural = false;
-      for (auto& pe : plan) procedural = procedural || pe.first->S.mediaLevel >= 2;
-      cudaGraphLaunch(s->graph[procedural ? 1 : 0], st);
+      bool plain = true;
+      for (auto& pe : plan) {
+        const DevScene& S = pe.first->S;
+        procedural = procedural || S.mediaLevel >= 2;
+        plain = plain && S.mediaLevel == 0 && !S.envOn && S.numPointLights == 0;
+      }
+      cudaGraphLaunch(s->graph[procedural ? 1 : (plain ? 2 : 0)], st);
       cudaEventRecord(e1, st);
       const cudaError_t ce = cudaStreamSynchronize(st);
       float ms = 0;

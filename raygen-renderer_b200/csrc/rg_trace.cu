@@ -2051,7 +2051,8 @@ void launchShade(const DevScene* single, const DevRender* singleR, const DevJob*
                  int grid, cudaStream_t st, int multiMediaLevel) {
   if (!single) {
     if (multiMediaLevel >= 2) k_shade<true, true, 2><<<grid, kShadeBlock, 0, st>>>(DevScene{}, DevRender{}, jobs, Q, iter);
-    else k_shade<true, true, 1><<<grid, kShadeBlock, 0, st>>>(DevScene{}, DevRender{}, jobs, Q, iter);
+    else if (multiMediaLevel == 1) k_shade<true, true, 1><<<grid, kShadeBlock, 0, st>>>(DevScene{}, DevRender{}, jobs, Q, iter);
+    else k_shade<true, false, 0><<<grid, kShadeBlock, 0, st>>>(DevScene{}, DevRender{}, jobs, Q, iter);
     return;
   }
   const bool env = single->envOn != 0;

@@ -16,7 +16,8 @@ void launchGenerate(const DevJob* jobs, const DevWave* W, const DevQueues& Q, in
 void launchExtend(const DevScene* single, const DevJob* jobs, int width, const DevQueues& Q, int iter, int grid,
                   cudaStream_t st);
 // single == nullptr: the multi-job kernel; multiMediaLevel 2 includes the
-// procedural-media code, 1 homogeneous media only (no volume-light queue)
+// procedural-media code, 1 homogeneous media only (no volume-light queue), 0 neither
+// media nor an environment
 void launchShade(const DevScene* single, const DevRender* singleR, const DevJob* jobs, const DevQueues& Q, int iter,
                  int grid, cudaStream_t st, int multiMediaLevel = 2);
 void launchConnect(const DevScene* single, const DevJob* jobs, int width, const DevQueues& Q, int iter, int which,
