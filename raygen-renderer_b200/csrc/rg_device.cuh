@@ -201,8 +201,8 @@ struct DevJob {
 
 // A wave is a list of segments; segment k holds paths
 // [pathBase, pathBase + numPixels * samples) of job `slot`:
-//   path = pathBase + s * numPixels + i, pixel = pixelList ? pixelList[pixelOffset + i] : pixelOffset + i,
-//   sample = cnt[pixel] + s.
+//   path = pathBase + place * samples + s, i = tileOrder(place),
+//   pixel = pixelList ? pixelList[pixelOffset + i] : pixelOffset + i, sample = cnt[pixel] + s.
 struct DevSegment {
   int slot;
   int numPixels;

@@ -616,6 +616,33 @@ __device__ void primaryRay(const DevRender& R, const Rng& rng, int x, int y, V3&
   }
 }
 
+// Order of a segment's pixels among its paths: place i of n -> pixel index.  Rows are taken 32
+// at a time in blocks of 32 x 32 pixels, blocks in tiles of 8 x 4; columns past the last block
+// and rows past the last 32 follow in row order.  Path p of a segment is sample p % samples of
+// place p / samples, so a warp's primary rays, and a shade window's bounces, come from one
+// pixel or a few neighbours and their traversals share nodes and triangles.  In row order, one
+// sample after the other: 146.9 ms of tracing for 1920x1080 with 8 samples on the spheres scene
+// (extend 78.3, connect 29.9, shade 36.0); in tiles 145.9; in tiles with a pixel's samples side
+// by side 142.0 (75.6, 29.4, 34.6).  A room at 256x256: 0.891 -> 0.881.
+__device__ __forceinline__ int tileOrder(int i, int n, int W) {
+  if (W > n >> 5) return i;
+  const int group = 32 * W, g = i / group, r = i - g * group;
+  if (n - g * group < group) return i;
+  const int cols = W & ~31;
+  if (r < 32 * cols) {
+    const int block = r >> 10, tile = (r >> 5) & 31, l = r & 31;
+    return g * group + ((tile >> 2) * 4 + (l >> 3)) * W + block * 32 + (tile & 3) * 8 + (l & 7);
+  }
+  const int e = r - 32 * cols, w = W - cols;
+  return g * group + (e / w) * W + cols + e % w;
+}
+
+// Pixel at a place of a segment (a pixel list holds the rows of 32-wide tiles).
+__device__ __forceinline__ int segmentPixel(const DevSegment& seg, const DevRender& R, int place) {
+  const int i = tileOrder(place, seg.numPixels, seg.pixelList ? 32 : R.width);
+  return seg.pixelList ? seg.pixelList[seg.pixelOffset + i] : seg.pixelOffset + i;
+}
+
 __global__ void __launch_bounds__(256) k_generate(const DevJob* __restrict__ jobs, const DevWave* __restrict__ Wp,
                                                   DevQueues Q) {
   const DevWave W = *Wp;
@@ -627,11 +654,10 @@ __global__ void __launch_bounds__(256) k_generate(const DevJob* __restrict__ job
   }
   for (int p = blockIdx.x * blockDim.x + threadIdx.x; p < numPaths; p += gridDim.x * blockDim.x) {
     const DevSegment seg = W.segs[segmentOfPath(W, p)];
-    const int local = p - seg.pathBase;
-    const int i = local % seg.numPixels, sl = local / seg.numPixels;
-    const int pixel = seg.pixelList ? seg.pixelList[seg.pixelOffset + i] : seg.pixelOffset + i;
     const DevJob& J = jobs[seg.slot];
     const DevRender& R = J.R;
+    const int local = p - seg.pathBase, place = local / seg.samples, sl = local - place * seg.samples;
+    const int pixel = segmentPixel(seg, R, place);
     const int x = pixel % R.width, y = pixel / R.width;
     const uint32_t sample = (uint32_t)(J.cnt[pixel] + sl);
     Rng rng;
@@ -1725,11 +1751,10 @@ __global__ void __launch_bounds__(128) k_simple(const DevJob* __restrict__ jobs,
   uint32_t nodes = 0, tris = 0;
   for (int p = blockIdx.x * blockDim.x + threadIdx.x; p < numPaths; p += gridDim.x * blockDim.x) {
     const DevSegment seg = W.segs[segmentOfPath(W, p)];
-    const int local = p - seg.pathBase;
-    const int li = local % seg.numPixels, sl = local / seg.numPixels;
-    const int pixel = seg.pixelList ? seg.pixelList[seg.pixelOffset + li] : seg.pixelOffset + li;
     const DevScene& S = jobs[seg.slot].S;
     const DevRender& R = jobs[seg.slot].R;
+    const int local = p - seg.pathBase, place = local / seg.samples, sl = local - place * seg.samples;
+    const int pixel = segmentPixel(seg, R, place);
     const int x = pixel % R.width, y = pixel / R.width;
     const uint32_t sample = (uint32_t)(jobs[seg.slot].cnt[pixel] + sl);
     Rng rng;
@@ -1796,14 +1821,12 @@ __global__ void __launch_bounds__(256) k_accumulate(const DevJob* __restrict__ j
   const DevWave W = *Wp;
   for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < W.numPixelsTotal; t += gridDim.x * blockDim.x) {
     const DevSegment seg = W.segs[segmentOfPixel(W, t)];
-    const int i = t - seg.pixBase;
-    const int pixel = seg.pixelList ? seg.pixelList[seg.pixelOffset + i] : seg.pixelOffset + i;
     const DevJob& J = jobs[seg.slot];
     const DevRender& R = J.R;
+    const int place = t - seg.pixBase, pixel = segmentPixel(seg, R, place);
     float sr = 0, sg = 0, sb = 0, qr = 0, qg = 0, qb = 0;
     for (int s = 0; s < seg.samples; s++) {
-      const int p = seg.pathBase + s * seg.numPixels + i;
-      const float4 l = Q.pathL[p];
+      const float4 l = Q.pathL[seg.pathBase + place * seg.samples + s];
       const bool noHit = (__float_as_int(l.w) & kVtxEyeNoHit) != 0;
       float r = l.x, g = l.y, b = l.z;
       if (noHit && r == 0.0f && g == 0.0f && b == 0.0f) { r = R.backR; g = R.backG; b = R.backB; }
