@@ -5,15 +5,21 @@
 // array's pages and the copy out of the driver's buffer, against 0.7 ms on the
 // link.  Here a few host threads, each with two page-locked slots and a stream
 // of its own, take chunks in turn: while one slot is on the link, the other is
-// copied.  Page-locked callers and small copies keep the direct copy.
+// copied.  Page-locked callers, small copies and images into pages that are already
+// there keep the direct copy.
 //
 // The page-locked slots and streams are pooled (at most kKept sets, 8 MB each)
 // while any renderer or denoiser exists, and freed with the last one; threads
 // live only for the copy.  Every set is used by one copy at a time.
 #include <cuda_runtime.h>
 
+#include <sys/mman.h>
+#include <unistd.h>
+
 #include <algorithm>
 #include <atomic>
+#include <cstdint>
+#include <cstdlib>
 #include <cstring>
 #include <mutex>
 #include <thread>
@@ -26,13 +32,26 @@ namespace {
 
 constexpr int kWorkers = 8;
 constexpr size_t kChunk = size_t(512) << 10;
-// Below this a direct copy is as fast (the threads take about 0.1 ms to start).
-constexpr size_t kStagedBytes = size_t(3) << 20;
+// Direct / staged copies on 16 host cores, ms.  To the device: 3 MB 0.42 / 0.23, 8 MB 1.13 / 0.45,
+// 33 MB 2.98 / 1.48, 128 MB 12.0 / 5.3.  To untouched pages: 3 MB 1.42 / 0.75, 8 MB 3.73 / 0.85,
+// 33 MB 14.1 / 2.3.  To touched pages: 8 MB 0.46 / 0.71, 33 MB 1.82 / 1.88, 64 MB 3.50 / 3.16.
+constexpr size_t kStagedBytes = size_t(3) << 20, kStagedTouched = size_t(48) << 20;
+// A set takes 1 - 1.6 ms to make, which a staged copy earns at about 0.05 ms per MB to the device and
+// six times that to untouched pages: copies stay direct until those that could have been staged
+// would nearly have paid for it (the first 1M shadow rays, 28 MB: 2.7 ms with a set made for them,
+// 4.0 without).
+constexpr size_t kSetCost = size_t(16) << 20;
+constexpr int kUntouchedGain = 6;
 constexpr int kKept = 2;
+// The slots are page-locked where they lie, in huge pages: a first copy waits 1.2 ms for them,
+// and 3.3 - 6.3 ms for the 2048 small pages of a cudaHostAlloc.
+constexpr size_t kHugePage = size_t(2) << 20, kSlotBytes = kWorkers * 2 * kChunk;
+static_assert(kSlotBytes % kHugePage == 0, "whole huge pages");
 
 struct Stage {
   int device = 0;
   unsigned char* slots = nullptr;  // [kWorkers][2][kChunk], page-locked
+  bool registered = false;
   cudaStream_t stream[kWorkers] = {};
   cudaEvent_t done[kWorkers][2] = {};
   cudaEvent_t start = nullptr;
@@ -43,12 +62,15 @@ struct Stage {
       if (stream[w]) cudaStreamDestroy(stream[w]);
     }
     if (start) cudaEventDestroy(start);
-    if (slots) cudaFreeHost(slots);
+    if (registered) cudaHostUnregister(slots);
+    std::free(slots);
   }
   bool init(int dev) {
     device = dev;
-    if (cudaHostAlloc((void**)&slots, kWorkers * 2 * kChunk, cudaHostAllocPortable) != cudaSuccess) slots = nullptr;
-    bool ok = slots && cudaEventCreateWithFlags(&start, cudaEventDisableTiming) == cudaSuccess;
+    slots = static_cast<unsigned char*>(std::aligned_alloc(kHugePage, kSlotBytes));
+    if (slots) madvise(slots, kSlotBytes, MADV_HUGEPAGE);
+    registered = slots && cudaHostRegister(slots, kSlotBytes, cudaHostRegisterPortable) == cudaSuccess;
+    bool ok = registered && cudaEventCreateWithFlags(&start, cudaEventDisableTiming) == cudaSuccess;
     for (int w = 0; ok && w < kWorkers; ++w) {
       ok = cudaStreamCreateWithFlags(&stream[w], cudaStreamNonBlocking) == cudaSuccess;
       for (int s = 0; ok && s < 2; ++s) ok = cudaEventCreateWithFlags(&done[w][s], cudaEventDisableTiming) == cudaSuccess;
@@ -60,9 +82,10 @@ struct Stage {
 
 std::mutex g_mu;
 int g_users = 0;
+size_t g_missed = 0;  // gain of the copies made directly for want of a set
 Stage* g_free[kKept] = {};
 
-Stage* acquire() {
+Stage* acquire(size_t gain) {
   int dev = 0;
   if (cudaGetDevice(&dev) != cudaSuccess) return nullptr;
   {
@@ -70,6 +93,11 @@ Stage* acquire() {
     if (g_users == 0) return nullptr;  // nothing would keep the set: not worth its allocation
     for (auto& f : g_free)
       if (f && f->device == dev) return std::exchange(f, nullptr);
+    if (gain < kSetCost - g_missed) {
+      g_missed += gain;
+      return nullptr;
+    }
+    g_missed = 0;
   }
   Stage* s = new (std::nothrow) Stage();
   if (s && !s->init(dev)) {
@@ -99,6 +127,17 @@ bool pageable(const void* p) {
     return false;
   }
   return a.type == cudaMemoryTypeUnregistered;
+}
+
+// Whether the bytes lie in pages that are already there (looked up at 16 of them).
+bool touched(const unsigned char* p, size_t bytes) {
+  const uintptr_t page = (uintptr_t)sysconf(_SC_PAGESIZE), a = (uintptr_t)p;
+  for (int k = 0; k < 16; ++k) {
+    unsigned char in = 0;
+    const uintptr_t at = (a + (bytes - 1) / 15 * k) & ~(page - 1);
+    if (mincore((void*)at, 1, &in) != 0 || !(in & 1)) return false;
+  }
+  return true;
 }
 
 // One worker's share: chunks off the common counter, two in flight.
@@ -139,7 +178,8 @@ bool staged(bool toHost, void* host, void* dev, size_t bytes, cudaStream_t after
   if (bytes < kStagedBytes || !pageable(host)) return false;
   cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
   if (cudaStreamIsCapturing(after, &cap) != cudaSuccess || cap != cudaStreamCaptureStatusNone) return false;
-  Stage* s = acquire();
+  if (toHost && bytes < kStagedTouched && touched((const unsigned char*)host, bytes)) return false;
+  Stage* s = acquire(toHost ? bytes * kUntouchedGain : bytes);
   if (!s) return false;
   const int chunks = (int)std::min<size_t>(kWorkers, (bytes + 2 * kChunk - 1) / (2 * kChunk));
   const int cores = (int)std::thread::hardware_concurrency();
@@ -180,8 +220,10 @@ StageUser::~StageUser() {
   Stage* old[kKept] = {};
   {
     std::lock_guard<std::mutex> lk(g_mu);
-    if (--g_users == 0)
+    if (--g_users == 0) {
       for (int i = 0; i < kKept; ++i) old[i] = std::exchange(g_free[i], nullptr);
+      g_missed = 0;
+    }
   }
   for (auto* s : old) delete s;
 }

@@ -45,6 +45,19 @@ def test_query_sizes(rg, n):
     r.close()
 
 
+def test_sizes_once_slots_are_there(rg):
+    """The first large batch makes the slots; around 3 MB in, with and without ragged chunks."""
+    r = renderer(rg)
+    r.trace_closest(rays_of(1500000, 1))
+    for n in (131071, 131072, 131073, 174763, 400001):
+        rays = rays_of(n, n)
+        want_tuv, want_prim = in_pieces(r, rays)
+        tuv, prim = r.trace_closest(rays)
+        np.testing.assert_array_equal(prim, want_prim)
+        np.testing.assert_array_equal(tuv, want_tuv)
+    r.close()
+
+
 def test_threads_with_their_own_handles(rg):
     errors = []
 
