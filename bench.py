@@ -14,7 +14,7 @@ depth 3, seed 1.  A step is one full render of that job.
                uploads the scene (rg_set_scene, BVH build included), renders and
                reads the HDR image back (rg_get_hdr); host wall clock.
 * roofline   : closest-hit (extend) kernel: algorithmic bytes = rays x 48 B
-               (32 B ray in + 16 B hit out) + nodes visited x 208 B (8-wide) + triangles
+               (32 B ray in + 16 B hit out) + nodes visited x 128 B (8-wide) + triangles
                tested x 48 B, over its CUDA-event time, against the measured HBM
                copy bandwidth.
 * cpu_baseline: the CPU restatement (oracle, reference compiler flags) on the
@@ -212,7 +212,7 @@ def pinned_array(shape):
 
 def cpu_scene(scene_ptr):
     sys.path.insert(0, os.path.join(ROOT, "oracle"))
-    import oracle  # checker / baseline only
+    import oracle  # comparison and baseline only
     t0 = time.time()
     o = oracle.OracleScene(scene_ptr, bins=16, fast=True)
     return o, time.time() - t0
@@ -858,7 +858,7 @@ def main():
     s = r.stats()
     os.environ.pop("RG_PROFILE_KERNELS", None)
     ext_ms = s["extend_ms"]
-    node_bytes = 208 if st.bvhWidth == 8 else 64  # 8-wide: header + float planes of 8 child boxes
+    node_bytes = 128 if st.bvhWidth == 8 else 64  # 8-wide: header + half planes of 8 child boxes
     alg_bytes = s["closest_rays"] * 48 + s["nodes_visited"] * node_bytes + s["tris_tested"] * 48
     launches_ext = s["waves"] * (DEPTH + 2)
     achieved = alg_bytes / (ext_ms * 1e-3) / 1e9 if ext_ms > 0 else None
@@ -914,7 +914,7 @@ def main():
             "config": {"workload": "heavy geometry single job: 4 x 1,003,520-triangle displaced icospheres "
                                    "in a 20x20 room, 16 emissive quads, metal/dielectric",
                        "triangles": ntris, "resolution": f"{Wr}x{Hr}", "spp": args.spp, "max_depth": DEPTH,
-                       "bvh": f"device binned SAH (32 bins), {st.bvhWidth}-wide" + (" (float planes)" if st.bvhWidth == 8 else ""),
+                       "bvh": f"device binned SAH (32 bins), {st.bvhWidth}-wide" + (" (half planes)" if st.bvhWidth == 8 else ""),
                        "bvh_build_ms": round(build_ms, 2),
                        "l2": "inputs larger than L2 (BVH + triangles ~400 MB)",
                        "parallelism": f"replicas x{world}" if world > 1 else "single GPU"},

@@ -145,7 +145,8 @@ struct rg_server {
   DevBuf<int> errWord;
   DevSegment* hostSegs = nullptr;
   DevWave* hostWave = nullptr;
-  // wave graphs: [0] homogeneous media only, [1] procedural media and volume lights
+  // wave graphs: [0] homogeneous media only, [1] procedural media and volume lights, [2] area
+  // lights only
   cudaGraphExec_t graph[3] = {nullptr, nullptr, nullptr};
   int maxIter = 12;
   // statistics
