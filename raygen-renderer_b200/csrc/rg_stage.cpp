@@ -19,7 +19,6 @@
 #include <algorithm>
 #include <atomic>
 #include <cstdint>
-#include <cstdlib>
 #include <cstring>
 #include <mutex>
 #include <thread>
@@ -45,12 +44,14 @@ constexpr int kUntouchedGain = 6;
 constexpr int kKept = 2;
 // The slots are page-locked where they lie, in huge pages: a first copy waits 1.2 ms for them,
 // and 3.3 - 6.3 ms for the 2048 small pages of a cudaHostAlloc.
-constexpr size_t kHugePage = size_t(2) << 20, kSlotBytes = kWorkers * 2 * kChunk;
+constexpr size_t kHugePage = size_t(2) << 20, kSlotBytes = kWorkers * 2 * kChunk,
+                 kMapBytes = kSlotBytes + kHugePage;
 static_assert(kSlotBytes % kHugePage == 0, "whole huge pages");
 
 struct Stage {
   int device = 0;
   unsigned char* slots = nullptr;  // [kWorkers][2][kChunk], page-locked
+  void* map = nullptr;
   bool registered = false;
   cudaStream_t stream[kWorkers] = {};
   cudaEvent_t done[kWorkers][2] = {};
@@ -63,12 +64,17 @@ struct Stage {
     }
     if (start) cudaEventDestroy(start);
     if (registered) cudaHostUnregister(slots);
-    std::free(slots);
+    if (map) munmap(map, kMapBytes);
   }
   bool init(int dev) {
     device = dev;
-    slots = static_cast<unsigned char*>(std::aligned_alloc(kHugePage, kSlotBytes));
-    if (slots) madvise(slots, kSlotBytes, MADV_HUGEPAGE);
+    map = mmap(nullptr, kMapBytes, PROT_READ | PROT_WRITE, MAP_PRIVATE | MAP_ANONYMOUS, -1, 0);
+    if (map == MAP_FAILED) map = nullptr;
+    if (map) {
+      slots = reinterpret_cast<unsigned char*>(((uintptr_t)map + kHugePage - 1) & ~(uintptr_t)(kHugePage - 1));
+      madvise(slots, kSlotBytes, MADV_HUGEPAGE);
+      madvise(slots, kSlotBytes, MADV_DONTFORK);  // a forked child must not turn the locked pages copy-on-write
+    }
     registered = slots && cudaHostRegister(slots, kSlotBytes, cudaHostRegisterPortable) == cudaSuccess;
     bool ok = registered && cudaEventCreateWithFlags(&start, cudaEventDisableTiming) == cudaSuccess;
     for (int w = 0; ok && w < kWorkers; ++w) {
