@@ -881,12 +881,6 @@ __global__ void k_innerFlags(int numNodes, const BNode* __restrict__ nodes, int*
   if (i < numNodes) flags[i] = nodes[i].left >= 0 ? 1 : 0;
 }
 
-// Margin of every box against the rounding of the slab test, besides the relative one below:
-// a plane's distance is (origin + scale p - o) inv with three roundings, each of up to 2^-24 of
-// the distance between the ray's origin and the node, which the scene's reach bounds
-// (largest view-space coordinate, the camera being the origin, and extent).
-constexpr float kReachMargin = 4.0f / 16777216.0f;
-
 __device__ __forceinline__ float inflateLo(float x) { return x - fmaxf(fabsf(x), 1.0f) * 2e-6f; }
 __device__ __forceinline__ float inflateHi(float x) { return x + fmaxf(fabsf(x), 1.0f) * 2e-6f; }
 
@@ -948,14 +942,6 @@ __global__ void __launch_bounds__(128) k_collapse(const int* __restrict__ count,
                                                   const BNode* __restrict__ nodes, const int* __restrict__ primIdx,
                                                   float4* __restrict__ nodes8, int* counters, int2* __restrict__ nextTasks,
                                                   int* nextCount, int* __restrict__ triOrder, int maxNodes8) {
-  // the scene's reach, from the root's box
-  float reach = 0.0f, span = 0.0f;
-  for (int k = 0; k < 3; k++) {
-    const float a = nodes[0].bmin[k], b = nodes[0].bmax[k];
-    reach = fmaxf(reach, fmaxf(fabsf(a), fabsf(b)));
-    span = fmaxf(span, b - a);
-  }
-  const float margin = kReachMargin * (reach + span);
   constexpr unsigned kAll = 0xffffffffu;
   const int numTasks = *count;
   const int lane = threadIdx.x & 7, shift = threadIdx.x & 24;  // lane of the node's eight, their place in the warp
@@ -1019,8 +1005,8 @@ __global__ void __launch_bounds__(128) k_collapse(const int* __restrict__ count,
     const bool mine = lane < nc;
     float lo[3], hi[3], ctr[3], cc[3];
     for (int k = 0; k < 3; k++) {
-      lo[k] = minOf(mine ? inflateLo(bmin[k]) - margin : FLT_MAX);
-      hi[k] = maxOf(mine ? inflateHi(bmax[k]) + margin : -FLT_MAX);
+      lo[k] = minOf(mine ? inflateLo(bmin[k]) : FLT_MAX);
+      hi[k] = maxOf(mine ? inflateHi(bmax[k]) : -FLT_MAX);
       ctr[k] = 0.5f * (lo[k] + hi[k]);
       cc[k] = 0.5f * (bmin[k] + bmax[k]);
     }
@@ -1088,7 +1074,9 @@ __global__ void __launch_bounds__(128) k_collapse(const int* __restrict__ count,
     // The origin of the planes is, per axis, the node's low end, centre or high end: the one
     // closest to the planes of thin boxes (walls, floors, lamps), whose rounding matters most
     // because rays start and end at such surfaces.
-    float org[3], ext = 0.0f;
+    // margin: against the slab test's rounding, which is up to 2 x 2^-24 of the planes' distance from
+    // their origin besides a part that grows with the ray's way to the box (kNearScale)
+    float org[3], margin[3], ext = 0.0f;
     for (int k = 0; k < 3; k++) {
       const float cand[3] = {ctr[k], lo[k], hi[k]}, thin = (hi[k] - lo[k]) * (1.0f / 256.0f);
       float best = FLT_MAX;
@@ -1101,7 +1089,9 @@ __global__ void __launch_bounds__(128) k_collapse(const int* __restrict__ count,
           org[k] = cand[q];
         }
       }
-      ext = fmaxf(ext, fmaxf(__fsub_ru(hi[k], org[k]), __fsub_ru(org[k], lo[k])));
+      const float e = fmaxf(__fsub_ru(hi[k], org[k]), __fsub_ru(org[k], lo[k]));
+      margin[k] = e * (8.0f / 16777216.0f);
+      ext = fmaxf(ext, __fadd_ru(e, margin[k]));
     }
     // planes as half values, rounded outward; an empty slot keeps an inverted box, and a node
     // that is not of finite size has boxes that every ray enters
@@ -1122,8 +1112,8 @@ __global__ void __launch_bounds__(128) k_collapse(const int* __restrict__ count,
         __half v = __float2half_rn(h ? -65504.0f : 65504.0f);
         if (full) {
           if (!finite) v = h ? __float2half_ru(INFINITY) : __float2half_rd(-INFINITY);
-          else if (h) v = __float2half_ru(__fsub_ru(inflateHi(cMax[k]) + margin, org[k]) * toHalf);
-          else v = __float2half_rd(__fsub_rd(inflateLo(cMin[k]) - margin, org[k]) * toHalf);
+          else if (h) v = __float2half_ru(__fsub_ru(inflateHi(cMax[k]) + margin[k], org[k]) * toHalf);
+          else v = __float2half_rd(__fsub_rd(inflateLo(cMin[k]) - margin[k], org[k]) * toHalf);
         }
         reinterpret_cast<__half*>(o + ((2 + 2 * k + h) ^ sw))[lane] = v;
       }

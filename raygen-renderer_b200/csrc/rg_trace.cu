@@ -1945,7 +1945,7 @@ __global__ void __launch_bounds__(128) k_queryWarp(DevScene S, const float* __re
     const float scale = __uint_as_float(pack & 0x7f800000u);
     const V3 Sc = v3(scale * inv.x, scale * inv.y, scale * inv.z);
     const V3 C = v3((g.x - o.x) * inv.x, (g.y - o.y) * inv.y, (g.z - o.z) * inv.z);
-    const float tmin = fmax3f(fmaf(pl[0][0], Sc.x, C.x), fmaf(pl[1][0], Sc.y, C.y), fmaf(pl[2][0], Sc.z, C.z));
+    const float tmin = kNearScale * fmax3f(fmaf(pl[0][0], Sc.x, C.x), fmaf(pl[1][0], Sc.y, C.y), fmaf(pl[2][0], Sc.z, C.z));
     const float tfar = fmin3f(fmaf(pl[0][1], Sc.x, C.x), fmaf(pl[1][1], Sc.y, C.y), fmaf(pl[2][1], Sc.z, C.z));
     const unsigned hits = __ballot_sync(kAll, fmaxf(tmin, 0.0f) <= fminf(tfar, tmax)) & 0xffu;
     const uint32_t imask = pack & 0xffu;
