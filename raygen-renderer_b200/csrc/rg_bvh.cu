@@ -266,9 +266,10 @@ __device__ __forceinline__ void binPrim(uint32_t (&sb)[13], const uint32_t (&v)[
 // with primIdx in the partition), so the pass reads them coalesced.
 __global__ void __launch_bounds__(256) k_bin(int n, const int* __restrict__ primNode, const BNode* __restrict__ nodes,
                                              const float4* __restrict__ bmin, const float4* __restrict__ bmax,
-                                             BinData* bins, int nbins) {
+                                             BinData* bins, int nbins, const int* __restrict__ err) {
   __shared__ uint32_t sb[2][kMaxBins][13];
   __shared__ int sNode[2];  // lowest and highest open node id of the chunk
+  const bool failed = *err != 0;
   const int first = blockIdx.x * kBinChunk;
   const int last = min(n, first + kBinChunk);
   if (threadIdx.x == 0) {
@@ -302,7 +303,7 @@ __global__ void __launch_bounds__(256) k_bin(int n, const int* __restrict__ prim
   }
   __syncthreads();
   const int nodeA = sNode[0], nodeB = sNode[1];
-  if (nodeB < 0) return;
+  if (nodeB < 0 || failed) return;
   const BNode ndA = nodes[nodeA], ndB = nodes[nodeB];
   const bool onA = ndA.binSlot >= 0 && ndA.cmax[ndA.axis] - ndA.cmin[ndA.axis] >= 1e-12f;
   const bool onB = ndB.binSlot >= 0 && ndB.cmax[ndB.axis] - ndB.cmin[ndB.axis] >= 1e-12f;
@@ -360,7 +361,8 @@ __global__ void __launch_bounds__(256) k_bin(int n, const int* __restrict__ prim
 // block inside one node, global atomics across nodes.
 __global__ void __launch_bounds__(256) k_binAny(int n, const int* __restrict__ primNode, const BNode* __restrict__ nodes,
                                              const float4* __restrict__ bmin, const float4* __restrict__ bmax,
-                                             BinData* bins, int nbins) {
+                                             BinData* bins, int nbins, const int* __restrict__ err) {
+  if (*err) return;
   __shared__ uint32_t sb[kMaxBins][13];
   const int first = blockIdx.x * kBinChunk;
   if (first >= n) return;
@@ -571,8 +573,12 @@ __device__ __forceinline__ int warpScanI(int v, int lane, bool reverse) {
 // Split of node nd from its bins, lane b's bin in (cnt, b*, c*): ordered-uint bounds of the
 // primitives and of their centroids, identities when empty.  All lanes return the split (bin,
 // -1 leaf, -2 index median) and the children's counts and bounds (bmin, bmax, cmin, cmax).
+// A cost that is no number (a box of NaN, an area that overflows) compares with nothing and
+// can leave the lanes with different splits.  Lane 0's is the split; the node is refused (split
+// -1) where another lane would put its bin on the other side.
 struct WarpSplit {
   int split;
+  bool refused;
   int count[2];
   float bounds[2][12];
 };
@@ -621,8 +627,14 @@ __device__ __forceinline__ WarpSplit decideSplit(const BNode& nd, int nbins, int
   WarpSplit r;
   r.split = best;
   if (best < 0 && nd.count > maxLeaf) r.split = forced >= 0 ? forced : -2;  // -2: index median
+  const int own = r.split;
+  r.split = __shfl_sync(0xffffffffu, own, 0);
+  const bool same = !any || r.split < 0 || (own >= 0 && (lane <= own) == (lane <= r.split));
+  r.refused = !__all_sync(0xffffffffu, same);
+  if (r.refused) r.split = -1;
   const int at = r.split >= 0 ? r.split : 0;
-  r.count[0] = r.split >= 0 ? __shfl_sync(0xffffffffu, lc, at) : nd.count / 2;
+  const int lcAt = __shfl_sync(0xffffffffu, lc, at);
+  r.count[0] = r.split >= 0 ? lcAt : nd.count / 2;
   r.count[1] = (r.split >= 0 ? total : nd.count) - r.count[0];
   for (int k = 0; k < 3; k++) {
     // bounds: the scans at the split; centroid bounds: reductions of each side's bins
@@ -669,7 +681,8 @@ __device__ __forceinline__ void writeChild(BNode* nodes, int left, int side, int
 // still split (BVH_LEAF_SIZE 4, bvh.cpp:23) go to the block-wise pass.
 __global__ void __launch_bounds__(128) k_splitWarp(const int* count, int first, int most, const int* __restrict__ tasks,
                                                   BNode* nodes, BinData* bins, int nbins, int* nodeCounter, int* nextTasks,
-                                                  int* nextCount, int* smallTasks, int* smallCount, int maxLeaf) {
+                                                  int* nextCount, int* smallTasks, int* smallCount, int maxLeaf,
+                                                  int* err) {
   const int t = (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 5);
   const int lane = threadIdx.x & 31;
   if (t >= tasksOf(count, first, most)) return;
@@ -693,6 +706,7 @@ __global__ void __launch_bounds__(128) k_splitWarp(const int* count, int first, 
   const WarpSplit sp = decideSplit(nd, nbins, maxLeaf, cnt, bin);
   int left = -1;
   if (lane == 0) {
+    if (sp.refused) atomicCAS(err, 0, kErrPartition);
     if (sp.split != -1) left = atomicAdd(nodeCounter, 2);
     nodes[id].binSlot = -1;
     nodes[id].left = left;
@@ -716,7 +730,7 @@ constexpr int kSubThreads = 256;
 __global__ void __launch_bounds__(kSubThreads) k_subtrees(const int* __restrict__ count, const int* __restrict__ tasks,
                                                           BNode* nodes, int* primIdx, const float4* __restrict__ bmin,
                                                           const float4* __restrict__ bmax, int nbins, int* nodeCounter,
-                                                          int maxLeaf) {
+                                                          int maxLeaf, int* err) {
   constexpr int kWarps = kSubThreads / 32, kList = kSubtree / 5 + 1;  // nodes of five primitives and more
   __shared__ float sB[6][kSubtree];
   __shared__ int sIdx[kSubtree];
@@ -725,7 +739,10 @@ __global__ void __launch_bounds__(kSubThreads) k_subtrees(const int* __restrict_
   __shared__ int sList[2][kList];
   __shared__ int sCount[2], sBase;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const int numTasks = *count;
+  if (threadIdx.x == 0) sBase = *(volatile int*)err ? 0 : *count;  // one answer for the block: others may set it
+  __syncthreads();
+  const int numTasks = sBase;
+  __syncthreads();
   for (int task = blockIdx.x; task < numTasks; task += gridDim.x) {
     const int root = tasks[task];
     const int start = nodes[root].start, n = nodes[root].count;
@@ -782,6 +799,7 @@ __global__ void __launch_bounds__(kSubThreads) k_subtrees(const int* __restrict_
         for (int k = 0; k < 12; k++) bin[k] = bins[lane][k];
         const WarpSplit sp = decideSplit(nd, nbins, maxLeaf, lane < nbins ? (int)bins[lane][12] : 0, bin);
         if (lane == 0) {
+          if (sp.refused) atomicCAS(err, 0, kErrPartition);
           nodes[id].axis = nd.axis;
           nodes[id].binSlot = -1;
           nodes[id].left = sp.split == -1 ? -1 : left;
@@ -804,11 +822,16 @@ __global__ void __launch_bounds__(kSubThreads) k_subtrees(const int* __restrict_
           const bool toLeft = in && (sp.split == -2 ? j < sp.count[0] : binAt(p) <= sp.split);
           const unsigned m = __ballot_sync(0xffffffffu, toLeft);
           const int before = nl + __popc(m & ((1u << lane) - 1u));
-          if (in) sPerm[1][s0 + (toLeft ? before : sp.count[0] + j - before)] = (uint16_t)p;
+          const int to = toLeft ? before : sp.count[0] + j - before;
+          if (in && to < nd.count) sPerm[1][s0 + to] = (uint16_t)p;
           nl += __popc(m);
         }
         __syncwarp();
-        for (int j = lane; j < nd.count; j += 32) sPerm[0][s0 + j] = sPerm[1][s0 + j];
+        if (nl == sp.count[0]) {  // else not every place was written: the order stays
+          for (int j = lane; j < nd.count; j += 32) sPerm[0][s0 + j] = sPerm[1][s0 + j];
+        } else if (lane == 0) {
+          atomicCAS(err, 0, kErrPartition);
+        }
         __syncwarp();
       }
     }
@@ -823,10 +846,12 @@ __global__ void __launch_bounds__(kSubThreads) k_subtrees(const int* __restrict_
 // against 31 + 12 us, 20k 31 against 10).
 __global__ void k_partitionFlags(int n, const int* __restrict__ primNode, const BNode* __restrict__ nodes,
                                  const float4* __restrict__ bmin, const float4* __restrict__ bmax, int nbins,
-                                 int* __restrict__ flags) {
+                                 int* __restrict__ flags, const int* __restrict__ err) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
-  const int node = primNode[i];
+  const bool failed = *err != 0;
+  int node = primNode[i];
+  if (failed) node = -1;
   int flag = 0;
   if (node >= 0) {
     const BNode& nd = nodes[node];
@@ -845,7 +870,9 @@ __global__ void k_partitionFlags(int n, const int* __restrict__ primNode, const 
 // Partition, pass 2 (after an exclusive scan of the flags into `before`): a stable
 // scatter of each split node's primitives into its children's ranges, with their
 // bounds; primitives of closed nodes and new leaves stay where they are.  No
-// atomics, so the order (and the BVH) is the same on every run.
+// atomics, so the order (and the BVH) is the same on every run.  A primitive past its
+// child's range is an error of the build; it is not written, and the kernels launched behind
+// take every primitive, also one that was never written, as closed.
 __global__ void k_partitionScatter(int n, const int* __restrict__ primIdx, const int* __restrict__ primNode,
                                    const BNode* __restrict__ nodes, const float4* __restrict__ bmin,
                                    const float4* __restrict__ bmax, const int* __restrict__ flags,
@@ -853,7 +880,9 @@ __global__ void k_partitionScatter(int n, const int* __restrict__ primIdx, const
                                    float4* __restrict__ outMin, float4* __restrict__ outMax, int openCount, int* err) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
-  const int node = primNode[i];
+  const bool failed = *(volatile int*)err != 0;
+  int node = primNode[i];
+  if (failed) node = -1;
   int pos = i, outN = -1;
   if (node >= 0) {
     const BNode& nd = nodes[node];
@@ -941,9 +970,10 @@ __global__ void k_gather(int n, const int* __restrict__ primIdx, const float4* _
 __global__ void __launch_bounds__(128) k_collapse(const int* __restrict__ count, const int2* __restrict__ tasks,
                                                   const BNode* __restrict__ nodes, const int* __restrict__ primIdx,
                                                   float4* __restrict__ nodes8, int* counters, int2* __restrict__ nextTasks,
-                                                  int* nextCount, int* __restrict__ triOrder, int maxNodes8) {
+                                                  int* nextCount, int* __restrict__ triOrder, int maxNodes8,
+                                                  const int* __restrict__ err) {
   constexpr unsigned kAll = 0xffffffffu;
-  const int numTasks = *count;
+  const int numTasks = *err ? 0 : *count;
   const int lane = threadIdx.x & 7, shift = threadIdx.x & 24;  // lane of the node's eight, their place in the warp
   auto of = [&](auto v, int l) { return __shfl_sync(kAll, v, l, 8); };
   auto minOf = [&](float v) {
@@ -1265,17 +1295,20 @@ rg_status buildDeviceBvh(DeviceScene& ds, int nbins, bool wide, cudaStream_t st,
         k_prepareLevel<<<gridFor(warpSplit ? nt : (long long)nt * nbins, 256), 256, 0, st>>>(count, c0, nt, curTasks, nodes.p,
                                                                                           bins.p, nbins, !warpSplit);
         if (warpSplit) {
-          k_bin<<<gridFor(n, kBinChunk), 256, 0, st>>>(n, curNode, nodes.p, curLo, curHi, bins.p, nbins);
+          k_bin<<<gridFor(n, kBinChunk), 256, 0, st>>>(n, curNode, nodes.p, curLo, curHi, bins.p, nbins,
+                                                   counters.p + C_BUILD_ERROR);
           k_splitWarp<<<gridFor((long long)nt * 32, 128), 128, 0, st>>>(
               count, c0, nt, curTasks, nodes.p, bins.p, nbins, counters.p + C_NODES, nxtTasks, nextCount, smallTasks.p,
-              counters.p + C_SMALL, wide ? kWideMaxLeaf : kMaxLeaf);
+              counters.p + C_SMALL, wide ? kWideMaxLeaf : kMaxLeaf, counters.p + C_BUILD_ERROR);
         } else {
-          k_binAny<<<gridFor(n, kBinChunk), 256, 0, st>>>(n, curNode, nodes.p, curLo, curHi, bins.p, nbins);
+          k_binAny<<<gridFor(n, kBinChunk), 256, 0, st>>>(n, curNode, nodes.p, curLo, curHi, bins.p, nbins,
+                                                   counters.p + C_BUILD_ERROR);
           k_split<<<gridFor(nt, 128), 128, 0, st>>>(count, c0, nt, curTasks, nodes.p, bins.p, nbins, counters.p + C_NODES,
                                                      nxtTasks, nextCount, wide ? kWideMaxLeaf : kMaxLeaf);
         }
       }
-      k_partitionFlags<<<gridFor(n, 256), 256, 0, st>>>(n, curNode, nodes.p, curLo, curHi, nbins, pflags.p);
+      k_partitionFlags<<<gridFor(n, 256), 256, 0, st>>>(n, curNode, nodes.p, curLo, curHi, nbins, pflags.p,
+                                                          counters.p + C_BUILD_ERROR);
       cub::DeviceScan::ExclusiveSum(scanTmp.p, scanBytes, pflags.p, pbefore.p, n, st);
       k_partitionScatter<<<gridFor(n, 256), 256, 0, st>>>(n, curIdx, curNode, nodes.p, curLo, curHi, pflags.p, pbefore.p, altIdx,
                                                           altNode, altLo, altHi, openCount, counters.p + C_BUILD_ERROR);
@@ -1302,7 +1335,8 @@ rg_status buildDeviceBvh(DeviceScene& ds, int nbins, bool wide, cudaStream_t st,
   if (warpSplit && n > 4)
     k_subtrees<<<std::min(n / 5 + 1, 148 * 8), kSubThreads, 0, st>>>(counters.p + C_SMALL, smallTasks.p, nodes.p, curIdx,
                                                                     curLo, curHi, nbins, counters.p + C_NODES,
-                                                                    wide ? kWideMaxLeaf : kMaxLeaf);
+                                                                    wide ? kWideMaxLeaf : kMaxLeaf,
+                                                                    counters.p + C_BUILD_ERROR);
   ds.buildLevels = levels;
   if (!ds.triVerts.alloc((size_t)n * 3) || !ds.triShade.alloc((size_t)n * 3) || !ds.triOrig.alloc(n)) {
     err = "out of device memory (triangles)";
@@ -1337,7 +1371,8 @@ rg_status buildDeviceBvh(DeviceScene& ds, int nbins, bool wide, cudaStream_t st,
       while (more > 0) {
         const long long most = std::min<long long>((long long)n / 5 + 2, lv < 10 ? 1ll << (3 * lv) : (long long)n);
         k_collapse<<<(int)std::min<long long>((most + 15) / 16, 148 * 16), 128, 0, st>>>(
-            levelCount.p + lv, cur, nodes.p, curIdx, ds.nodes8.p, c8.p, nxt, levelCount.p + lv + 1, order.p, cap);
+            levelCount.p + lv, cur, nodes.p, curIdx, ds.nodes8.p, c8.p, nxt, levelCount.p + lv + 1, order.p, cap,
+            counters.p + C_BUILD_ERROR);
         std::swap(cur, nxt);
         if (++lv < ahead) continue;
         cudaMemcpyAsync(&more, levelCount.p + lv, sizeof(int), cudaMemcpyDeviceToHost, st);
