@@ -7,7 +7,7 @@
 // reference's filter exactly (B3 5x5 taps at step 2^level, luminance /
 // normal / depth edge stops, firefly pre-clamp, albedo demodulation) with
 // FP32 colour and FP16 guide buffers; every pass is one kernel, one thread
-// per pixel, reading its taps through the read-only cache.
+// per one or two pixels.
 #include <cuda_fp16.h>
 
 #include <algorithm>
@@ -40,11 +40,11 @@ __device__ __forceinline__ __half guideHalf(float v) { return __float2half(v); }
 template <typename T>
 __device__ __forceinline__ float guideAt(const T* g, int i) { return __half2float(guideHalf(g[i])); }
 
-// Firefly pre-clamp + albedo demodulation (rayrenderer.cpp:2685-2722), and what the
-// levels read per tap: the colour with its luminance in w, and the normal and depth
-// guides as one 8-byte word.
 // The denoiser's passes follow one another on the stream as programmatic dependents: a
-// pass's blocks come up while the previous pass drains and wait here for its results.
+// pass's blocks come up while the previous pass drains and wait here for its results.  Its
+// grid is thus alive while what it reads is still written, so the passes read with ordinary
+// loads: the read-only path (const __restrict__, __ldg) is for data that nobody writes while
+// the kernel lives.
 __device__ __forceinline__ void afterPreviousPass() {
   asm volatile("griddepcontrol.launch_dependents;");
   asm volatile("griddepcontrol.wait;" ::: "memory");
@@ -63,11 +63,12 @@ void launchPass(void (*kernel)(P...), dim3 grid, dim3 block, cudaStream_t st, A.
   cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);
 }
 
+// Firefly pre-clamp + albedo demodulation (rayrenderer.cpp:2685-2722), and what the
+// levels read per tap: the colour with its luminance in w, and the normal and depth
+// guides as one 8-byte word.
 template <typename T>
-__global__ void __launch_bounds__(256) k_prepass(int w, int h, const float4* __restrict__ noisy, const T* __restrict__ normal,
-                                                 const T* __restrict__ depth, const T* __restrict__ albedo,
-                                                 const T* __restrict__ albedoA, float4* __restrict__ out,
-                                                 uint2* __restrict__ guide) {
+__global__ void __launch_bounds__(256) k_prepass(int w, int h, const float4* noisy, const T* normal, const T* depth,
+                                                 const T* albedo, const T* albedoA, float4* out, uint2* guide) {
   afterPreviousPass();
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= w * h) return;
@@ -81,7 +82,7 @@ __global__ void __launch_bounds__(256) k_prepass(int w, int h, const float4* __r
       if (dx == 0 && dy == 0) continue;
       const int nx = x + dx;
       if (nx < 0 || nx >= w) continue;
-      const float4 q = __ldg(&noisy[ny * w + nx]);
+      const float4 q = noisy[ny * w + nx];
       const float l = lum3(q.x, q.y, q.z);
       if (l > maxN) maxN = l;
     }
@@ -134,9 +135,8 @@ __device__ __forceinline__ float ex2Ftz(float x) {
 // 249 with packed guides, 219 with the logarithms folded, 187 with two pixels a thread, 174
 // with the passes launched as programmatic dependents (54 x 44, 6 levels: 71 -> 40).
 template <int NPX, bool INSIDE, bool POS>
-__device__ __forceinline__ void atrousPixels(int w, int h, int x, int y, const float4* __restrict__ src,
-                                             float4* __restrict__ dst, const uint2* __restrict__ guide, int step,
-                                             float invC2, float sigN, float dScale) {
+__device__ __forceinline__ void atrousPixels(int w, int h, int x, int y, const float4* src, float4* dst,
+                                             const uint2* guide, int step, float invC2, float sigN, float dScale) {
   // base-2 logarithms of the B3 kernel's taps 1/16, 1/4, 3/8, 1/4, 1/16
   constexpr float kLg[5] = {-4.0f, -2.0f, -1.41503749927884381f, -2.0f, -4.0f};
   float4 cc[NPX];
@@ -146,8 +146,8 @@ __device__ __forceinline__ void atrousPixels(int w, int h, int x, int y, const f
   for (int j = 0; j < NPX; ++j) {
     sx[j] = sy[j] = sz[j] = ws[j] = 0.0f;
     const int yy = min(y + j * step, h - 1);  // rows past the image compute a copy that is not stored
-    cc[j] = __ldg(&src[yy * w + x]);
-    cg[j] = unpackGuide(__ldg(&guide[yy * w + x]));
+    cc[j] = src[yy * w + x];
+    cg[j] = unpackGuide(guide[yy * w + x]);
   }
 #pragma unroll
   for (int k = -2; k < NPX + 2; ++k) {
@@ -158,8 +158,8 @@ __device__ __forceinline__ void atrousPixels(int w, int h, int x, int y, const f
       const int nx = x + (kx - 2) * step;
       if (!INSIDE && (nx < 0 || nx >= w)) continue;
       const int si = ny * w + nx;
-      const float4 sc = __ldg(&src[si]);
-      const Guide sg = unpackGuide(__ldg(&guide[si]));
+      const float4 sc = src[si];
+      const Guide sg = unpackGuide(guide[si]);
 #pragma unroll
       for (int j = 0; j < NPX; ++j) {
         const int ky = k - j + 2;
@@ -193,9 +193,8 @@ __device__ __forceinline__ void atrousPixels(int w, int h, int x, int y, const f
 // invC2 and dScale carry the factor log2(e).  Row t of threads holds rows
 // (t / step) step NPX + t % step + j step, j < NPX.
 template <int NPX>
-__global__ void __launch_bounds__(128) k_atrous(int w, int h, const float4* __restrict__ src, float4* __restrict__ dst,
-                                                const uint2* __restrict__ guide, int level, float invC2, float sigN,
-                                                float dScale) {
+__global__ void __launch_bounds__(128) k_atrous(int w, int h, const float4* src, float4* dst, const uint2* guide,
+                                                int level, float invC2, float sigN, float dScale) {
   afterPreviousPass();
   const int step = 1 << level, r = 2 * step;
   const int x0 = blockIdx.x * blockDim.x, t0 = blockIdx.y * blockDim.y, t1 = t0 + (int)blockDim.y - 1;
@@ -218,9 +217,8 @@ static void launchAtrous(int w, int h, const float4* src, float4* dst, const uin
 
 // Remodulate and blend with the noisy input (rayrenderer.cpp:2752-2771).
 template <typename T>
-__global__ void __launch_bounds__(256) k_remod(int n, const float4* __restrict__ filtered, const float4* __restrict__ noisy,
-                                               const T* __restrict__ albedo, const T* __restrict__ albedoA, float intensity,
-                                               float4* __restrict__ out) {
+__global__ void __launch_bounds__(256) k_remod(int n, const float4* filtered, const float4* noisy, const T* albedo,
+                                               const T* albedoA, float intensity, float4* out) {
   afterPreviousPass();
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
