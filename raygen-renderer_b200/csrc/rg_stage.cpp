@@ -91,9 +91,7 @@ int g_users = 0;
 size_t g_missed = 0;  // gain of the copies made directly for want of a set
 Stage* g_free[kKept] = {};
 
-Stage* acquire(size_t gain) {
-  int dev = 0;
-  if (cudaGetDevice(&dev) != cudaSuccess) return nullptr;
+Stage* acquire(int dev, size_t gain) {
   {
     std::lock_guard<std::mutex> lk(g_mu);
     if (g_users == 0) return nullptr;  // nothing would keep the set: not worth its allocation
@@ -126,13 +124,14 @@ void release(Stage* s) {
   delete s;
 }
 
-bool pageable(const void* p) {
+cudaMemoryType typeOf(const void* p, int* device = nullptr) {
   cudaPointerAttributes a;
   if (cudaPointerGetAttributes(&a, p) != cudaSuccess) {
     cudaGetLastError();
-    return false;
+    return cudaMemoryTypeManaged;  // neither pageable nor a device's own: copied directly
   }
-  return a.type == cudaMemoryTypeUnregistered;
+  if (device) *device = a.device;
+  return a.type;
 }
 
 // Whether the bytes lie in pages that are already there (looked up at 16 of them).
@@ -181,11 +180,15 @@ cudaError_t work(Stage& s, int w, bool toHost, unsigned char* host, unsigned cha
 
 // The staged copy; false: not done (no staging to be had), copy directly.
 bool staged(bool toHost, void* host, void* dev, size_t bytes, cudaStream_t after, cudaError_t& err) {
-  if (bytes < kStagedBytes || !pageable(host)) return false;
+  if (bytes < kStagedBytes || typeOf(host) != cudaMemoryTypeUnregistered) return false;
+  // a set's streams and events belong to the device that is current here; a thread may copy from
+  // another one's memory
+  int current = 0, device = 0;
+  if (cudaGetDevice(&current) != cudaSuccess || typeOf(dev, &device) != cudaMemoryTypeDevice || device != current) return false;
   cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
   if (cudaStreamIsCapturing(after, &cap) != cudaSuccess || cap != cudaStreamCaptureStatusNone) return false;
   if (toHost && bytes < kStagedTouched && touched((const unsigned char*)host, bytes)) return false;
-  Stage* s = acquire(toHost ? bytes * kUntouchedGain : bytes);
+  Stage* s = acquire(device, toHost ? bytes * kUntouchedGain : bytes);
   if (!s) return false;
   const int chunks = (int)std::min<size_t>(kWorkers, (bytes + 2 * kChunk - 1) / (2 * kChunk));
   const int cores = (int)std::thread::hardware_concurrency();

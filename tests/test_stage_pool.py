@@ -1,0 +1,66 @@
+"""The pool of page-locked slots behind large copies (rg_stage.cpp), on the CPU: the file is
+compiled against a CUDA runtime whose devices are host memory (fake_cudart.cpp), which counts the
+sets of slots made and refuses what the real one refuses."""
+import ctypes
+import os
+import subprocess
+import threading
+
+import numpy as np
+import pytest
+
+HERE = os.path.dirname(os.path.abspath(__file__))
+CSRC = os.path.join(os.path.dirname(HERE), "raygen-renderer_b200", "csrc")
+MB = 1 << 20
+
+
+@pytest.fixture(scope="session")
+def built(tmp_path_factory):
+    out = tmp_path_factory.mktemp("stage") / "libstage.so"
+    cuda = os.environ.get("CUDA_HOME", "/usr/local/cuda")
+    subprocess.run(["g++", "-O1", "-std=c++17", "-fPIC", "-shared", "-I" + CSRC, "-I" + os.path.join(cuda, "include"),
+                    os.path.join(HERE, "fake_cudart.cpp"), os.path.join(CSRC, "rg_stage.cpp"), "-o", str(out),
+                    "-lpthread"], check=True)
+    lib = ctypes.CDLL(str(out))
+    lib.fake_user.restype = ctypes.c_void_p
+    lib.fake_user_end.argtypes = [ctypes.c_void_p]
+    lib.fake_device.restype = ctypes.c_void_p
+    lib.fake_round_trip.argtypes = [ctypes.c_int, ctypes.c_void_p, ctypes.c_void_p, ctypes.c_size_t]
+    lib.fake_upload.argtypes = [ctypes.c_int, ctypes.c_void_p, ctypes.c_size_t]
+    return lib
+
+
+@pytest.fixture
+def lib(built):
+    user = built.fake_user()
+    yield built
+    built.fake_current(0)
+    built.fake_capture_fails(0)
+    built.fake_user_end(user)  # the last user: the pool is empty again
+
+
+def data(mb, seed=0):
+    return np.random.default_rng(seed).integers(0, 256, mb * MB, dtype=np.uint8)
+
+
+def round_trip(lib, device, a):
+    back = np.empty_like(a)
+    assert lib.fake_round_trip(device, a.ctypes.data, back.ctypes.data, a.nbytes) == 0
+    np.testing.assert_array_equal(a, back)
+
+
+def test_copies_and_one_set(lib):
+    """20 MB pays for a set; the copies after it use the same one."""
+    before = lib.fake_sets_made()
+    for k in range(5):
+        round_trip(lib, 0, data(20, k)[k:])
+    assert lib.fake_sets_made() - before == 1
+
+
+def test_device_of_the_memory(lib):
+    """A thread whose current device is another one than the handle's, as a program's reader
+    threads are (their current device is 0 unless set): the copy is made all the same."""
+    lib.fake_current(0)
+    round_trip(lib, 1, data(20))
+    round_trip(lib, 0, data(20))
+    round_trip(lib, 1, data(20))
