@@ -8,9 +8,10 @@
 // copied.  Page-locked callers, small copies and images into pages that are already
 // there keep the direct copy.
 //
-// The page-locked slots and streams are pooled (at most kKept sets, 8 MB each)
-// while any renderer or denoiser exists, and freed with the last one; threads
-// live only for the copy.  Every set is used by one copy at a time.
+// The page-locked slots and streams are pooled (at most kKept sets of 8 MB per
+// device) while any renderer or denoiser exists, and freed with the last one;
+// threads live only for the copy.  Every set is used by one copy at a time, and no
+// set is made that would not be kept: copies beyond the sets are direct.
 #include <cuda_runtime.h>
 
 #include <sys/mman.h>
@@ -41,7 +42,7 @@ constexpr size_t kStagedBytes = size_t(3) << 20, kStagedTouched = size_t(48) << 
 // 4.0 without).
 constexpr size_t kSetCost = size_t(16) << 20;
 constexpr int kUntouchedGain = 6;
-constexpr int kKept = 2;
+constexpr int kKept = 2, kDevices = 64;
 // The slots are page-locked where they lie, in huge pages: a first copy waits 1.2 ms for them,
 // and 3.3 - 6.3 ms for the 2048 small pages of a cudaHostAlloc.
 constexpr size_t kHugePage = size_t(2) << 20, kSlotBytes = kWorkers * 2 * kChunk,
@@ -88,38 +89,48 @@ struct Stage {
 
 std::mutex g_mu;
 int g_users = 0;
-size_t g_missed = 0;  // gain of the copies made directly for want of a set
-Stage* g_free[kKept] = {};
+struct Pool {
+  Stage* idle[kKept] = {};
+  int made = 0;       // sets of this device, idle and in use
+  size_t missed = 0;  // gain of the copies made directly for want of a set
+} g_pool[kDevices];
 
 Stage* acquire(int dev, size_t gain) {
+  if (dev >= kDevices) return nullptr;
+  Pool& pool = g_pool[dev];
   {
     std::lock_guard<std::mutex> lk(g_mu);
     if (g_users == 0) return nullptr;  // nothing would keep the set: not worth its allocation
-    for (auto& f : g_free)
-      if (f && f->device == dev) return std::exchange(f, nullptr);
-    if (gain < kSetCost - g_missed) {
-      g_missed += gain;
+    for (auto& s : pool.idle)
+      if (s) return std::exchange(s, nullptr);
+    if (pool.made == kKept) return nullptr;  // all in use
+    if (gain < kSetCost - pool.missed) {
+      pool.missed += gain;
       return nullptr;
     }
-    g_missed = 0;
+    pool.missed = 0;
+    pool.made++;
   }
   Stage* s = new (std::nothrow) Stage();
-  if (s && !s->init(dev)) {
-    delete s;
-    s = nullptr;
-  }
-  return s;
+  if (s && s->init(dev)) return s;
+  delete s;
+  std::lock_guard<std::mutex> lk(g_mu);
+  pool.made--;
+  return nullptr;
 }
 
 void release(Stage* s) {
   {
     std::lock_guard<std::mutex> lk(g_mu);
-    if (g_users > 0)
-      for (auto& f : g_free)
-        if (!f) {
-          f = s;
+    Pool& pool = g_pool[s->device];
+    if (g_users > 0) {
+      for (auto& place : pool.idle)
+        if (!place) {
+          place = s;
           return;
         }
+    }
+    pool.made--;
   }
   delete s;
 }
@@ -226,15 +237,18 @@ StageUser::StageUser() {
 }
 
 StageUser::~StageUser() {
-  Stage* old[kKept] = {};
+  Stage* old[kDevices][kKept] = {};
   {
     std::lock_guard<std::mutex> lk(g_mu);
-    if (--g_users == 0) {
-      for (int i = 0; i < kKept; ++i) old[i] = std::exchange(g_free[i], nullptr);
-      g_missed = 0;
+    if (--g_users > 0) return;
+    for (int d = 0; d < kDevices; ++d) {
+      g_pool[d].missed = 0;
+      for (int i = 0; i < kKept; ++i)
+        if ((old[d][i] = std::exchange(g_pool[d].idle[i], nullptr))) g_pool[d].made--;
     }
   }
-  for (auto* s : old) delete s;
+  for (auto& sets : old)
+    for (auto* s : sets) delete s;
 }
 
 cudaError_t copyToHost(void* dst, const void* devSrc, size_t bytes, cudaStream_t after) {

@@ -64,3 +64,30 @@ def test_device_of_the_memory(lib):
     round_trip(lib, 1, data(20))
     round_trip(lib, 0, data(20))
     round_trip(lib, 1, data(20))
+
+
+def test_sets_are_kept_per_device(lib):
+    """Every device keeps the sets it made: a copy does not make one that is thrown away after it."""
+    before = lib.fake_sets_made()
+    for k in range(6):
+        for device in range(4):
+            lib.fake_current(device)
+            round_trip(lib, device, data(20, k))
+    assert lib.fake_sets_made() - before == 4
+
+
+def test_concurrent_copies_make_no_more_sets_than_are_kept(lib):
+    before = lib.fake_sets_made()
+    a, errors = data(40), []
+
+    def work():
+        for _ in range(6):
+            errors.append(lib.fake_upload(0, a.ctypes.data, a.nbytes))
+
+    threads = [threading.Thread(target=work) for _ in range(8)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert errors == [0] * 48
+    assert lib.fake_sets_made() - before <= 2
