@@ -197,7 +197,11 @@ bool staged(bool toHost, void* host, void* dev, size_t bytes, cudaStream_t after
   int current = 0, device = 0;
   if (cudaGetDevice(&current) != cudaSuccess || typeOf(dev, &device) != cudaMemoryTypeDevice || device != current) return false;
   cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
-  if (cudaStreamIsCapturing(after, &cap) != cudaSuccess || cap != cudaStreamCaptureStatusNone) return false;
+  if (cudaStreamIsCapturing(after, &cap) != cudaSuccess) {
+    cudaGetLastError();  // the launch after a direct copy must not find this query's error
+    return false;
+  }
+  if (cap != cudaStreamCaptureStatusNone) return false;
   if (toHost && bytes < kStagedTouched && touched((const unsigned char*)host, bytes)) return false;
   Stage* s = acquire(device, toHost ? bytes * kUntouchedGain : bytes);
   if (!s) return false;

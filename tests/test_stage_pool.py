@@ -91,3 +91,11 @@ def test_concurrent_copies_make_no_more_sets_than_are_kept(lib):
         t.join()
     assert errors == [0] * 48
     assert lib.fake_sets_made() - before <= 2
+
+
+def test_a_refused_capture_query_leaves_no_error_behind(lib):
+    """Another thread's capture refuses the query of the default stream's state: the copy is a
+    direct one, and the launch after it does not find the query's error."""
+    lib.fake_capture_fails(1)
+    round_trip(lib, 0, data(20))
+    assert lib.fake_last_error() == 0
