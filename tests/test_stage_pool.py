@@ -3,8 +3,10 @@ compiled against a CUDA runtime whose devices are host memory (fake_cudart.cpp),
 sets of slots made and refuses what the real one refuses."""
 import ctypes
 import os
+import signal
 import subprocess
 import threading
+import time
 
 import numpy as np
 import pytest
@@ -16,6 +18,8 @@ MB = 1 << 20
 
 @pytest.fixture(scope="session")
 def built(tmp_path_factory):
+    if len(os.sched_getaffinity(0)) < 4:
+        pytest.skip("copies are direct on few cores")
     out = tmp_path_factory.mktemp("stage") / "libstage.so"
     cuda = os.environ.get("CUDA_HOME", "/usr/local/cuda")
     subprocess.run(["g++", "-O1", "-std=c++17", "-fPIC", "-shared", "-I" + CSRC, "-I" + os.path.join(cuda, "include"),
@@ -99,3 +103,74 @@ def test_a_refused_capture_query_leaves_no_error_behind(lib):
     lib.fake_capture_fails(1)
     round_trip(lib, 0, data(20))
     assert lib.fake_last_error() == 0
+
+
+def test_one_core_copies_directly(lib):
+    """A thread that may use one core or two makes no set: its copies would be slower for it."""
+    cores = os.sched_getaffinity(0)
+    before = lib.fake_sets_made()
+    try:
+        os.sched_setaffinity(0, {min(cores)})
+        for k in range(3):
+            round_trip(lib, 0, data(20, k))
+    finally:
+        os.sched_setaffinity(0, cores)
+    assert lib.fake_sets_made() == before
+
+
+def test_threads_are_kept_with_the_set(lib):
+    """A copy starts no threads once its set is there, and they go with the set."""
+    def threads():
+        return len(os.listdir("/proc/self/task"))
+
+    none = threads()
+    round_trip(lib, 0, data(20))
+    kept = threads()
+    assert none < kept <= none + 7
+    seen = []
+
+    def watch():
+        while not done.is_set():
+            seen.append(threads())
+
+    done = threading.Event()
+    watcher = threading.Thread(target=watch)
+    watcher.start()
+    for k in range(10):
+        round_trip(lib, 0, data(20, k))
+    done.set()
+    watcher.join()
+    assert max(seen) <= kept + 1  # and the watcher
+    second = lib.fake_user()
+    lib.fake_user_end(second)
+    assert threads() == kept
+
+
+def test_threads_end_with_the_last_user(built):
+    before = len(os.listdir("/proc/self/task"))
+    user = built.fake_user()
+    round_trip(built, 0, data(20))
+    built.fake_user_end(user)
+    assert len(os.listdir("/proc/self/task")) == before
+
+
+def test_a_forked_child_may_end_its_users(built):
+    """A child inherits the handles but no threads: closing the last one there returns."""
+    user = built.fake_user()
+    round_trip(built, 0, data(20))
+    child = os.fork()
+    if child == 0:
+        built.fake_user_end(user)
+        os._exit(0)
+    for _ in range(200):
+        pid, status = os.waitpid(child, os.WNOHANG)
+        if pid:
+            break
+        time.sleep(0.05)
+    else:
+        os.kill(child, signal.SIGKILL)
+        os.waitpid(child, 0)
+        pytest.fail("the child hangs")
+    assert status == 0
+    round_trip(built, 0, data(20))
+    built.fake_user_end(user)
