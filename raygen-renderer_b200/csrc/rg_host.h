@@ -45,7 +45,7 @@ void trimPoolMemory();
 // copyToDevice when src may be changed, with work later put on `after` behind the copy.
 cudaError_t copyToHost(void* dst, const void* devSrc, size_t bytes, cudaStream_t after);
 cudaError_t copyToDevice(void* devDst, const void* src, size_t bytes, cudaStream_t after);
-// Held by each renderer and denoiser: the pooled slots live as long as any does.
+// Held by each renderer, denoiser and server: the pooled slots live as long as any does.
 struct StageUser {
   StageUser();
   ~StageUser();

@@ -108,6 +108,7 @@ size_t jobDeviceBytes(const ServerJob& j) {
 using namespace rg;
 
 struct rg_server {
+  StageUser stage;
   rg_settings base{};
   rg_server_config cfg{};
   std::atomic<rg_denoiser*> denoiser{nullptr};  // jobs with denoise == 2

@@ -9,7 +9,7 @@
 // there keep the direct copy.
 //
 // The page-locked slots, streams and threads are pooled (at most kKept sets of 8 MB
-// per device) while any renderer or denoiser exists, and freed with the last one.
+// per device) while any renderer, denoiser or server exists, and freed with the last.
 // Every set is used by one copy at a time, and no set is made that would not be
 // kept: copies beyond the sets are direct.
 #include <cuda_runtime.h>
@@ -151,6 +151,7 @@ struct Stage {
     return true;
   }
   void help(int w) {
+    pthread_setname_np(pthread_self(), "rg_copy");
     cudaSetDevice(device);
     std::unique_lock<std::mutex> lk(mu);
     for (int last = 0;;) {
