@@ -23,7 +23,7 @@ def built(tmp_path_factory):
     out = tmp_path_factory.mktemp("stage") / "libstage.so"
     cuda = os.environ.get("CUDA_HOME", "/usr/local/cuda")
     subprocess.run(["g++", "-O1", "-std=c++17", "-fPIC", "-shared", "-I" + CSRC, "-I" + os.path.join(cuda, "include"),
-                    os.path.join(HERE, "fake_cudart.cpp"), os.path.join(CSRC, "rg_stage.cpp"), "-o", str(out),
+                    os.path.join(HERE, "fake_cudart.cpp"), os.path.join(CSRC, "rg_stage.cpp"), "-o", str(out), "-Wl,-Bsymbolic",
                     "-lpthread"], check=True)
     lib = ctypes.CDLL(str(out))
     lib.fake_user.restype = ctypes.c_void_p
@@ -154,6 +154,7 @@ def test_threads_end_with_the_last_user(built):
     assert len(os.listdir("/proc/self/task")) == before
 
 
+@pytest.mark.filterwarnings("ignore:.*multi-threaded.*:DeprecationWarning")
 def test_a_forked_child_may_end_its_users(built):
     """A child inherits the handles but no threads: closing the last one there returns."""
     user = built.fake_user()
