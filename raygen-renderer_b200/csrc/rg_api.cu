@@ -13,7 +13,6 @@
 #include <chrono>
 #include <condition_variable>
 #include <climits>
-#include <functional>
 #include <cstdlib>
 #include <unordered_map>
 #include <cmath>
@@ -1135,6 +1134,56 @@ rg_status prepareScene(const rg_scene_desc* d, int bins, bool wide, cudaStream_t
 
 }  // namespace rg
 
+namespace {
+
+// One batch query: `rays` (and `tmax`) in, `launch(scene, in, out)` on h->stream, then the
+// results in two parts (host array, bytes).
+template <typename Launch>
+rg_status runQuery(rg_handle* h, const float* rays, const float* tmax, int n, size_t outWords, const Launch& launch,
+                   void* out0, size_t bytes0, void* out1, size_t bytes1) {
+  QueryBuffers& b = h->query;
+  const size_t inWords = (size_t)n * (tmax ? 7 : 6);
+  if (!b.io.alloc(inWords + 1 + outWords)) return RG_ERR_OUT_OF_MEMORY;
+  const bool small = n <= QueryBuffers::kSmall && b.host;
+  cudaStream_t st = h->stream;
+  float* error = b.io.p + inWords;
+  DevScene S = h->dscene;
+  S.error = reinterpret_cast<int*>(error);  // this query's flag only
+  int derr = 0;
+  if (small) {
+    std::memcpy(b.host, rays, sizeof(float) * 6 * n);
+    if (tmax) std::memcpy(b.host + sizeof(float) * 6 * n, tmax, sizeof(float) * n);
+    std::memcpy(b.host + sizeof(float) * inWords, &derr, sizeof(int));
+    RG_CUDA_CHECK(cudaMemcpyAsync(b.io.p, b.host, sizeof(float) * (inWords + 1), cudaMemcpyHostToDevice, st));
+  } else {
+    RG_CUDA_CHECK(cudaMemsetAsync(error, 0, sizeof(int), st));
+    RG_CUDA_CHECK(copyToDevice(b.io.p, rays, sizeof(float) * 6 * n, st));
+    if (tmax) RG_CUDA_CHECK(copyToDevice(b.io.p + (size_t)6 * n, tmax, sizeof(float) * n, st));
+  }
+  launch(S, b.io.p, error + 1);
+  if (small) {
+    unsigned char* o = b.host + sizeof(float) * inWords;
+    RG_CUDA_CHECK(cudaMemcpyAsync(o, error, sizeof(int) + bytes0 + bytes1, cudaMemcpyDeviceToHost, st));
+    RG_CUDA_CHECK(cudaStreamSynchronize(st));
+    std::memcpy(&derr, o, sizeof(int));
+    std::memcpy(out0, o + sizeof(int), bytes0);
+    if (bytes1) std::memcpy(out1, o + sizeof(int) + bytes0, bytes1);
+  } else {
+    const unsigned char* o = reinterpret_cast<const unsigned char*>(error + 1);
+    RG_CUDA_CHECK(copyToHost(out0, o, bytes0, st));
+    if (bytes1) RG_CUDA_CHECK(copyToHost(out1, o + bytes0, bytes1, st));
+    RG_CUDA_CHECK(copyToHost(&derr, error, sizeof(int), st));
+    b.trim();
+  }
+  if (derr) {
+    setLastError("device error flag raised: " + std::to_string(derr));
+    return RG_ERR_DEVICE_STATUS;
+  }
+  return RG_OK;
+}
+
+}  // namespace
+
 extern "C" {
 
 rg_status rg_set_scene(rg_handle* h, const rg_scene_desc* d) {
@@ -1772,52 +1821,6 @@ rg_status rg_probe_sampling(int32_t which, const float* in, int32_t n, float* ou
 rg_status rg_get_view_matrix(rg_handle* h, float* m16) {
   if (!h || !m16) return RG_ERR_INVALID_ARGUMENT;
   std::memcpy(m16, h->view.m, sizeof(float) * 16);
-  return RG_OK;
-}
-
-// One batch query: `rays` (and `tmax`) in, `launch(scene, in, out)` on h->stream, then the
-// results in two parts (host array, bytes).
-static rg_status runQuery(rg_handle* h, const float* rays, const float* tmax, int n, size_t outWords,
-                          const std::function<void(const DevScene&, const float*, float*)>& launch, void* out0, size_t bytes0,
-                          void* out1, size_t bytes1) {
-  QueryBuffers& b = h->query;
-  const size_t inWords = (size_t)n * (tmax ? 7 : 6);
-  if (!b.io.alloc(inWords + 1 + outWords)) return RG_ERR_OUT_OF_MEMORY;
-  const bool small = n <= QueryBuffers::kSmall && b.host;
-  cudaStream_t st = h->stream;
-  float* error = b.io.p + inWords;
-  DevScene S = h->dscene;
-  S.error = reinterpret_cast<int*>(error);  // this query's flag only
-  int derr = 0;
-  if (small) {
-    std::memcpy(b.host, rays, sizeof(float) * 6 * n);
-    if (tmax) std::memcpy(b.host + sizeof(float) * 6 * n, tmax, sizeof(float) * n);
-    std::memcpy(b.host + sizeof(float) * inWords, &derr, sizeof(int));
-    RG_CUDA_CHECK(cudaMemcpyAsync(b.io.p, b.host, sizeof(float) * (inWords + 1), cudaMemcpyHostToDevice, st));
-  } else {
-    RG_CUDA_CHECK(cudaMemsetAsync(error, 0, sizeof(int), st));
-    RG_CUDA_CHECK(copyToDevice(b.io.p, rays, sizeof(float) * 6 * n, st));
-    if (tmax) RG_CUDA_CHECK(copyToDevice(b.io.p + (size_t)6 * n, tmax, sizeof(float) * n, st));
-  }
-  launch(S, b.io.p, error + 1);
-  if (small) {
-    unsigned char* o = b.host + sizeof(float) * inWords;
-    RG_CUDA_CHECK(cudaMemcpyAsync(o, error, sizeof(int) + bytes0 + bytes1, cudaMemcpyDeviceToHost, st));
-    RG_CUDA_CHECK(cudaStreamSynchronize(st));
-    std::memcpy(&derr, o, sizeof(int));
-    std::memcpy(out0, o + sizeof(int), bytes0);
-    if (bytes1) std::memcpy(out1, o + sizeof(int) + bytes0, bytes1);
-  } else {
-    const unsigned char* o = reinterpret_cast<const unsigned char*>(error + 1);
-    RG_CUDA_CHECK(copyToHost(out0, o, bytes0, st));
-    if (bytes1) RG_CUDA_CHECK(copyToHost(out1, o + bytes0, bytes1, st));
-    RG_CUDA_CHECK(copyToHost(&derr, error, sizeof(int), st));
-    b.trim();
-  }
-  if (derr) {
-    setLastError("device error flag raised: " + std::to_string(derr));
-    return RG_ERR_DEVICE_STATUS;
-  }
   return RG_OK;
 }
 
