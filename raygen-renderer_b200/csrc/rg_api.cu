@@ -281,15 +281,42 @@ using namespace rg;
 // Buffers of the ray-batch queries, kept between calls: allocating and freeing them took a
 // third of a 1000-ray query.  One device array holds the inputs, the query's error word and
 // the outputs, in this order, so a batch of up to kSmall rays is one copy in (its error word
-// zero), the kernel, and one copy out, through a page-locked array; a larger one is copied
-// from and to the caller's arrays.  More than 64 MB are given back after the call.
+// zero), the kernel, and one copy out, through a host array; a larger one is copied from and
+// to the caller's arrays.  More than 64 MB are given back after the call.
+// The host array is page-locked once the small batches have moved kLockBytes through it: that
+// takes 0.1 - 2.5 ms (the more, the more device memory the process has had), which a 1000-ray
+// query earns at 4 us (43 -> 39 us, 16384 rays 135 -> 90), and a handle that asks for a few
+// rays, or none, never.
 struct QueryBuffers {
   static constexpr int kSmall = 16384;
   static constexpr size_t kHostBytes = (size_t)kSmall * 44 + 16;  // 7 floats in, the error word, 4 words out
+  static constexpr size_t kLockBytes = size_t(16) << 20;
   DevBuf<float> io;
   unsigned char* host = nullptr;
-  ~QueryBuffers() {
-    if (host) cudaFreeHost(host);
+  bool locked = false;
+  size_t moved = 0;  // through the array while it is not page-locked
+  ~QueryBuffers() { dropHost(); }
+  void dropHost() {
+    if (locked) cudaFreeHost(host);
+    else std::free(host);
+    host = nullptr;
+    locked = false;
+  }
+  // The host array for a batch of `bytes` both ways; nullptr: the batch goes the large ones' way.
+  unsigned char* hostFor(size_t bytes) {
+    if (!locked && (moved += bytes) >= kLockBytes) {
+      moved = 0;
+      void* p = nullptr;
+      if (cudaHostAlloc(&p, kHostBytes, cudaHostAllocDefault) == cudaSuccess) {
+        dropHost();
+        host = (unsigned char*)p;
+        locked = true;
+      } else {
+        cudaGetLastError();
+      }
+    }
+    if (!host) host = (unsigned char*)std::malloc(kHostBytes);
+    return host;
   }
   void trim() {
     if (io.bytes() > (size_t(64) << 20)) io.release();
@@ -631,10 +658,6 @@ rg_status rg_create(const rg_settings* s, rg_handle** out) {
     setLastError("cudaStreamCreate failed");
     delete h;
     return RG_ERR_CUDA;
-  }
-  if (cudaHostAlloc((void**)&h->query.host, QueryBuffers::kHostBytes, cudaHostAllocDefault) != cudaSuccess) {
-    cudaGetLastError();  // small queries copy from and to the caller's arrays then
-    h->query.host = nullptr;
   }
   *out = h;
   return RG_OK;
@@ -1144,17 +1167,18 @@ rg_status runQuery(rg_handle* h, const float* rays, const float* tmax, int n, si
   QueryBuffers& b = h->query;
   const size_t inWords = (size_t)n * (tmax ? 7 : 6);
   if (!b.io.alloc(inWords + 1 + outWords)) return RG_ERR_OUT_OF_MEMORY;
-  const bool small = n <= QueryBuffers::kSmall && b.host;
+  unsigned char* host = n <= QueryBuffers::kSmall ? b.hostFor(sizeof(float) * (inWords + 1 + outWords)) : nullptr;
+  const bool small = host != nullptr;
   cudaStream_t st = h->stream;
   float* error = b.io.p + inWords;
   DevScene S = h->dscene;
   S.error = reinterpret_cast<int*>(error);  // this query's flag only
   int derr = 0;
   if (small) {
-    std::memcpy(b.host, rays, sizeof(float) * 6 * n);
-    if (tmax) std::memcpy(b.host + sizeof(float) * 6 * n, tmax, sizeof(float) * n);
-    std::memcpy(b.host + sizeof(float) * inWords, &derr, sizeof(int));
-    RG_CUDA_CHECK(cudaMemcpyAsync(b.io.p, b.host, sizeof(float) * (inWords + 1), cudaMemcpyHostToDevice, st));
+    std::memcpy(host, rays, sizeof(float) * 6 * n);
+    if (tmax) std::memcpy(host + sizeof(float) * 6 * n, tmax, sizeof(float) * n);
+    std::memcpy(host + sizeof(float) * inWords, &derr, sizeof(int));
+    RG_CUDA_CHECK(cudaMemcpyAsync(b.io.p, host, sizeof(float) * (inWords + 1), cudaMemcpyHostToDevice, st));
   } else {
     RG_CUDA_CHECK(cudaMemsetAsync(error, 0, sizeof(int), st));
     RG_CUDA_CHECK(copyToDevice(b.io.p, rays, sizeof(float) * 6 * n, st));
@@ -1162,7 +1186,7 @@ rg_status runQuery(rg_handle* h, const float* rays, const float* tmax, int n, si
   }
   launch(S, b.io.p, error + 1);
   if (small) {
-    unsigned char* o = b.host + sizeof(float) * inWords;
+    unsigned char* o = host + sizeof(float) * inWords;
     RG_CUDA_CHECK(cudaMemcpyAsync(o, error, sizeof(int) + bytes0 + bytes1, cudaMemcpyDeviceToHost, st));
     RG_CUDA_CHECK(cudaStreamSynchronize(st));
     std::memcpy(&derr, o, sizeof(int));
