@@ -1174,8 +1174,8 @@ __global__ void __launch_bounds__(kShadeBlock, RG_SHADE_MIN_BLOCKS) k_shade(DevS
                                                int iter) {
   const int count = Q.counters[iter * kCountersPerIter + C_RAYS];
   const int inB = iter & 1, outB = (iter + 1) & 1;
-  // Each block iteration takes kWin consecutive queue entries (two per thread)
-  // and shades them grouped by the branch their hit takes (a counting sort in
+  // Each block iteration takes a window of consecutive queue entries (at most kWin, two per
+  // thread) and shades them grouped by the branch their hit takes (a counting sort in
   // shared memory), so that a warp mostly runs one lobe: incoherent bounces
   // otherwise leave a third of the lanes active and the kernel waiting on
   // instruction fetch.  Classes: 0 emitter, 1 diffuse, 2 rough glossy,
@@ -1187,13 +1187,20 @@ __global__ void __launch_bounds__(kShadeBlock, RG_SHADE_MIN_BLOCKS) k_shade(DevS
   __shared__ int sOrder[2][kWin];
   if (threadIdx.x < 2 * kBins) sBin[threadIdx.x / kBins][threadIdx.x % kBins] = 0;
   __syncthreads();
+  // Few rays: smaller windows, so that half the grid's blocks, as many as are resident, share them.
+  // In windows of 896, 57600 rays keep 64 of the 148 SMs busy, and a render whose vertices take long
+  // waits for them: heat haze and a cloud under an environment map, 160x90 with 4 samples 2.81 ->
+  // 1.70 ms, 320x180 with 8 4.19 -> 3.09, the cube room at 256x256 0.422 -> 0.417 of shade time;
+  // renders of many waves are unchanged.
+  const int spread = max((int)gridDim.x / 2, 1);
+  const int win = min(kWin, max(32, ((count + spread - 1) / spread + 31) & ~31));
   int buf = 0;
-  for (int base = blockIdx.x * kWin; base < count; base += gridDim.x * kWin, buf ^= 1) {
+  for (int base = blockIdx.x * win; base < count; base += gridDim.x * win, buf ^= 1) {
     {
       int key[kPer], rank[kPer];
 #pragma unroll
       for (int h = 0; h < kPer; ++h) {
-        const int q0 = base + h * kShadeBlock + threadIdx.x;
+        const int i0 = h * kShadeBlock + threadIdx.x, q0 = i0 < win ? base + i0 : count;
         key[h] = kBins - 1;
         if (q0 < count) {
           const int prim0 = __float_as_int(Q.hits[q0].w);
@@ -1221,7 +1228,10 @@ __global__ void __launch_bounds__(kShadeBlock, RG_SHADE_MIN_BLOCKS) k_shade(DevS
       }
       __syncthreads();
 #pragma unroll
-      for (int h = 0; h < kPer; ++h) sOrder[buf][sBin[buf][key[h]] + rank[h]] = base + h * kShadeBlock + threadIdx.x;
+      for (int h = 0; h < kPer; ++h) {
+        const int i0 = h * kShadeBlock + threadIdx.x;
+        sOrder[buf][sBin[buf][key[h]] + rank[h]] = i0 < win ? base + i0 : count;
+      }
       __syncthreads();
     }
     for (int h = 0; h < kPer; ++h) {
