@@ -176,7 +176,6 @@ __global__ void k_initRoot(int n, const uint32_t* rb, BNode* nodes, int* primIdx
   }
 }
 
-// Prepare open nodes of a level: pick the widest centroid axis.
 // Task counts live on the device (`count`, of which this launch takes [first, first + most)), so
 // that levels can be launched before the previous ones have run.
 __device__ __forceinline__ int tasksOf(const int* count, int first, int most) { return max(0, min(*count - first, most)); }
@@ -189,6 +188,7 @@ __device__ __forceinline__ int widestAxis(const BNode& nd) {  // bvh.cpp:125-131
   return axis;
 }
 
+// Prepare open nodes of a level: pick the widest centroid axis.
 __global__ void k_prepareLevel(const int* count, int first, int most, const int* tasks, BNode* nodes, BinData* bins, int nbins,
                                bool resetBins) {
   const int numTasks = tasksOf(count, first, most);
@@ -1166,8 +1166,6 @@ inline int gridFor(long long n, int block) { return (int)((n + block - 1) / bloc
 
 }  // namespace
 
-// Builds the view-space triangle arrays and the BVH for `n` triangles whose
-// world-space inputs are already on the device (DeviceSceneBuild fields).
 // Per-level host timing of the build, printed to stderr when RG_TRACE_HOST is set.
 struct BuildTrace {
   bool on = std::getenv("RG_TRACE_HOST") != nullptr;
@@ -1197,6 +1195,8 @@ struct BvhScratch {
 
 void freeBvhScratch(BvhScratch* s) { delete s; }
 
+// Builds the view-space triangle arrays and the BVH of a scene whose world-space inputs are already
+// on the device (DeviceScene::in*).  Grids of looping kernels count the 148 SMs of a B200.
 rg_status buildDeviceBvh(DeviceScene& ds, int nbins, bool wide, cudaStream_t st, std::string& err) {
   BuildTrace trace;
   const int n = ds.numTris;

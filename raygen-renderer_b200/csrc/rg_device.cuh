@@ -15,9 +15,10 @@ constexpr float kRRMin = 0.05f, kRRMax = 0.95f;  // rayrenderer.cpp:44-45
 constexpr int kMaxLeaf = 8;                   // triangles per leaf in the device BVH
 constexpr int kMaxMediumCount = 64;           // cap on a medium's octaves, strata and march steps
 constexpr int kStackSize = 64;
-// 8-wide BVH node, 128 bytes (8 float4): child base, triangle base, 8 meta bytes; the
-// node's centre and a word of plane scale, inner and leaf masks; then per axis the 8
-// child boxes' lo and hi planes as half values relative to the centre (k_collapse).
+// 8-wide BVH node, 128 bytes (8 float4): child base, triangle base, 8 meta bytes; the planes'
+// origin (per axis the node's low end, centre or high end) and a word of plane scale and inner
+// mask; then per axis the 8 child boxes' lo and hi planes as half values relative to the origin
+// (k_collapse).
 constexpr int kNode8Vec = 8;
 
 // occluder classes (bit per shadow-ray predicate)

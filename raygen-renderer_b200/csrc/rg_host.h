@@ -41,8 +41,9 @@ void trimPoolMemory();
 
 // Copies between the caller's memory and the device (rg_stage.cpp): large ones from or to
 // pageable memory are made by several host threads through page-locked slots.  The copy
-// comes after the work already on `after`.  copyToHost returns when dst holds the bytes;
-// copyToDevice when src may be changed, with work later put on `after` behind the copy.
+// comes after the work already on `after`.  copyToHost returns when dst holds the bytes.
+// copyToDevice returns with work later put on `after` behind the copy; a pageable src may be
+// changed then, a page-locked one when `after` has been waited for (the device reads it in place).
 cudaError_t copyToHost(void* dst, const void* devSrc, size_t bytes, cudaStream_t after);
 cudaError_t copyToDevice(void* devDst, const void* src, size_t bytes, cudaStream_t after);
 // Held by each renderer, denoiser and server: the pooled slots live as long as any does.

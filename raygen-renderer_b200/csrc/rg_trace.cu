@@ -1152,11 +1152,15 @@ void launchTriMaterial(const DevScene& S, int n, int* triMat, cudaStream_t st) {
 // Block shape of the shade kernel: two blocks of 448 threads per SM (72 registers, 28 warps), two
 // rays per thread, so windows of 896 rays.  The kernel waits for its gathers: with two blocks of
 // 256 threads (128 registers, 16 warps) it issued in 30% of the cycles, and the warps are worth
-// the spills that the bound costs (140 - 1200 bytes).  Shade of 4M triangles 1080p 32 spp / 1M in
+// the spills that the bound costs (470 - 1670 bytes stored, 440 - 2120 loaded).  Shade of 4M triangles 1080p 32 spp / 1M in
 // fog / 150k triangles / the cube room: 2 x 256 43.2 / 33.3 / 3.00 / 0.473 ms, 2 x 320 37.6 / 31.6 /
 // 2.71 / 0.432, 2 x 384 36.3 / 31.5 / 2.58 / 0.433, 2 x 448 36.0 / 29.9 / 2.53 / 0.427, 2 x 512
 // 36.2 / 29.5 / 2.54 / 0.456, 1 x 1024 37.6 / 28.2 / 2.68 / 0.460, 3 x 256 37.9 / 34.4 / 2.61 /
 // 0.429; the grid has to be a multiple of the resident blocks (3 x 256 in a grid of 4 per SM: 53).
+// The variants with more code gain as much.  Whole trace at 960x540, 16 spp with the unbounded kernel
+// / 2 x 256 / 2 x 448 / 1 x 512: environment 6.2 / 5.0 / 4.4 / 4.6 ms, with fog 17.8 / 15.2 / 12.7 /
+// 13.6, with heat haze and a cloud 44.0 / 34.1 / 27.8 / 29.7; without one a cloud 13.0 / 8.6 / 7.6 /
+// 7.9, a flame in fog 23.2 / 15.0 / 14.3 / 13.6.
 // Unbounded, the multi-job kernel took 173-222 registers, one block of 256 per SM (24 jobs
 // through the server 64 ms of device time, 51 now).
 #ifndef RG_SHADE_BLOCK
