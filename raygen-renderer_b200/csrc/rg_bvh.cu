@@ -880,7 +880,7 @@ __global__ void k_partitionScatter(int n, const int* __restrict__ primIdx, const
                                    float4* __restrict__ outMin, float4* __restrict__ outMax, int openCount, int* err) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
-  const bool failed = *(volatile int*)err != 0;
+  const bool failed = *err != 0;
   int node = primNode[i];
   if (failed) node = -1;
   int pos = i, outN = -1;
