@@ -756,7 +756,7 @@ __global__ void __launch_bounds__(128) k_connect(const DevJob* __restrict__ jobs
 // 1M triangles in fog 52.0 -> 41.1 / 26.1 -> 19.2; 20k triangles at 800x600, 4 spp
 // 2.24 -> 1.64 / 1.67 -> 1.20; the cube room at 256x256, 16 spp 0.52 -> 0.38 /
 // 0.29 -> 0.22.  With half-plane nodes and paths in blocks of pixels these cases take
-// 75.6 / 29.4, 35.6 / 17.3, 1.53 / 1.14 and 0.34 / 0.22 ms.  kDirect: 4 / 8 / 12 / 16 / 24 / never gives 99.5 / 91.9 / 90.5 /
+// 76.3 / 29.4, 35.9 / 17.3, 1.54 / 1.14 and 0.34 / 0.22 ms.  kDirect: 4 / 8 / 12 / 16 / 24 / never gives 99.5 / 91.9 / 90.5 /
 // 90.2 / 92.4 / 90.3 ms on the first and 1.77 / 1.69 / 1.64 / 1.78 / 2.03 / 2.16
 // ms on the 20k-triangle scene.  The batch's lower bound on lanes with a node
 // (4 - 20) moves nothing.
